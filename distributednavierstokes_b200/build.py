@@ -7,6 +7,7 @@ only when it or a header changed), then the objects are linked into the
 shared library next to this file, so that it travels with the source tree.
 nvcc cross-compiles without a GPU.
 """
+import concurrent.futures
 import os
 import shutil
 import subprocess
@@ -17,13 +18,14 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(ROOT, "_build")
 OUT = os.path.join(HERE, "libdnsb.so")
-SOURCES = ["dnsb.cu", "cnn.cu"]
+SOURCES = ["dnsb.cu", "fftany.cu", "cnn.cu"]
 INCLUDES = [os.path.join(ROOT, "include", h) for h in ("dnsb.h", "dnsb_cnn.h")]
 # headers each translation unit includes (a change rebuilds its object)
 HEADERS = {
     "dnsb.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "spectral.cuh", "spectral4.cuh", "stencil.cuh",
                 "tma.cuh", "ysolve.cuh", "gradmom.cuh", "zyz.cuh", "spsolver.cuh", "lowshells.cuh",
-                "cnn_host.h"],
+                "cnn_host.h", "fftany.h", "launch.h"],
+    "fftany.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "fftany.cuh", "fftany.h", "launch.h", "pdl.cuh"],
     "cnn.cu": ["cnn.cuh", "cnn_host.h"],
 }
 
@@ -70,14 +72,18 @@ def build(force=False, verbose=False):
     os.makedirs(BUILD, exist_ok=True)
     hc = _host_compiler()
     base = [_nvcc()] + NVCC_FLAGS + (["-ccbin", hc] if hc else [])
-    changed = False
-    for s in SOURCES:
+    stale = [s for s in SOURCES if force or _stale(_obj(s), _deps(s))]
+
+    def compile_one(s):
         o = _obj(s)
-        if force or _stale(o, _deps(s)):
-            cmd = base + (["-Xptxas", "-v"] if verbose else []) + ["-c", "-o", o + ".tmp", os.path.join(CSRC, s)]
-            subprocess.run(cmd, check=True)
-            os.replace(o + ".tmp", o)
-            changed = True
+        cmd = base + (["-Xptxas", "-v"] if verbose else []) + ["-c", "-o", o + ".tmp", os.path.join(CSRC, s)]
+        subprocess.run(cmd, check=True)
+        os.replace(o + ".tmp", o)
+
+    # the translation units side by side: each takes a minute or more
+    with concurrent.futures.ThreadPoolExecutor(len(SOURCES)) as pool:
+        list(pool.map(compile_one, stale))
+    changed = bool(stale)
     objs = [_obj(s) for s in SOURCES]
     if force or changed or _stale(OUT, objs):
         cmd = [_nvcc()] + ARCH + ["-shared"] + (["-ccbin", hc] if hc else []) + ["-o", OUT + ".tmp"] + objs

@@ -12,6 +12,11 @@ namespace dnsb {
 
 enum Stag { STAG_X = 0, STAG_Y = 1, STAG_Z = 2, STAG_P = 3 };
 
+// what the transform kernels read, write and do (spectral.cuh, fftany.cuh)
+enum RInMode { RIN_DIVERGENCE = 0, RIN_REAL = 1, RIN_FIELD = 2, RIN_PRODUCT = 3 };
+enum ROutMode { ROUT_INTERIOR = 0, ROUT_IMAGES = 1, ROUT_REAL = 2 };
+enum YFourierMode { YF_SOLVE = 0, YF_FORWARD = 1, YF_INVERSE = 2 };
+
 struct Fields3 {
   double *x, *y, *z;
 };
@@ -108,7 +113,7 @@ __device__ __forceinline__ void store_img(double *__restrict__ f, const Geo &g, 
 
 // Out-of-line images for callers that write the interior value themselves
 // and only need the ghost images of edge cells (keeps unrolled loops small).
-__device__ __noinline__ void store_images_of(double *__restrict__ f, int nx, int ny, int nz,
+inline __device__ __noinline__ void store_images_of(double *__restrict__ f, int nx, int ny, int nz,
                                              int NX, int NY, int wall, int I, int J, int K,
                                              double v, int stag) {
   store_images_core(f, nx, ny, nz, NX, NY, wall, I, J, K, v, stag);

@@ -31,6 +31,8 @@
 #include "cnn_host.h"
 #include "common.cuh"
 #include "fft.cuh"
+#include "fftany.h"
+#include "launch.h"
 #include "spectral.cuh"
 #include "spectral4.cuh"
 #include "ysolve.cuh"
@@ -158,7 +160,9 @@ struct dnsb_ctx {
   int zyz_c = 0;                       // CTAs per cluster of k_zyz (0: three kernels)
   int zyz_mode = 1;                    // 1: k_zyz (32-row chunks), 2: k_zyz2 (16-row chunks)
   int nkx_active = 0;                  // z-FFTs on kx < nkx_active only (0: all; spectral solver)
-  int x1 = 0, x2 = 0, z1 = 0, z2 = 0;  // four-step splits of nx/2 and nz (0: generic kernels)
+  int x1 = 0, x2 = 0, z1 = 0, z2 = 0;  // compile-time four-step splits of nx/2 and nz (0: none)
+  AnySplit ax, ay_, az;  // run-time splits of nx/2, ny and nz (tier 0: none, the Stockham kernels)
+  int Lx_set = 0, Lz_set = 0, Ly_set = 0;  // lines per block asked for (0: the launch rules)
   int L4z = 8;                         // lines per CTA of the z-FFT
   // divergence x-FFT with its output pass in registers (3 % faster at
   // 384x256x384 than the separate shared-memory pass)
@@ -287,25 +291,6 @@ const dim3 cell_block(32, 8, 1);
 
 CFields3 cf(const double *x, const double *y, const double *z) { return CFields3{x, y, z}; }
 Fields3 ff(double *x, double *y, double *z) { return Fields3{x, y, z}; }
-
-// opt in to the dynamic shared memory a kernel launches with (needed whenever
-// static + dynamic shared memory exceeds 48 KB; requested unconditionally).
-// The attribute belongs to the kernel function (per device), not to the
-// context, so contexts of different sizes in one process may only ever raise
-// it: the largest request per (device, kernel) is kept.
-template <class K>
-cudaError_t raise_smem(int device, K kernel, size_t bytes) {
-  static std::mutex mu;
-  static std::map<std::pair<int, const void *>, size_t> granted;
-  std::lock_guard<std::mutex> lock(mu);
-  size_t &cur = granted[{device, reinterpret_cast<const void *>(kernel)}];
-  if (bytes <= cur && cur != 0) return cudaSuccess;
-  const size_t want = std::max(bytes, cur);
-  const cudaError_t e =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
-  if (e == cudaSuccess) cur = want;
-  return e;
-}
 
 template <class K>
 int allow_smem(dnsb_ctx *c, K kernel, size_t bytes) {
@@ -752,6 +737,10 @@ int allow_fft4_split(dnsb_ctx *c, int a, int b) {
 int launch_rfftx(dnsb_ctx *c, int mode, const double *a, const double *b, const double *cc) {
   const Geo &g = c->g;
   if (c->x1) return launch_rfftx4(c, mode, a, b, cc);
+  if (c->ax.tier) {
+    LAUNCH(c, DNSB_KIND_RFFTX, CK(c, any_rfftx(g, c->ax, c->Lx_set, mode, c->S, a, b, cc, c->twM, c->twN, c->stream)));
+    return 0;
+  }
   dim3 grid(g.ny * ((g.nz + c->Lx - 1) / c->Lx));
   if (mode == RIN_DIVERGENCE)
     LAUNCH(c, DNSB_KIND_RFFTX, k_rfftx<RIN_DIVERGENCE><<<grid, SPEC_THREADS, c->smem_rx, c->stream>>>(g, c->S, a, b, cc, c->pM, c->Lx, c->twM, c->twN));
@@ -765,6 +754,11 @@ int launch_rfftx(dnsb_ctx *c, int mode, const double *a, const double *b, const 
 int launch_fftz(dnsb_ctx *c, bool inv) {
   const Geo &g = c->g;
   if (c->z1 && !c->use_tma) return launch_fftz4(c, inv);
+  if (c->az.tier && !c->use_tma) {
+    LAUNCH(c, inv ? DNSB_KIND_IFFTZ : DNSB_KIND_FFTZ,
+           CK(c, any_fftz(g, c->az, c->nkx_active ? c->nkx_active : g.nkx, c->Lz_set, inv, c->S, c->twz, c->stream)));
+    return 0;
+  }
   long long nlines = (long long)g.ny * (c->nkx_active && !c->use_tma ? c->nkx_active : g.nkx);
   if (c->use_tma) {
     const long long ngroups = (nlines + c->Lz - 1) / c->Lz;
@@ -776,6 +770,24 @@ int launch_fftz(dnsb_ctx *c, bool inv) {
   dim3 grid((unsigned)((nlines + c->Lz - 1) / c->Lz));
   if (inv) LAUNCH(c, DNSB_KIND_IFFTZ, k_fftz<true><<<grid, SPEC_THREADS, c->smem_z, c->stream>>>(g, c->S, c->pz, c->Lz, c->twz));
   else LAUNCH(c, DNSB_KIND_FFTZ, k_fftz<false><<<grid, SPEC_THREADS, c->smem_z, c->stream>>>(g, c->S, c->pz, c->Lz, c->twz));
+  return 0;
+}
+
+// the periodic y-transforms of S (YFourierMode)
+int launch_yfourier(dnsb_ctx *c, int mode) {
+  const Geo &g = c->g;
+  const int nkx = c->nkx_active ? c->nkx_active : g.nkx;
+  if (c->ay_.tier) {
+    LAUNCH(c, DNSB_KIND_YSOLVE,
+           CK(c, any_y(g, c->ay_, nkx, c->Ly_set, mode, c->S, c->twy, c->lam1, c->lam2, c->lam3, c->stream)));
+    return 0;
+  }
+  const dim3 grid((unsigned)(nkx * ((g.nz + c->Ly - 1) / c->Ly)));
+  LAUNCH(c, DNSB_KIND_YSOLVE,
+         (mode == YF_SOLVE ? k_yfourier<YF_SOLVE>
+          : mode == YF_FORWARD ? k_yfourier<YF_FORWARD>
+                               : k_yfourier<YF_INVERSE>)<<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(
+             g, c->S, c->py, c->Ly, c->twy, c->lam1, c->lam2, c->lam3));
   return 0;
 }
 
@@ -798,16 +810,18 @@ int launch_ysolve(dnsb_ctx *c) {
                    g, c->S, c->work, c->ay, c->by, c->cy, c->lam1, c->lam3));
     }
 #undef YT
-  } else {
-    dim3 grid(g.nkx * ((g.nz + c->Ly - 1) / c->Ly));
-    LAUNCH(c, DNSB_KIND_YSOLVE, k_yfourier<YF_SOLVE><<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(g, c->S, c->py, c->Ly, c->twy, c->lam1, c->lam2, c->lam3));
+    return 0;
   }
-  return 0;
+  return launch_yfourier(c, YF_SOLVE);
 }
 
 int launch_irfftx(dnsb_ctx *c, int mode, double *out) {
   const Geo &g = c->g;
   if (c->x1) return launch_irfftx4(c, mode, out);
+  if (c->ax.tier) {
+    LAUNCH(c, DNSB_KIND_IRFFTX, CK(c, any_irfftx(g, c->ax, c->Lx_set, mode, c->S, out, c->twM, c->twN, c->stream)));
+    return 0;
+  }
   dim3 grid(g.ny * ((g.nz + c->Lx - 1) / c->Lx));
   if (mode == ROUT_INTERIOR)
     LAUNCH(c, DNSB_KIND_IRFFTX, k_irfftx<ROUT_INTERIOR><<<grid, SPEC_THREADS, c->smem_ix, c->stream>>>(g, c->S, out, c->pM, c->Lx, c->twM, c->twN));
@@ -1140,11 +1154,7 @@ int spectrum_of(dnsb_ctx *c, const double *u) {
   int rc;
   if ((rc = launch_rfftx(c, RIN_FIELD, u, nullptr, nullptr))) return rc;
   if ((rc = launch_fftz(c, false))) return rc;
-  dim3 grid(g.nkx * ((g.nz + c->Ly - 1) / c->Ly));
-  k_yfourier<YF_FORWARD><<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(g, c->S, c->py, c->Ly, c->twy,
-                                                                       c->lam1, c->lam2, c->lam3);
-  CKL(c);
-  return 0;
+  return launch_yfourier(c, YF_FORWARD);
 }
 
 // E[0..nb) (device) = energies of the floor shells, summed in a fixed order
@@ -1175,10 +1185,7 @@ int shell_scale_dev(dnsb_ctx *c, double *const u[3], const double *f, int nb) {
     if ((rc = spectrum_of(c, u[comp]))) return rc;
     k_scaleshells<<<RED_BLOCKS, 256, 0, c->stream>>>(g, c->S, f, nb);
     CKL(c);
-    dim3 grid(g.nkx * ((g.nz + c->Ly - 1) / c->Ly));
-    k_yfourier<YF_INVERSE><<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(g, c->S, c->py, c->Ly, c->twy,
-                                                                         c->lam1, c->lam2, c->lam3);
-    CKL(c);
+    if ((rc = launch_yfourier(c, YF_INVERSE))) return rc;
     if ((rc = launch_fftz(c, true))) return rc;
     if ((rc = launch_irfftx(c, ROUT_IMAGES, u[comp]))) return rc;
   }
@@ -1224,10 +1231,7 @@ int shell_clamp_dev(dnsb_ctx *c, double *const u[3], double *E, const double *er
     c->S = Ss[comp];
     k_scaleshells<<<RED_BLOCKS, 256, 0, c->stream>>>(g, c->S, f, nb);
     CKL(c);
-    dim3 grid(g.nkx * ((g.nz + c->Ly - 1) / c->Ly));
-    k_yfourier<YF_INVERSE><<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(g, c->S, c->py, c->Ly, c->twy,
-                                                                         c->lam1, c->lam2, c->lam3);
-    CKL(c);
+    if ((rc = launch_yfourier(c, YF_INVERSE))) return rc;
     if ((rc = launch_fftz(c, true))) return rc;
     if ((rc = launch_irfftx(c, ROUT_IMAGES, u[comp]))) return rc;
   }
@@ -1478,9 +1482,17 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
   c->smem_z = sizeof(double2) * (2 * (size_t)c->Lz * (nz + 1) + nz);
   c->smem_y = sizeof(double2) * (2 * (size_t)c->Ly * ny + ny);
   c->smem_zt = sizeof(double2) * (2 * (size_t)c->Lz * nz + 2 * (size_t)c->Lz * (nz + 1) + nz) + 16;
-  // four-step kernels for the lengths with a register split (DNSB_FFT4=0: off)
+  // four-step kernels for the lengths with a register split (DNSB_FFT4=0: off):
+  // compile-time splits along x and z where there is one, else and along a
+  // periodic y the run-time splits
   if (envint("DNSB_FFT4", 1) != 0) {
     int a = 0, b = 0;
+    c->ax = any_split(M);
+    c->az = any_split(nz);
+    if (!g.wall) c->ay_ = any_split(ny);
+    c->Lx_set = tuned(tun ? tun->lines_x : 0, "DNSB_LX", 0);
+    c->Lz_set = tuned(tun ? tun->lines_z : 0, "DNSB_LZ", 0);
+    c->Ly_set = tuned(tun ? tun->lines_y : 0, "DNSB_LY", 0);
     c->L4z = std::max(1, tuned(tun ? tun->lines_z4 : 0, "DNSB_L4Z", 8));
     c->rx_post = envint("DNSB_RXPOST", c->rx_post) != 0;
     c->ix_pairs = envint("DNSB_IXPAIRS", c->ix_pairs) != 0;
@@ -1517,6 +1529,10 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
     }
     c->mom_planes = std::max(1, std::min(64, mp));
     c->tgrid.z = (nz + c->mom_planes - 1) / c->mom_planes;
+  }
+  if (any_allow(device, c->ax, c->ay_, c->az) != cudaSuccess) {
+    fail(c, DNSB_ECUDA, "shared-memory opt-in of the transform kernels failed");
+    return bail(DNSB_ECUDA);
   }
   if ((c->x1 && (rc = allow_fft4_split(c, c->x1, c->x2))) ||
       (c->z1 && (rc = allow_fft4_split(c, c->z1, c->z2))))
@@ -2229,10 +2245,7 @@ int dnsb_spectrum_sample(dnsb_ctx *c, const double *ux, const double *uy, const 
   for (int comp = 0; comp < 3; comp++) {
     if ((rc = launch_rfftx(c, RIN_FIELD, u[comp], nullptr, nullptr))) return rc;
     if ((rc = launch_fftz(c, false))) return rc;
-    dim3 grid(g.nkx * ((g.nz + c->Ly - 1) / c->Ly));
-    k_yfourier<YF_FORWARD><<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(g, c->S, c->py, c->Ly, c->twy,
-                                                                  c->lam1, c->lam2, c->lam3);
-    CKL(c);
+    if ((rc = launch_yfourier(c, YF_FORWARD))) return rc;
     k_binshells<false><<<RED_BLOCKS, 256, 0, c->stream>>>(g, c->S, E, nbins);
     CKL(c);
   }
@@ -2783,10 +2796,7 @@ int sp_to_phys(dnsb_spectral *p, const double2 *uhc, double *v) {
   SPK(p, cudaMemsetAsync(c->S, 0, sizeof(double2) * (size_t)g.nkx * g.ny * g.nz, c->stream));
   k_sp_scatter<<<RED_BLOCKS, 256, 0, c->stream>>>(p->s, uhc, c->S, n3);
   SPKL(p);
-  dim3 grid(c->nkx_active * ((g.nz + c->Ly - 1) / c->Ly));
-  k_yfourier<YF_INVERSE><<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(g, c->S, c->py, c->Ly, c->twy,
-                                                                       c->lam1, c->lam2, c->lam3);
-  SPKL(p);
+  SPRC(p, launch_yfourier(c, YF_INVERSE));
   SPRC(p, launch_fftz(c, true));
   SPRC(p, launch_irfftx(c, ROUT_REAL, v));
   return 0;
@@ -2798,10 +2808,7 @@ int sp_from_phys(dnsb_spectral *p, const double *r) {
   const Geo &g = c->g;
   SPRC(p, launch_rfftx(c, RIN_REAL, r, nullptr, nullptr));
   SPRC(p, launch_fftz(c, false));
-  dim3 grid(c->nkx_active * ((g.nz + c->Ly - 1) / c->Ly));
-  k_yfourier<YF_FORWARD><<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(g, c->S, c->py, c->Ly, c->twy,
-                                                                       c->lam1, c->lam2, c->lam3);
-  SPKL(p);
+  SPRC(p, launch_yfourier(c, YF_FORWARD));
   return 0;
 }
 
@@ -2810,17 +2817,14 @@ int sp_from_phys(dnsb_spectral *p, const double *r) {
 int sp_from_product(dnsb_spectral *p, const double *va, const double *vb) {
   dnsb_ctx *c = p->c;
   const Geo &g = c->g;
-  if (!c->x1) {
+  if (!c->x1 && !c->ax.tier) {
     k_sp_product<<<RED_BLOCKS, 256, 0, c->stream>>>(sp_n3(p), va, vb, p->r);
     SPKL(p);
     return sp_from_phys(p, p->r);
   }
   SPRC(p, launch_rfftx(c, RIN_PRODUCT, va, vb, nullptr));
   SPRC(p, launch_fftz(c, false));
-  dim3 grid(c->nkx_active * ((g.nz + c->Ly - 1) / c->Ly));
-  k_yfourier<YF_FORWARD><<<grid, SPEC_THREADS, c->smem_y, c->stream>>>(g, c->S, c->py, c->Ly, c->twy,
-                                                                       c->lam1, c->lam2, c->lam3);
-  SPKL(p);
+  SPRC(p, launch_yfourier(c, YF_FORWARD));
   return 0;
 }
 

@@ -19,9 +19,6 @@ namespace dnsb {
 
 constexpr int SPEC_THREADS = 256;
 
-enum RInMode { RIN_DIVERGENCE = 0, RIN_REAL = 1, RIN_FIELD = 2, RIN_PRODUCT = 3 };
-enum ROutMode { ROUT_INTERIOR = 0, ROUT_IMAGES = 1, ROUT_REAL = 2 };
-
 // Real forward FFT along x of L lines (j fixed, kz = k0..k0+L-1) through
 // the half-length complex transform: z[m] = r[2m] + i r[2m+1],
 // X[k] = E[k] + w^k O[k] with E = (Z[k] + conj Z[M-k])/2,
@@ -268,7 +265,6 @@ __global__ void __launch_bounds__(128) k_thomas(Geo g, double2 *__restrict__ S,
 // y, divide by lambda1+lambda2+lambda3 (0 for the mean), inverse, 1/ny.
 // YF_FORWARD leaves the forward transform in S (spectra, shell operations);
 // YF_INVERSE only applies the inverse (with 1/ny).
-enum YFourierMode { YF_SOLVE = 0, YF_FORWARD = 1, YF_INVERSE = 2 };
 template <int YMODE>
 __global__ void __launch_bounds__(SPEC_THREADS, 3) k_yfourier(Geo g, double2 *__restrict__ S,
                                                           FFTPlan plan, int L,

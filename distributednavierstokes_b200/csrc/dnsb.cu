@@ -102,11 +102,9 @@ struct dnsb_ctx {
   int fuse = 1;       // fused projection + momentum between implicit stages
   double *pn = nullptr;  // pressure after stage 1 when fused
   dim3 tgrid, tblock;
-  // z-planes per CTA of the fused projection + momentum: 32 measured 1.5 %
-  // faster than 16 and 64 at 384x256x384 (its prologue projects two planes)
-  int gm_planes = 32;
+  int gm_planes = 32;  // z-planes per CTA of the fused projection + momentum (march_planes)
   std::map<const void *, CUtensorMap> gm_maps;  // TMA maps of the fused kernel's staged fields
-  int mom_planes = MC_Z;  // z planes per CTA of k_momentum_march
+  int mom_planes = 16;  // z planes per CTA of k_momentum_march (march_planes)
   // while a CUDA graph of LES steps is captured: the device word holding
   // the step size, read by the kernels that take dt (else nullptr)
   const double *dtp = nullptr;
@@ -132,6 +130,11 @@ struct dnsb_ctx {
   // the two-barrier k_gradmom_march at 384x256x384
   int gm_pipe = 1;
   dim3 gmgrid;
+  // least cells for the fused kernel in explicit steps: it saves two field
+  // passes of six (256^3 step 2.77 -> 2.70 ms, 192 x 128 x 192 0.847 ->
+  // 0.838), but a stage of fields that stay in L2 is faster as two kernels
+  // with more blocks (128^3 0.441 against 0.450, 64^3 0.116 against 0.121)
+  long long efuse_cells = 4000000;
 
   dim3 cgrid, cblock;  // launch shape of the per-cell step kernels
   // scratch
@@ -696,8 +699,8 @@ int launch_fftz4(dnsb_ctx *c, bool inv) {
   dim3 grid((unsigned)((nlines + c->L4z - 1) / c->L4z));
 #define ZF4(A, B)                                                                                  \
   if (c->z1 == A && c->z2 == B) {                                                                  \
-    if (inv) LAUNCH(c, DNSB_KIND_IFFTZ, k_fftz4<A, B, true><<<grid, F4_THREADS, c->smem_z4, c->stream>>>(g, c->S, c->L4z, c->twz)); \
-    else LAUNCH(c, DNSB_KIND_FFTZ, k_fftz4<A, B, false><<<grid, F4_THREADS, c->smem_z4, c->stream>>>(g, c->S, c->L4z, c->twz)); \
+    if (inv) LAUNCH(c, DNSB_KIND_IFFTZ, CK(c, launch_pdl(k_fftz4<A, B, true>, grid, dim3(F4_THREADS), c->smem_z4, c->stream, g, c->S, c->L4z, c->twz))); \
+    else LAUNCH(c, DNSB_KIND_FFTZ, CK(c, launch_pdl(k_fftz4<A, B, false>, grid, dim3(F4_THREADS), c->smem_z4, c->stream, g, c->S, c->L4z, c->twz))); \
     return 0;                                                                                      \
   }
   FFT4_SPLITS(ZF4)
@@ -753,7 +756,11 @@ int launch_rfftx(dnsb_ctx *c, int mode, const double *a, const double *b, const 
 
 int launch_fftz(dnsb_ctx *c, bool inv) {
   const Geo &g = c->g;
-  if (c->z1 && !c->use_tma) return launch_fftz4(c, inv);
+  // from 128 on the run-time split is the faster (128-thread blocks whose
+  // threads all hold a transform; 256^3 53.9 -> 44.0 us, 384 x 256 x 384 128 ->
+  // 113); shorter lines are bound by latency and keep the constant indices
+  // (64^3: 2.8 us against 3.4)
+  if (c->z1 && !c->use_tma && (g.nz < 128 || !c->az.tier)) return launch_fftz4(c, inv);
   if (c->az.tier && !c->use_tma) {
     LAUNCH(c, inv ? DNSB_KIND_IFFTZ : DNSB_KIND_FFTZ,
            CK(c, any_fftz(g, c->az, c->nkx_active ? c->nkx_active : g.nkx, c->Lz_set, inv, c->S, c->twz, c->stream)));
@@ -799,8 +806,8 @@ int launch_ysolve(dnsb_ctx *c) {
 #define YT(MR)                                                                                    \
   case MR:                                                                                        \
     LAUNCH(c, DNSB_KIND_YSOLVE,                                                                   \
-           k_ythomas<MR><<<grid, block, ythomas_smem(MR), c->stream>>>(g, c->S, c->ycin, c->ay,   \
-                                                        c->by, c->cy, c->lam1, c->lam3));         \
+           CK(c, launch_pdl(k_ythomas<MR>, grid, block, ythomas_smem(MR), c->stream, g, c->S, c->ycin, c->ay,   \
+                                                        c->by, c->cy, c->lam1, c->lam3)));         \
     break;
     switch (ythomas_rows(g.ny)) {
       YT(1) YT(2) YT(3) YT(4) YT(6) YT(8) YT(12) YT(16)
@@ -979,17 +986,35 @@ bool use_tile(const dnsb_ctx *c, const double *ux, const double *uy, const doubl
   return c->mom_tile && aligned16(ux) && aligned16(uy) && aligned16(uz);
 }
 
-void launch_cn(dnsb_ctx *c, Fields3 out, CFields3 V, const double *tab) {
+// z-planes per CTA of a marching kernel on `cols` columns: as many as leave
+// `ctas` CTAs, at most `most`.  More planes amortise the prologue (two or
+// three planes of loads, one or two projections); fewer keep the SMs busy
+// while CTAs end (swept over 1-64 planes on 32^3 ... 384 x 256 x 384).
+//   momentum, 1.7 CTAs per SM, 8 planes: 64^3 9.1 us (16 planes before the
+//     halving rule's 2: 9.7), 128^3 51.8 (16: 61.6), 256^3 324 (16: 335)
+//   fused projection + momentum, 2.6 CTAs per SM, 22 planes: 100 x 75 x 90
+//     38 us (32: 69), 192 x 128 x 192 160 (32: 195), 384 x 256 x 384 1143 (32: 1144)
+int march_planes(long cols, int nz, int most, long ctas) {
+  int p = std::min(nz, most);
+  while (p > 1 && cols * ((nz + p - 1) / p) < ctas) p--;
+  return p;
+}
+
+cudaError_t launch_cn(dnsb_ctx *c, Fields3 out, CFields3 V, const double *tab) {
   const Geo &g = c->g;
   const dim3 grid = cn_grid(g), block(CN_LINES, CN_CHUNKS);
   switch (c->cn_mr) {
-    case 1: k_cn<1><<<grid, block, c->smem_cn, c->stream>>>(g, out, V, tab); break;
-    case 2: k_cn<2><<<grid, block, c->smem_cn, c->stream>>>(g, out, V, tab); break;
-    case 4: k_cn<4><<<grid, block, c->smem_cn, c->stream>>>(g, out, V, tab); break;
-    case 8: k_cn<8><<<grid, block, c->smem_cn, c->stream>>>(g, out, V, tab); break;
-    case 16: k_cn<16><<<grid, block, c->smem_cn, c->stream>>>(g, out, V, tab); break;
-    default: k_cn<32><<<grid, block, c->smem_cn, c->stream>>>(g, out, V, tab); break;
+#define CN_LAUNCH(MR) \
+  case MR: return launch_pdl(k_cn<MR>, grid, block, c->smem_cn, c->stream, g, out, V, tab);
+    CN_ROWS(CN_LAUNCH)
+#undef CN_LAUNCH
+    default: return cudaErrorInvalidValue;  // dnsb_create refuses such ny
   }
+}
+
+void launch_cn_tables(dnsb_ctx *c, double dt, double al0, double al1, double al2) {
+  k_cn_tables<<<6, CN_TABLE_THREADS, cn_table_smem(c->g.ny), c->stream>>>(
+      c->g.ny, c->cn_mr, CN_CHUNKS, c->ycoef, c->ytab, dt, c->g.visc, al0, al1, al2);
 }
 
 int do_step(dnsb_ctx *c, double *ux, double *uy, double *uz, double *p, double *qx, double *qy,
@@ -999,49 +1024,71 @@ int do_step(dnsb_ctx *c, double *ux, double *uy, double *uz, double *p, double *
   // projection + next momentum fused (needs 16-byte aligned planes to stage)
   const bool fused = c->implicit && c->fuse && c->pn && use_tile(c, ux, uy, uz) &&
                      aligned16(delta) && aligned16(p);
+  const bool efused = !c->implicit && c->fuse && (long long)g.nx * g.ny * g.nz >= c->efuse_cells &&
+                      use_tile(c, ux, uy, uz) && aligned16(p);
+  double *const uf[3] = {ux, uy, uz};
   CK(c, cudaMemsetAsync(c->umax, 0, 3 * UMAX_SLOTS * sizeof(unsigned long long), c->stream));
-  if (c->implicit)
-    LAUNCH(c, DNSB_KIND_OTHER,
-           k_cn_tables<<<1, CN_TABLE_THREADS, 0, c->stream>>>(g.ny, c->cn_mr, CN_CHUNKS, c->ycoef, c->ytab, dt,
-                                                g.visc, RK_AL[0], RK_AL[1], RK_AL[2]));
+  // the Crank-Nicolson tables of the three stages: in the first momentum's
+  // extra block layer, or ahead of the per-cell momentum
+  CnTabArgs ct{}, no_ct{};
+  if (c->implicit && use_tile(c, ux, uy, uz))
+    ct = CnTabArgs{c->ytab, c->ycoef, c->cn_mr, {RK_AL[0], RK_AL[1], RK_AL[2]}};
+  else if (c->implicit)
+    LAUNCH(c, DNSB_KIND_OTHER, launch_cn_tables(c, dt, RK_AL[0], RK_AL[1], RK_AL[2]));
   for (int s = 0; s < 3; s++) {
     const double A = RK_A[s], B = RK_B[s], al = RK_AL[s];
     const int readq = A != 0.0;
     unsigned long long *um = s == 2 ? c->umax : nullptr;
     if (!c->implicit) {
-      if (use_tile(c, ux, uy, uz))
+      // W of this stage: the context's fields, except that with the fused
+      // projection + momentum stage 2's lies in u (whose projected values of
+      // stages 1 and 2 are never stored)
+      double *const *W = efused && s == 1 ? uf : c->W, *const *Wn = s == 0 ? uf : c->W;
+      if (s > 0 && efused) {
+        // the momentum of this stage ran inside the previous stage's projection
+      } else if (use_tile(c, ux, uy, uz))
         LAUNCH(c, DNSB_KIND_MOMENTUM,
-               k_momentum_march<MOM_EXPLICIT><<<c->tgrid, c->tblock, 0, c->stream>>>(
-                   g, ff(qx, qy, qz), cf(ux, uy, uz), ff(c->W[0], c->W[1], c->W[2]), nullptr, A,
-                   dt, B, 0.0, readq, c->ymet, 0.0, c->mom_planes, c->dtp));
+               CK(c, launch_pdl(k_momentum_march<MOM_EXPLICIT>, c->tgrid, c->tblock, 0, c->stream, g,
+                                ff(qx, qy, qz), cf(ux, uy, uz), ff(W[0], W[1], W[2]), nullptr, A, dt, B,
+                                0.0, readq, c->ymet, 0.0, c->mom_planes, c->dtp, no_ct)));
       else
         LAUNCH(c, DNSB_KIND_MOMENTUM,
                k_momentum<MOM_EXPLICIT><<<c->cgrid, c->cblock, 0, c->stream>>>(
-                   g, ff(qx, qy, qz), cf(ux, uy, uz), ff(c->W[0], c->W[1], c->W[2]), nullptr, A,
-                   dt, B, 0.0, readq, c->ymet, 0.0));
-      if ((rc = launch_rfftx(c, RIN_DIVERGENCE, c->W[0], c->W[1], c->W[2]))) return rc;
+                   g, ff(qx, qy, qz), cf(ux, uy, uz), ff(W[0], W[1], W[2]), nullptr, A, dt, B, 0.0, readq,
+                   c->ymet, 0.0));
+      if ((rc = launch_rfftx(c, RIN_DIVERGENCE, W[0], W[1], W[2]))) return rc;
       if ((rc = poisson_from_spectrum(c, ROUT_IMAGES, p))) return rc;
-      LAUNCH(c, DNSB_KIND_GRAD,
-             k_grad<GRAD_EXPLICIT><<<c->cgrid, c->cblock, 0, c->stream>>>(
-                 g, ff(ux, uy, uz), cf(c->W[0], c->W[1], c->W[2]), p, nullptr, 0.0, um));
+      if (s < 2 && efused)
+        LAUNCH(c, DNSB_KIND_GRADMOM,
+               CK(c, launch_pdl(k_gradmom_pipe<MOM_EXPLICIT>, c->gmgrid, c->tblock, GRADMOM_PIPE_SMEM_EXPLICIT,
+                                c->stream, g, c->gm_planes, cf(W[0], W[1], W[2]), p, nullptr, nullptr, 0.0,
+                                ff(qx, qy, qz), ff(Wn[0], Wn[1], Wn[2]), RK_A[s + 1], dt, RK_B[s + 1], 0.0,
+                                c->ymet, 0.0, c->dtp)));
+      else
+        LAUNCH(c, DNSB_KIND_GRAD,
+               CK(c, launch_pdl(k_grad<GRAD_EXPLICIT>, c->cgrid, c->cblock, 0, c->stream, g, ff(ux, uy, uz),
+                                cf(W[0], W[1], W[2]), p, nullptr, 0.0, um)));
     } else {
       const double adt = al * dt;
       const double th = al * dt * g.visc / 2;
       if (s > 0 && fused) {
         // the momentum of this stage ran inside the previous stage's projection
-      } else if (use_tile(c, ux, uy, uz))
+      } else if (use_tile(c, ux, uy, uz)) {
+        dim3 grid = c->tgrid;
+        if (s == 0) grid.z++;
         LAUNCH(c, DNSB_KIND_MOMENTUM,
-               k_momentum_march<MOM_IMPLICIT><<<c->tgrid, c->tblock, 0, c->stream>>>(
-                   g, ff(qx, qy, qz), cf(ux, uy, uz), ff(c->V[0], c->V[1], c->V[2]), p, A, dt, B,
-                   adt, readq, c->ymet, th, c->mom_planes, c->dtp));
-      else
+               CK(c, launch_pdl(k_momentum_march<MOM_IMPLICIT>, grid, c->tblock, 0, c->stream, g,
+                                      ff(qx, qy, qz), cf(ux, uy, uz), ff(c->V[0], c->V[1], c->V[2]), p, A,
+                                      dt, B, adt, readq, c->ymet, th, c->mom_planes, c->dtp,
+                                      s == 0 ? ct : no_ct)));
+      } else
         LAUNCH(c, DNSB_KIND_MOMENTUM,
                k_momentum<MOM_IMPLICIT><<<c->cgrid, c->cblock, 0, c->stream>>>(
                    g, ff(qx, qy, qz), cf(ux, uy, uz), ff(c->V[0], c->V[1], c->V[2]), p, A, dt, B,
                    adt, readq, c->ymet, th));
       LAUNCH(c, DNSB_KIND_CN,
-             launch_cn(c, ff(ux, uy, uz), cf(c->V[0], c->V[1], c->V[2]),
-                       c->ytab + (long long)s * 2 * cn_tab_stride(g.ny)));
+             CK(c, launch_cn(c, ff(ux, uy, uz), cf(c->V[0], c->V[1], c->V[2]),
+                             c->ytab + (long long)s * 2 * cn_tab_stride(g.ny))));
       if ((rc = launch_rfftx(c, RIN_DIVERGENCE, ux, uy, uz))) return rc;
       if ((rc = poisson_from_spectrum(c, ROUT_IMAGES, delta))) return rc;
       if (s < 2 && fused) {
@@ -1058,18 +1105,23 @@ int do_step(dnsb_ctx *c, double *ux, double *uy, double *uz, double *p, double *
                      pin, pout, 1.0 / adt, ff(qx, qy, qz), ff(c->V[0], c->V[1], c->V[2]), A1, dt, B1,
                      al1 * dt, c->ymet, al1 * dt * g.visc / 2, c->deverr, c->wait_limit));
         else
+        if (c->gm_pipe == 1 || c->gm_pipe == 3)
+          LAUNCH(c, DNSB_KIND_GRADMOM,
+                 CK(c, launch_pdl(k_gradmom_pipe<MOM_IMPLICIT>, c->gmgrid, c->tblock, GRADMOM_PIPE_SMEM, c->stream, g,
+                                        c->gm_planes, cf(ux, uy, uz), delta, pin, pout, 1.0 / adt,
+                                        ff(qx, qy, qz), ff(c->V[0], c->V[1], c->V[2]), A1, dt, B1, al1 * dt,
+                                        c->ymet, al1 * dt * g.visc / 2, nullptr)));
+        else
         LAUNCH(c, DNSB_KIND_GRADMOM,
-               (c->gm_pipe == 2 ? k_gradmom_deep : c->gm_pipe ? k_gradmom_pipe : k_gradmom_march)<<<
-                   c->gmgrid, c->tblock,
-                   c->gm_pipe == 2 ? GRADMOM_DEEP_SMEM : c->gm_pipe ? GRADMOM_PIPE_SMEM : GRADMOM_SMEM,
+               (c->gm_pipe == 2 ? k_gradmom_deep : k_gradmom_march)<<<
+                   c->gmgrid, c->tblock, c->gm_pipe == 2 ? GRADMOM_DEEP_SMEM : GRADMOM_SMEM,
                    c->stream>>>(
                    g, c->gm_planes, cf(ux, uy, uz), delta, pin, pout, 1.0 / adt, ff(qx, qy, qz),
                    ff(c->V[0], c->V[1], c->V[2]), A1, dt, B1, al1 * dt, c->ymet,
                    al1 * dt * g.visc / 2));
       } else {
         LAUNCH(c, DNSB_KIND_GRAD,
-               k_grad<GRAD_IMPLICIT><<<c->cgrid, c->cblock, 0, c->stream>>>(
-                   g, ff(ux, uy, uz), cf(ux, uy, uz), delta, p, 1.0 / adt, um));
+               CK(c, launch_pdl(k_grad<GRAD_IMPLICIT>, c->cgrid, c->cblock, 0, c->stream, g, ff(ux, uy, uz), cf(ux, uy, uz), delta, p, 1.0 / adt, um)));
       }
     }
   }
@@ -1085,8 +1137,7 @@ int do_project(dnsb_ctx *c, double *ux, double *uy, double *uz, double *psi) {
   if ((rc = launch_rfftx(c, RIN_DIVERGENCE, ux, uy, uz))) return rc;
   if ((rc = poisson_from_spectrum(c, ROUT_IMAGES, psi))) return rc;
   LAUNCH(c, DNSB_KIND_GRAD,
-         k_grad<GRAD_EXPLICIT><<<c->cgrid, c->cblock, 0, c->stream>>>(
-             g, ff(ux, uy, uz), cf(ux, uy, uz), psi, nullptr, 0.0, nullptr));
+         CK(c, launch_pdl(k_grad<GRAD_EXPLICIT>, c->cgrid, c->cblock, 0, c->stream, g, ff(ux, uy, uz), cf(ux, uy, uz), psi, nullptr, 0.0, nullptr)));
   c->umax_for[0] = c->umax_for[1] = c->umax_for[2] = nullptr;
   return 0;
 }
@@ -1436,17 +1487,18 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
       (rc = upload(c, &c->twy, twy)))
     return bail(rc);
   if ((rc = dalloc(c, &c->ytab, 6 * (size_t)cn_tab_stride(ny)))) return bail(rc);
-  c->cn_mr = 1;
-  while (c->cn_mr * CN_CHUNKS < ny) c->cn_mr *= 2;
-  c->smem_cn = sizeof(double) * (5 * (size_t)cn_skew_pitch(ny, c->cn_mr) + 2 * CN_CHUNKS + 2 * CN_CHUNKS * CN_LINES);
-  if (c->implicit && c->cn_mr > 32) {
+  c->cn_mr = cn_rows(ny);
+  if (c->implicit && !c->cn_mr) {
     fail(c, DNSB_EUNSUP, "semi-implicit y-diffusion supports ny <= %d", 32 * CN_CHUNKS);
     return bail(DNSB_EUNSUP);
   }
-  if ((rc = allow_smem(c, k_cn<1>, c->smem_cn)) || (rc = allow_smem(c, k_cn<2>, c->smem_cn)) ||
-      (rc = allow_smem(c, k_cn<4>, c->smem_cn)) || (rc = allow_smem(c, k_cn<8>, c->smem_cn)) ||
-      (rc = allow_smem(c, k_cn<16>, c->smem_cn)) || (rc = allow_smem(c, k_cn<32>, c->smem_cn)))
-    return bail(rc);
+  c->smem_cn = c->cn_mr ? sizeof(double) * (5 * (size_t)cn_skew_pitch(ny, c->cn_mr) + 2 * CN_CHUNKS +
+                                            2 * CN_CHUNKS * CN_LINES)
+                        : 0;
+#define CN_ALLOW(MR) \
+  if (c->cn_mr == MR && (rc = allow_smem(c, k_cn<MR>, c->smem_cn))) return bail(rc);
+  CN_ROWS(CN_ALLOW)
+#undef CN_ALLOW
 
   // launch shapes: L lines per CTA, two line buffers each within ~100 KB;
   // DNSB_LX / DNSB_LZ / DNSB_LY / DNSB_CELL_BLOCK ("32x8") override them
@@ -1471,11 +1523,10 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
     c->cgrid = dim3((nx + bx - 1) / bx, (ny + by - 1) / by, nz);
     c->mom_tile = envint("DNSB_MOMTILE", 1) != 0;
     c->fuse = envint("DNSB_FUSE", 1) != 0;
+    c->efuse_cells = envint("DNSB_EFUSE", 4000000);
     c->tblock = dim3(MC_X, MC_Y, 1);
-    c->tgrid = dim3((nx + MC_X - 1) / MC_X, (ny + MC_Y - 1) / MC_Y, (nz + MC_Z - 1) / MC_Z);
-    c->gm_planes = std::max(4, std::min(256, tuned(tun ? tun->gm_planes : 0, "DNSB_GMZ", c->gm_planes)));
+    c->tgrid = dim3((nx + MC_X - 1) / MC_X, (ny + MC_Y - 1) / MC_Y, nz);
     c->gm_pipe = std::max(0, std::min(3, envint("DNSB_GMPIPE", c->gm_pipe)));
-    c->gmgrid = dim3(c->tgrid.x, c->tgrid.y, (nz + c->gm_planes - 1) / c->gm_planes);
   }
   c->smem_rx = sizeof(double2) * (2 * (size_t)c->Lx * (M + 1) + M + (M + 1));
   c->smem_ix = sizeof(double2) * (2 * (size_t)c->Lx * (M + 2) + M + (M + 1));
@@ -1519,15 +1570,11 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
       c->nsm = nsm;
   }
   {
-    // planes per momentum CTA: MC_Z, halved while the grid would give
-    // fewer than two CTAs per SM (small boxes), DNSB_MOMZ overrides
     const long cols = (long)c->tgrid.x * c->tgrid.y;
-    int mp = envint("DNSB_MOMZ", 0);
-    if (mp <= 0) {
-      mp = MC_Z;
-      while (mp > 2 && cols * ((nz + mp - 1) / mp) < 2L * c->nsm) mp /= 2;
-    }
-    c->mom_planes = std::max(1, std::min(64, mp));
+    const int mp = envint("DNSB_MOMZ", 0), gp = tuned(tun ? tun->gm_planes : 0, "DNSB_GMZ", 0);
+    c->mom_planes = std::max(1, std::min(64, mp > 0 ? mp : march_planes(cols, nz, 8, c->nsm * 17L / 10)));
+    c->gm_planes = std::max(gp > 0 ? 4 : 1, std::min(256, gp > 0 ? gp : march_planes(cols, nz, 22, c->nsm * 257L / 100)));
+    c->gmgrid = dim3(c->tgrid.x, c->tgrid.y, (nz + c->gm_planes - 1) / c->gm_planes);
     c->tgrid.z = (nz + c->mom_planes - 1) / c->mom_planes;
   }
   if (any_allow(device, c->ax, c->ay_, c->az) != cudaSuccess) {
@@ -1592,10 +1639,12 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
       if ((rc = dalloc(c, &c->V[i], G))) return bail(rc);
     }
   }
+  if (!c->implicit && (rc = allow_smem(c, k_gradmom_pipe<MOM_EXPLICIT>, GRADMOM_PIPE_SMEM_EXPLICIT)))
+    return bail(rc);
   if (c->implicit && c->fuse) {
     if ((rc = dalloc(c, &c->pn, G))) return bail(rc);
     if ((rc = allow_smem(c, k_gradmom_march, GRADMOM_SMEM)) ||
-        (rc = allow_smem(c, k_gradmom_pipe, GRADMOM_PIPE_SMEM)) ||
+        (rc = allow_smem(c, k_gradmom_pipe<MOM_IMPLICIT>, GRADMOM_PIPE_SMEM)) ||
         (rc = allow_smem(c, k_gradmom_tma, GRADMOM_TMA_SMEM)) ||
         (rc = allow_smem(c, k_gradmom_deep, GRADMOM_DEEP_SMEM)))
       return bail(rc);
@@ -1686,9 +1735,9 @@ int dnsb_momentum(dnsb_ctx *c, double *qx, double *qy, double *qz, const double 
     return c ? fail(c, DNSB_EINVAL, "null field") : DNSB_EINVAL;
   if (ensure_device(c)) return DNSB_ECUDA;
   if (use_tile(c, ux, uy, uz))
-    k_momentum_march<MOM_ONLY><<<c->tgrid, c->tblock, 0, c->stream>>>(
-        c->g, ff(qx, qy, qz), cf(ux, uy, uz), ff(nullptr, nullptr, nullptr), nullptr, A, dt, 0.0,
-        0.0, 1, c->ymet, 0.0, c->mom_planes, c->dtp);
+    CK(c, launch_pdl(k_momentum_march<MOM_ONLY>, c->tgrid, c->tblock, 0, c->stream, c->g, ff(qx, qy, qz),
+                     cf(ux, uy, uz), ff(nullptr, nullptr, nullptr), nullptr, A, dt, 0.0, 0.0, 1, c->ymet, 0.0,
+                     c->mom_planes, c->dtp, CnTabArgs{}));
   else
     k_momentum<MOM_ONLY><<<cell_grid(c->g), cell_block, 0, c->stream>>>(
         c->g, ff(qx, qy, qz), cf(ux, uy, uz), ff(nullptr, nullptr, nullptr), nullptr, A, dt, 0.0,
@@ -2146,11 +2195,9 @@ int dnsb_imex_update(dnsb_ctx *c, double *ux, double *uy, double *uz, const doub
       g, ff(c->V[0], c->V[1], c->V[2]), cf(ux, uy, uz), cf(qx, qy, qz), p, B, adt, c->ymet, th);
   CKL(c);
   // tables for this alpha in stage slot 0
-  k_cn_tables<<<1, CN_TABLE_THREADS, 0, c->stream>>>(g.ny, c->cn_mr, CN_CHUNKS, c->ycoef, c->ytab, dt, g.visc,
-                                       alpha, alpha, alpha);
+  launch_cn_tables(c, dt, alpha, alpha, alpha);
   CKL(c);
-  launch_cn(c, ff(ux, uy, uz), cf(c->V[0], c->V[1], c->V[2]), c->ytab);
-  CKL(c);
+  CK(c, launch_cn(c, ff(ux, uy, uz), cf(c->V[0], c->V[1], c->V[2]), c->ytab));
   c->umax_for[0] = c->umax_for[1] = c->umax_for[2] = nullptr;
   return 0;
 }

@@ -32,7 +32,8 @@ int threads_for(int items) { return std::min(FA_THREADS, std::max(32, (items + 3
 // throughput, is what their transforms cost), and within shared memory.
 int lines_for(const AnySplit &sp, int asked, long long lines, int least, size_t bytes_per_line, size_t fixed) {
   int L = asked > 0 ? asked : std::max(least, FA_THREADS / std::max(sp.n1, sp.n2));
-  while (asked <= 0 && L > least && (lines + L - 1) / L < 2 * 148) L = std::max(least, L / 2);
+  while (asked <= 0 && L > least && (lines + L - 1) / L < 2 * 148 && L / 2 * std::max(sp.n1, sp.n2) >= 64)
+    L = std::max(least, L / 2);
   while (L > 1 && fixed + L * bytes_per_line > kSmemPerBlock) L--;
   return L;
 }
@@ -130,7 +131,7 @@ cudaError_t any_fftz(const Geo &g, const AnySplit &sp, int nkx, int lines, bool 
   const dim3 grid((unsigned)((nlines + L - 1) / L)), block(threads_for(L * std::max(sp.n1, sp.n2)));
   return by_tier(sp.tier, [&](auto t) {
     constexpr int T = decltype(t)::value;
-    return launch_dependent(inv ? k_fftz_any<T, true> : k_fftz_any<T, false>, grid, block,
+    return launch_pdl(inv ? k_fftz_any<T, true> : k_fftz_any<T, false>, grid, block,
                             smem_z(sp, L), stream, g.nz, sp.n1, sp.n2, L, nlines, S, twz);
   });
 }
@@ -143,7 +144,7 @@ cudaError_t any_y(const Geo &g, const AnySplit &sp, int nkx, int lines, int mode
     constexpr int T = decltype(t)::value;
     auto k = mode == YF_SOLVE ? k_y_any<T, YF_SOLVE>
              : mode == YF_FORWARD ? k_y_any<T, YF_FORWARD> : k_y_any<T, YF_INVERSE>;
-    return launch_dependent(k, grid, block, smem_y(sp, L), stream, g, sp.n1, sp.n2, L, S, twy, lam1,
+    return launch_pdl(k, grid, block, smem_y(sp, L), stream, g, sp.n1, sp.n2, L, S, twy, lam1,
                             lam2, lam3);
   });
 }
@@ -160,7 +161,7 @@ cudaError_t any_rfftx(const Geo &g, const AnySplit &sp, int lines, int mode, dou
              : mode == RIN_REAL     ? k_rfftx_any<T, RIN_REAL>
              : mode == RIN_FIELD    ? k_rfftx_any<T, RIN_FIELD>
                                     : k_rfftx_any<T, RIN_PRODUCT>;
-    return launch_dependent(k, grid, dim3(FA_THREADS), smem_x(sp, L), stream, g, sp.n1, sp.n2, L, S, a,
+    return launch_pdl(k, grid, dim3(FA_THREADS), smem_x(sp, L), stream, g, sp.n1, sp.n2, L, S, a,
                             b, c, twM, twN);
   });
 }
@@ -174,7 +175,7 @@ cudaError_t any_irfftx(const Geo &g, const AnySplit &sp, int lines, int mode, co
     auto k = mode == ROUT_INTERIOR ? k_irfftx_any<T, ROUT_INTERIOR>
              : mode == ROUT_IMAGES ? k_irfftx_any<T, ROUT_IMAGES>
                                    : k_irfftx_any<T, ROUT_REAL>;
-    return launch_dependent(k, grid, dim3(FA_THREADS), smem_x(sp, L), stream, g, sp.n1, sp.n2, L, S,
+    return launch_pdl(k, grid, dim3(FA_THREADS), smem_x(sp, L), stream, g, sp.n1, sp.n2, L, S,
                             out, twM, twN);
   });
 }

@@ -43,6 +43,26 @@ constexpr int FA_THREADS = 128;
 __host__ __device__ constexpr int fa_blocks(int tier) { return tier <= 10 ? 6 : tier <= 16 ? 4 : 3; }
 __host__ __device__ constexpr int fa_pitch(int n2) { return n2 | 1; }
 
+// t = tid, tid + nth, ... as (t / n, t % n) with one division for the loop
+// (n is a run-time value: a division per element cost as much as its loads)
+struct FaWalk {
+  int q, r, n, dq, dr;
+  __device__ __forceinline__ FaWalk(int n_) : n(n_) {
+    q = threadIdx.x / n;
+    r = threadIdx.x - q * n;
+    dq = blockDim.x / n;
+    dr = blockDim.x - dq * n;
+  }
+  __device__ __forceinline__ void next() {
+    q += dq;
+    r += dr;
+    if (r >= n) {
+      r -= n;
+      q++;
+    }
+  }
+};
+
 // f(integral_constant<r>) for the register size r
 template <int TIER, class F>
 __device__ __forceinline__ void fa_dispatch(int r, F f) {
@@ -104,14 +124,14 @@ __device__ __forceinline__ void fa_step2(int N1, int N2, int P, int LS, int L, c
 template <int TIER, bool INV>
 __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
     k_fftz_any(int n, int N1, int N2, int L, long long nlines, double2 *__restrict__ S,
-               const double2 *__restrict__ twz) {
+               const double2 *__restrict__ twz, int dep) {
   extern __shared__ double2 smem[];
   const int P = fa_pitch(N2), LS = N1 * P;
   double2 *buf = smem, *tw = smem + L * LS;
-  pdl_trigger();
+  pdl_trigger(dep);
   for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twz[t];
   __syncthreads();
-  pdl_wait();
+  pdl_wait(dep);
   const long long l0 = (long long)blockIdx.x * L;
   const int Lv = (int)min((long long)L, nlines - l0);
   double2 *src = S + l0 * n;
@@ -134,16 +154,17 @@ template <int TIER, int YMODE>
 __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
     k_y_any(Geo g, int N1, int N2, int L, double2 *__restrict__ S, const double2 *__restrict__ twy,
             const double *__restrict__ lam1, const double *__restrict__ lam2,
-            const double *__restrict__ lam3) {
+            const double *__restrict__ lam3, int dep) {
   extern __shared__ double2 smem[];
   const int n = g.ny;
   double2 *buf = smem, *tw = smem + L * n;  // buf[(k1 N2 + j2) L + l]
   const int ngrp = (g.nz + L - 1) / L;
-  const int kx = blockIdx.x / ngrp, k0 = (blockIdx.x - kx * ngrp) * L;
-  pdl_trigger();
+  const int bid = gridDim.x - 1 - blockIdx.x;  // last kx plane first: still in L2 from the z-transform
+  const int kx = bid / ngrp, k0 = (bid - kx * ngrp) * L;
+  pdl_trigger(dep);
   for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twy[t];
   __syncthreads();
-  pdl_wait();
+  pdl_wait(dep);
   constexpr bool INV = YMODE == YF_INVERSE;
   const double sc = YMODE == YF_FORWARD ? 1.0 : 1.0 / n;
   double2 *line0 = S + sidx(g, kx, 0, k0);
@@ -223,57 +244,64 @@ template <int TIER, int INMODE>
 __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
     k_rfftx_any(Geo g, int N1, int N2, int L, double2 *__restrict__ S, const double *in0,
                 const double *in1, const double *in2,
-                const double2 *__restrict__ twM, const double2 *__restrict__ twN) {
+                const double2 *__restrict__ twM, const double2 *__restrict__ twN, int dep) {
   extern __shared__ double2 smem[];
   const int M = N1 * N2, ls = M + 1, P = fa_pitch(N2), LS = N1 * P;
   double2 *buf = smem, *res = buf + L * LS, *tw = res + L * ls, *tn = tw + M;
   const int ngrp = (g.nz + L - 1) / L;
   const int j = blockIdx.x / ngrp, k0 = (blockIdx.x - j * ngrp) * L;
   const int Lv = min(L, g.nz - k0);
-  pdl_trigger();
+  pdl_trigger(dep);
   for (int t = threadIdx.x; t < M; t += blockDim.x) tw[t] = twM[t];
   for (int t = threadIdx.x; t <= M; t += blockDim.x) tn[t] = twN[t];
   const long long sy = g.NX, sz = (long long)g.NX * g.NY;
   const int J = j + 1;
   const double rdyJ = __ldg(g.rdy + J);
-  pdl_wait();
-  batched_copy<4>(
-      Lv * M,
-      [&](int t) {
-        const int l = t / M, m = t - l * M;
-        const int k = k0 + l;
-        if constexpr (INMODE == RIN_REAL || INMODE == RIN_PRODUCT) {
-          const long long ro = (long long)g.nx * (j + (long long)g.ny * k);
-          double2 z = *reinterpret_cast<const double2 *>(in0 + ro + 2 * m);
-          if constexpr (INMODE == RIN_PRODUCT) {
-            const double2 w = *reinterpret_cast<const double2 *>(in1 + ro + 2 * m);
-            z = make_double2(z.x * w.x, z.y * w.y);
-          }
-          return z;
-        } else {
-          const int c0 = gidx(g, 2 * m + 1, J, k + 1);
-          if constexpr (INMODE == RIN_FIELD) return make_double2(in0[c0], in0[c0 + 1]);
-          const double a0 = in0[c0 - 1], a1 = in0[c0], a2 = in0[c0 + 1];
-          const double b0 = in1[c0], b1 = in1[c0 - sy];
-          const double b2 = in1[c0 + 1], b3 = in1[c0 + 1 - sy];
-          const double d0 = in2[c0], d1 = in2[c0 - sz];
-          const double d2 = in2[c0 + 1], d3 = in2[c0 + 1 - sz];
-          return make_double2((a1 - a0) * g.rdx + (b0 - b1) * rdyJ + (d0 - d1) * g.rdz,
-                              (a2 - a1) * g.rdx + (b2 - b3) * rdyJ + (d2 - d3) * g.rdz);
-        }
-      },
-      [&](int t, double2 z) {
-        const int l = t / M, m = t - l * M;
-        res[l * ls + m] = z;
-      });
+  pdl_wait(dep);
+  auto load = [&](int l, int m) {
+    const int k = k0 + l;
+    if constexpr (INMODE == RIN_REAL || INMODE == RIN_PRODUCT) {
+      const long long ro = (long long)g.nx * (j + (long long)g.ny * k);
+      double2 z = *reinterpret_cast<const double2 *>(in0 + ro + 2 * m);
+      if constexpr (INMODE == RIN_PRODUCT) {
+        const double2 w = *reinterpret_cast<const double2 *>(in1 + ro + 2 * m);
+        z = make_double2(z.x * w.x, z.y * w.y);
+      }
+      return z;
+    } else {
+      const int c0 = gidx(g, 2 * m + 1, J, k + 1);
+      if constexpr (INMODE == RIN_FIELD) return make_double2(in0[c0], in0[c0 + 1]);
+      const double a0 = in0[c0 - 1], a1 = in0[c0], a2 = in0[c0 + 1];
+      const double b0 = in1[c0], b1 = in1[c0 - sy];
+      const double b2 = in1[c0 + 1], b3 = in1[c0 + 1 - sy];
+      const double d0 = in2[c0], d1 = in2[c0 - sz];
+      const double d2 = in2[c0 + 1], d3 = in2[c0 + 1 - sz];
+      return make_double2((a1 - a0) * g.rdx + (b0 - b1) * rdyJ + (d0 - d1) * g.rdz,
+                          (a2 - a1) * g.rdx + (b2 - b3) * rdyJ + (d2 - d3) * g.rdz);
+    }
+  };
+  constexpr int B = 4;  // values in flight per thread
+  for (FaWalk w(M); w.q < Lv;) {
+    double2 z[B];
+    int o[B];
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      o[u] = w.q < Lv ? w.q * ls + w.r : -1;
+      if (o[u] >= 0) z[u] = load(w.q, w.r);
+      w.next();
+    }
+#pragma unroll
+    for (int u = 0; u < B; u++)
+      if (o[u] >= 0) res[o[u]] = z[u];
+  }
   __syncthreads();
   fa_step1<TIER, false>(N1, N2, P, LS, Lv, tw, buf, [&](int l, int m) { return res[l * ls + m]; });
   __syncthreads();
   fa_step2<TIER, false>(N1, N2, P, LS, Lv, tw, buf,
                         [&](int l, int e, double2 v) { res[l * ls + e] = v; });
   __syncthreads();
-  for (int t = threadIdx.x; t < L * (M + 1); t += blockDim.x) {
-    const int kx = t / L, l = t - kx * L;
+  for (FaWalk w(L); w.q <= M; w.next()) {
+    const int kx = w.q, l = w.r;
     if (l >= Lv) continue;
     const double2 zk = res[l * ls + (kx == M ? 0 : kx)];
     const double2 zc = cconj(res[l * ls + (kx == 0 ? 0 : M - kx)]);
@@ -289,37 +317,38 @@ __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
 template <int TIER, int OUTMODE>
 __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
     k_irfftx_any(Geo g, int N1, int N2, int L, const double2 *S, double *__restrict__ out,
-                 const double2 *__restrict__ twM, const double2 *__restrict__ twN) {
+                 const double2 *__restrict__ twM, const double2 *__restrict__ twN, int dep) {
   extern __shared__ double2 smem[];
   const int M = N1 * N2, ls = M + 1, P = fa_pitch(N2), LS = N1 * P;
   double2 *buf = smem, *zb = buf + L * LS, *tw = zb + L * ls, *tn = tw + M;
   const int ngrp = (g.nz + L - 1) / L;
   const int j = blockIdx.x / ngrp, k0 = (blockIdx.x - j * ngrp) * L;
   const int Lv = min(L, g.nz - k0);
-  pdl_trigger();
+  pdl_trigger(dep);
   for (int t = threadIdx.x; t < M; t += blockDim.x) tw[t] = twM[t];
   for (int t = threadIdx.x; t <= M; t += blockDim.x) tn[t] = twN[t];
   __syncthreads();
-  pdl_wait();
+  pdl_wait(dep);
   // Z[k] = E + i O, E = (X[k] + conj X[M-k])/2, O = (X[k] - conj X[M-k]) conj(w^k)/2
   const int half = M / 2 + 1;
   const double2 *src = S + sidx(g, 0, j, k0);
   const long long skx = (long long)g.nz * g.ny;
   constexpr int B = 4;  // pairs in flight per thread
-  for (int base = threadIdx.x; base < L * half; base += B * blockDim.x) {
+  for (FaWalk w(L); w.q < half;) {
     double2 a[B], b[B];
+    FaWalk v = w;
 #pragma unroll
     for (int u = 0; u < B; u++) {
-      const int t = base + u * blockDim.x, k = t / L, l = t - k * L;
       a[u] = b[u] = make_double2(0.0, 0.0);
-      if (k < half && l < Lv) {
-        a[u] = src[k * skx + l];
-        b[u] = src[(M - k) * skx + l];
+      if (w.q < half && w.r < Lv) {
+        a[u] = src[w.q * skx + w.r];
+        b[u] = src[(M - w.q) * skx + w.r];
       }
+      w.next();
     }
 #pragma unroll
-    for (int u = 0; u < B; u++) {
-      const int t = base + u * blockDim.x, k = t / L, l = t - k * L;
+    for (int u = 0; u < B; u++, v.next()) {
+      const int k = v.q, l = v.r;
       if (k >= half || l >= Lv) continue;
       double2 *Z = zb + l * ls;
       if (k == 0) {
@@ -347,8 +376,8 @@ __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
   fa_step2<TIER, true>(N1, N2, P, LS, Lv, tw, buf,
                        [&](int l, int m, double2 z) { zb[l * ls + m] = cscale(z, sc); });
   __syncthreads();
-  for (int t = threadIdx.x; t < Lv * M; t += blockDim.x) {
-    const int l = t / M, m = t - l * M;
+  for (FaWalk w(M); w.q < Lv; w.next()) {
+    const int l = w.q, m = w.r;
     const double2 z = zb[l * ls + m];
     const int K = k0 + l + 1;
     if constexpr (OUTMODE == ROUT_REAL) {

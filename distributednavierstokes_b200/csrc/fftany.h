@@ -16,8 +16,7 @@ AnySplit any_split(int n);
 // opt in to the shared memory of the kernels of one split
 cudaError_t any_allow(int device, const AnySplit &x, const AnySplit &y, const AnySplit &z);
 
-// Each returns the launch's status; the grids are programmatic dependents of
-// the stream's previous kernel.  nkx: kx planes transformed; lines: lines per
+// Each returns the launch's status; the launches are launch_pdl's.  nkx: kx planes transformed; lines: lines per
 // block (0: the launch's own rule).
 cudaError_t any_fftz(const Geo &g, const AnySplit &sp, int nkx, int lines, bool inv, double2 *S,
                      const double2 *twz, cudaStream_t stream);

@@ -1,5 +1,5 @@
-// gradmom.cuh -- the projection of one semi-implicit RK3 stage fused with
-// the momentum of the next.
+// gradmom.cuh -- the projection of one RK3 stage fused with the momentum of
+// the next (semi-implicit; explicit in k_gradmom_pipe).
 //
 // Between stages s and s+1 of step! (src/timestep.jl:41-63) with implicit
 // y-diffusion, the reference runs
@@ -235,15 +235,19 @@ constexpr size_t GRADMOM_SMEM = sizeof(double) * (2 * 3 + 3 + 4 + 3 * 3) * GP_N;
 // u_z east and north) are the ones this thread read as plane K's centre in
 // the previous iteration and stay in registers.  Ring slots: u* 2, p 3,
 // delta 5, projected u 3 (x 3 components).
+// MOM_EXPLICIT: the same fusion for explicit stages (u = W - grad psi with
+// psi = delta, next W' = u + B q with ghost images into `out`, which must not
+// alias us): no pressure is staged or written.
+template <int MODE>
 __global__ void __launch_bounds__(MC_X *MC_Y, 3)
-    k_gradmom_pipe(Geo g, int planes, CFields3 us, const double *__restrict__ delta,
-                   const double *__restrict__ p_in, double *__restrict__ p_out, double radt,
+    k_gradmom_pipe(Geo g, int planes, CFields3 us, const double *delta,
+                   const double *p_in, double *__restrict__ p_out, double radt,
                    Fields3 q, Fields3 out, double A, double dt, double B, double adt,
-                   const double2 *__restrict__ ymet, double theta) {
+                   const double2 *__restrict__ ymet, double theta, const double *dtp, int dep) {
   extern __shared__ __align__(16) double gsm[];
   double *ustar = gsm;                    // [2 slots][3][GP_N]
-  double *pold = ustar + 2 * 3 * GP_N;    // [3 slots][GP_N]
-  double *dl = pold + 3 * GP_N;           // [5 slots][GP_N]
+  double *pold = ustar + 2 * 3 * GP_N;    // [3 slots][GP_N] (implicit)
+  double *dl = pold + (MODE == MOM_IMPLICIT ? 3 : 0) * GP_N;  // [5 slots][GP_N]
   double *unew = dl + 5 * GP_N;           // [3 slots][3][GP_N]
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int tid = tx + MC_X * ty;
@@ -324,6 +328,9 @@ __global__ void __launch_bounds__(MC_X *MC_Y, 3)
       }
     }
   };
+  pdl_trigger(dep);
+  pdl_wait(dep);
+  if (dtp) dt = *dtp;  // the step size from device memory (a step inside a CUDA graph)
   // rotating slots: d[i] holds delta of plane K+i (i = 0..4), un_* the
   // projected planes K, K+1, K+2, p_* the lagged pressure of K, K+1, K+2
   double *d[5] = {dl, dl + GP_N, dl + 2 * GP_N, dl + 3 * GP_N, dl + 4 * GP_N};
@@ -341,7 +348,7 @@ __global__ void __launch_bounds__(MC_X *MC_Y, 3)
   project_plane(us_slot(K0 - 1), dm1, d[0], un_m1);
   issue_us(K0);
   box(delta, K0 + 1, d[1]);
-  box(p_in, K0, p_cur);
+  if constexpr (MODE == MOM_IMPLICIT) box(p_in, K0, p_cur);
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();     // u* of K0 and delta of K0+1 landed; slot of u* K0-1 free after this
@@ -349,7 +356,7 @@ __global__ void __launch_bounds__(MC_X *MC_Y, 3)
   __syncthreads();     // every thread is done with u* of K0-1
   issue_us(K0 + 1);
   box(delta, K0 + 2, d[2]);
-  box(p_in, K0 + 1, p_next);
+  if constexpr (MODE == MOM_IMPLICIT) box(p_in, K0 + 1, p_next);
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
@@ -381,16 +388,19 @@ __global__ void __launch_bounds__(MC_X *MC_Y, 3)
         issue_us(K + 3);
         box(delta, K + 4, d[4]);
       }
-      box(p_in, K + 2, p_nn);
+      if constexpr (MODE == MOM_IMPLICIT) box(p_in, K + 2, p_nn);
     }
     cp_async_commit();
     if (inside) {
       const double *pk = p_cur + h, *pk1 = p_next + h;
       const double *dk = d[0] + h, *dk1 = d[1] + h;
-      nb.p0 = pk[0] + dk[0] * radt;
-      nb.pE = pk[1] + dk[1] * radt;
-      nb.pN = pk[SY] + dk[SY] * radt;
-      nb.pT = pk1[0] + dk1[0] * radt;
+      nb.p0 = nb.pE = nb.pN = nb.pT = 0.0;
+      if constexpr (MODE == MOM_IMPLICIT) {
+        nb.p0 = pk[0] + dk[0] * radt;
+        nb.pE = pk[1] + dk[1] * radt;
+        nb.pN = pk[SY] + dk[SY] * radt;
+        nb.pT = pk1[0] + dk1[0] * radt;
+      }
       const double *cx = un_cur + h, *tx_ = un_next + h;
       const double *cy = cx + GP_N, *ty_ = tx_ + GP_N;
       const double *cz = cx + 2 * GP_N, *tz_ = tx_ + 2 * GP_N;
@@ -401,9 +411,9 @@ __global__ void __launch_bounds__(MC_X *MC_Y, 3)
       nb.uz0 = cz[0]; nb.uzE = cz[1]; nb.uzW = cz[-1]; nb.uzN = cz[SY]; nb.uzS = cz[-SY];
       nb.uzT = tz_[0]; nb.uzB = bz0; nb.uzEB = bzE; nb.uzNB = bzN;
       bx0 = nb.ux0; by0 = nb.uy0; bz0 = nb.uz0; bzE = nb.uzE; bzN = nb.uzN;
-      const MomCell m = mom_compute<MOM_IMPLICIT>(g, J, nb, A, dt, B, adt, 1, ymet, theta);
-      mom_store<MOM_IMPLICIT>(g, I, J, K, m, q, out);
-      store_img(p_out, g, I, J, K, nb.p0, STAG_P);
+      const MomCell m = mom_compute<MODE>(g, J, nb, A, dt, B, adt, 1, ymet, theta);
+      mom_store<MODE>(g, I, J, K, m, q, out);
+      if constexpr (MODE == MOM_IMPLICIT) store_img(p_out, g, I, J, K, nb.p0, STAG_P);
     }
     double *t = un_cur;
     un_cur = un_next;
@@ -688,6 +698,7 @@ __global__ void __launch_bounds__(MC_X *MC_Y, 3)
 
 // Dynamic shared memory of k_gradmom_pipe.
 constexpr size_t GRADMOM_PIPE_SMEM = sizeof(double) * (2 * 3 + 3 + 5 + 3 * 3) * GP_N;
+constexpr size_t GRADMOM_PIPE_SMEM_EXPLICIT = sizeof(double) * (2 * 3 + 5 + 3 * 3) * GP_N;
 
 // k_gradmom_deep: k_gradmom_pipe with the raw data staged two planes ahead
 // instead of one.  Iteration K waits for the copies issued in iteration K-2

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 
 namespace dnsb {
@@ -34,13 +35,9 @@ cudaError_t raise_smem(int device, K kernel, size_t bytes) {
   return raise_smem_of(device, reinterpret_cast<const void *>(kernel), bytes);
 }
 
-// Launch as a programmatic dependent of the stream's previous kernel: the
-// grid may become resident while that kernel's last blocks run.  Only for
-// kernels that execute pdl_wait() before any access to memory that an earlier
-// kernel writes or reads (device_pdl.cuh).
 template <class... P, class... A>
-cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
-                             cudaStream_t stream, A... args) {
+cudaError_t launch_as(bool dependent, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                      cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -50,8 +47,44 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Resident blocks of a kernel on the whole device (cached per device, kernel
+// and launch shape).
+inline long resident_blocks(const void *kernel, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void *, int, size_t>, long> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = known.find({dev, kernel, threads, smem});
+  if (it != known.end()) return it->second;
+  int per = 0, nsm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;  // not known: an ordinary launch
+  }
+  return known[{dev, kernel, threads, smem}] = (long)per * nsm;
+}
+
+// Launch of a kernel whose last argument says whether it is a programmatic
+// dependent of the stream's previous kernel (pdl.cuh): where the grid is at
+// most four waves.  A dependent grid's launch and prologue run under the
+// previous kernel's tail (3 us per launch), but each block pays about 2 us in
+// griddepcontrol.wait, the later waves' blocks too: 64^3 step 152 -> 116 us and
+// 128^3 558 -> 526 with the rule; with every kernel dependent the 384 x 256 x
+// 384 step went from 8.05 to 8.75 ms (the Crank-Nicolson solve, 62 waves,
+// from 374 to 652 us).
+constexpr int kDependentWaves = 4;
+template <class K, class... A>
+cudaError_t launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  const long blocks = (long)grid.x * grid.y * grid.z;
+  const int dep = blocks <= kDependentWaves * resident_blocks(reinterpret_cast<const void *>(kernel),
+                                                              (int)(block.x * block.y * block.z), smem);
+  return launch_as(dep, kernel, grid, block, smem, stream, args..., dep);
 }
 
 }  // namespace dnsb

@@ -4,17 +4,24 @@
 
 namespace dnsb {
 
-// Returns once every grid this one depends on has finished and its writes
-// are visible (immediately for an ordinary launch).  Every block executes it
-// before its first access to memory that another kernel writes or reads, so
-// a chain of dependent launches keeps stream order.  What another kernel
-// of the stream writes is read through plain pointers: __ldg and const
-// __restrict__ allow the compiler to move a load above the wait.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel launched by launch_pdl (launch.h) takes as its last argument
+// whether it is a programmatic dependent of the stream's previous kernel.
+//
+// pdl_wait returns once every grid this one depends on has finished and its
+// writes are visible.  Every block executes it before its first access to
+// memory that another kernel writes or reads, so a chain of dependent
+// launches keeps stream order.  What another kernel of the stream writes is
+// read through plain pointers: __ldg and const __restrict__ allow the compiler
+// to move a load above the wait.
+__device__ __forceinline__ void pdl_wait(int dep) {
+  if (dep) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // Lets the dependent grid become resident in the slots this grid leaves free
 // (it takes effect once every block has executed it or exited, so it never
 // displaces a block of this grid).
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_trigger(int dep) {
+  if (dep) asm volatile("griddepcontrol.launch_dependents;");
+}
 
 }  // namespace dnsb

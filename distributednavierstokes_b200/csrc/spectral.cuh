@@ -13,6 +13,7 @@
 #pragma once
 #include "common.cuh"
 #include "fft.cuh"
+#include "pdl.cuh"
 #include "tma.cuh"
 
 namespace dnsb {
@@ -407,64 +408,93 @@ __global__ void __launch_bounds__(SPEC_THREADS, 3) k_irfftx(Geo g, const double2
 // (e = chunk end), G_k = g at the end of chunk k, H_k = h at its start.
 // tab layout per (stage, set): [ta | cp | ib | g | h](ny each), [G | H](CN_CHUNKS
 // each); ib = 1/beta; set 0 tangential, 1 normal.  coef: [at bt ct an bn cn].
-// m is the number of rows per chunk (a power of two, CN_CHUNKS * m >= ny).
+// m is the number of rows per chunk (cn_rows).
 constexpr int CN_CHUNKS = 16;
 constexpr int CN_LINES = 16;
 
 constexpr int CN_MAXCHUNKS = 32;
 __host__ __device__ constexpr long long cn_tab_stride(int ny) { return 5LL * ny + 2 * CN_MAXCHUNKS; }
+// Rows per chunk of k_cn: the least size with an instantiated kernel that
+// covers ny rows (a thread's rows beyond ny are loaded and swept as nothing,
+// so the power of two above 75 rows idled 41 % of them); 0: none does.
+#define CN_ROWS(X) X(1) X(2) X(3) X(4) X(5) X(6) X(8) X(10) X(12) X(16) X(20) X(24) X(32)
+inline int cn_rows(int ny) {
+#define CN_FIT(MR) \
+  if (MR * CN_CHUNKS >= ny) return MR;
+  CN_ROWS(CN_FIT)
+#undef CN_FIT
+  return 0;
+}
 // Shared-memory pitch of one k_cn table with rows skewed by their chunk.
 __host__ __device__ constexpr int cn_skew_pitch(int ny, int mr) { return ny + (ny + mr - 1) / mr; }
 
-// Launch with CN_TABLE_THREADS threads: threads 0..5 (stage, set) run the
-// sequential factorisation, then thread (stage, set, chunk) forms the
-// products of one chunk.
-constexpr int CN_TABLE_THREADS = 6 * CN_MAXCHUNKS;
-__global__ void k_cn_tables(int ny, int m, int nchunks, const double *__restrict__ coef,
-                            double *__restrict__ tab, double dt, double visc, double al0,
-                            double al1, double al2) {
-  const int t = threadIdx.x;
-  const int seq = t % 6, k = t / 6;
-  const int st = seq / 2, set = seq % 2;
-  double *ta = tab + (long long)(st * 2 + set) * cn_tab_stride(ny);
+// The tables of one (stage, set) by one block: the coefficients are staged in
+// shared memory, thread 0 runs the sequential factorisation on them (one
+// reciprocal per row), then the block writes the rows and forms the products
+// of each chunk.  sm: 5 ny doubles.  (A single block of six threads reading
+// the coefficients from global memory inside the recurrence, two divisions per
+// row, took 28.8 us at ny = 75 and 58.7 us at ny = 256 with the GPU idle.)
+__device__ __forceinline__ void cn_table_seq(int seq, int ny, int m, int nchunks,
+                                             const double *__restrict__ coef, double *__restrict__ tab,
+                                             double dt, double visc, double al, double *sm) {
+  const int tid = threadIdx.x + blockDim.x * threadIdx.y, nth = blockDim.x * blockDim.y;
+  const int set = seq % 2;
+  double *ta = tab + (long long)seq * cn_tab_stride(ny);
   double *cp = ta + ny, *ib = cp + ny, *gf = ib + ny, *hb = gf + ny;
   double *G = hb + ny, *H = G + CN_MAXCHUNKS;
-  if (k == 0) {
-    const double al = st == 0 ? al0 : st == 1 ? al1 : al2;
-    const double th = al * dt * visc / 2;
-    const double *a = coef + (set ? 3 : 0) * ny;
-    const double *b = a + ny, *c = b + ny;
-    double beta = 1 - th * b[0];
-    double cprev = -th * c[0] / beta;
-    ta[0] = th * a[0];
-    cp[0] = cprev;
-    ib[0] = 1.0 / beta;
+  double *sa = sm, *sb = sm + ny, *sc = sm + 2 * ny, *scp = sm + 3 * ny, *sf = sm + 4 * ny;
+  const double th = al * dt * visc / 2;
+  const double *a = coef + (set ? 3 : 0) * ny;
+  for (int j = tid; j < ny; j += nth) {
+    sa[j] = th * a[j];
+    sb[j] = 1 - th * a[ny + j];
+    sc[j] = -th * a[2 * ny + j];
+  }
+  __syncthreads();
+  if (tid == 0) {
+    double r = 1.0 / sb[0], c = sc[0] * r;
+    scp[0] = c;
+    sf[0] = r;
+    double a1 = sa[ny > 1], b1 = sb[ny > 1], c1 = sc[ny > 1];
     for (int j = 1; j < ny; j++) {
-      beta = (1 - th * b[j]) + th * a[j] * cprev;
-      cprev = -th * c[j] / beta;
-      ta[j] = th * a[j];
-      cp[j] = cprev;
-      ib[j] = 1.0 / beta;
+      const int jn = min(j + 1, ny - 1);
+      const double a2 = sa[jn], b2 = sb[jn], c2 = sc[jn];  // ahead of the recurrence
+      r = 1.0 / fma(a1, c, b1);
+      c = c1 * r;
+      scp[j] = c;
+      sf[j] = r;
+      a1 = a2;
+      b1 = b2;
+      c1 = c2;
     }
   }
-  __syncthreads();  // also orders the global writes above for the block
-  if (k >= nchunks) return;
-  const int s0 = k * m, e0 = min(ny, s0 + m) - 1;
-  G[k] = 1.0;
-  H[k] = 1.0;
-  if (s0 > e0) return;
-  double acc = 1.0;
-  for (int j = s0; j <= e0; j++) {
-    acc *= ta[j] * ib[j];
-    gf[j] = acc;
+  __syncthreads();
+  for (int j = tid; j < ny; j += nth) {
+    ta[j] = sa[j];
+    cp[j] = scp[j];
+    ib[j] = sf[j];
+    sf[j] *= sa[j];  // f_j = theta a_j / beta_j
   }
-  G[k] = acc;
-  acc = 1.0;
-  for (int j = e0; j >= s0; j--) {
-    acc *= -cp[j];
-    hb[j] = acc;
+  __syncthreads();
+  for (int k = tid; k < nchunks; k += nth) {
+    const int s0 = k * m, e0 = min(ny, s0 + m) - 1;
+    double g = 1.0, h = 1.0;
+    for (int j = s0; j <= e0; j++) gf[j] = (g *= sf[j]);
+    for (int j = e0; j >= s0; j--) hb[j] = (h *= -scp[j]);
+    G[k] = g;
+    H[k] = h;
   }
-  H[k] = acc;
+}
+
+// one block per (stage, set)
+constexpr int CN_TABLE_THREADS = 128;
+inline size_t cn_table_smem(int ny) { return sizeof(double) * 5 * (size_t)ny; }
+__global__ void __launch_bounds__(CN_TABLE_THREADS)
+    k_cn_tables(int ny, int m, int nchunks, const double *__restrict__ coef, double *__restrict__ tab,
+                double dt, double visc, double al0, double al1, double al2) {
+  extern __shared__ double cts[];
+  const int st = blockIdx.x / 2;
+  cn_table_seq(blockIdx.x, ny, m, nchunks, coef, tab, dt, visc, st == 0 ? al0 : st == 1 ? al1 : al2, cts);
 }
 
 // imexsolve_kernel! (src/ydiffusion.jl:94-109) on right-hand sides that the
@@ -481,7 +511,7 @@ __global__ void k_cn_tables(int ny, int m, int nchunks, const double *__restrict
 // shared memory.
 template <int MR>
 __global__ void __launch_bounds__(CN_LINES *CN_CHUNKS, 3) k_cn(Geo g, Fields3 out, CFields3 V,
-                                                              const double *__restrict__ tab) {
+                                                              const double *tab, int dep) {
   extern __shared__ double cs[];  // ta cp ib gf hb (ny each), G H, exchange
   const int i = threadIdx.x, ck = threadIdx.y;
   const int tid = i + CN_LINES * ck;
@@ -497,6 +527,8 @@ __global__ void __launch_bounds__(CN_LINES *CN_CHUNKS, 3) k_cn(Geo g, Fields3 ou
   const bool active = I <= g.nx;
   const int base = gidx(g, active ? I : I0, 1, K);
   const int s0 = ck * MR;
+  pdl_trigger(dep);
+  pdl_wait(dep);
   // 1. this thread's rows of the right-hand side
   double x[MR];
 #pragma unroll

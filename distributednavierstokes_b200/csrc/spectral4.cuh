@@ -6,6 +6,7 @@
 // transform, so these kernels stay bound by HBM traffic.
 #pragma once
 #include "fft4.cuh"
+#include "pdl.cuh"
 #include "spectral.cuh"
 
 namespace dnsb {
@@ -16,7 +17,7 @@ constexpr int F4_THREADS = 256;
 // scales by 1/nz.  Shared memory: transpose buffer + n twiddles.
 template <int N1, int N2, bool INV>
 __global__ void __launch_bounds__(F4_THREADS, 2) k_fftz4(Geo g, double2 *__restrict__ S, int L,
-                                                         const double2 *__restrict__ twz) {
+                                                         const double2 *__restrict__ twz, int dep) {
   constexpr int n = N1 * N2;
   extern __shared__ double2 smem[];
   double2 *buf = smem;
@@ -24,8 +25,10 @@ __global__ void __launch_bounds__(F4_THREADS, 2) k_fftz4(Geo g, double2 *__restr
   const long long nlines = (long long)g.ny * g.nkx;
   const long long l0 = (long long)blockIdx.x * L;
   const int Lv = (int)min((long long)L, nlines - l0);
+  pdl_trigger(dep);
   for (int t = threadIdx.x; t < n; t += blockDim.x) tw[t] = twz[t];
   __syncthreads();
+  pdl_wait(dep);
   double2 *src = S + l0 * n;
   const double sc = 1.0 / n;
   fft4_lines<N1, N2, INV>(

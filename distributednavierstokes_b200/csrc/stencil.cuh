@@ -11,6 +11,8 @@
 // the reference's divisions); halving uses *0.5 (exact).
 #pragma once
 #include "common.cuh"
+#include "pdl.cuh"
+#include "spectral.cuh"
 #include "tma.cuh"
 
 namespace dnsb {
@@ -235,10 +237,9 @@ __device__ __forceinline__ void mom_store(const Geo &g, int I, int J, int K, con
 }
 
 // Column of k_momentum_march: MC_X x MC_Y cells per CTA (one thread each)
-// walking `planes` planes in z (MC_Z on large grids; fewer where the grid
-// would otherwise leave SMs idle).  Planes are staged with a one-cell halo in x
+// walking `planes` planes in z (the launch's march_planes).  Planes are staged with a one-cell halo in x
 // and y in a ring of four.
-constexpr int MC_X = 32, MC_Y = 8, MC_Z = 16;  // measured best of 8-64 planes, 4-8 rows
+constexpr int MC_X = 32, MC_Y = 8;  // measured best of 4-8 rows
 constexpr int MP_X = MC_X + 2, MP_Y = MC_Y + 2, MP_N = MP_X * MP_Y;
 
 // momentum_kernel! with the velocity planes staged in shared memory: the
@@ -248,18 +249,39 @@ constexpr int MP_X = MC_X + 2, MP_Y = MC_Y + 2, MP_N = MP_X * MP_Y;
 // plane K+2 into the fourth slot while it computes plane K.  Same
 // arithmetic and stores as k_momentum.
 // 3 CTAs of 256 per SM (80 registers; faster than 2 CTAs without the cap)
+// ct.tab (implicit): the first block layer writes the Crank-Nicolson tables
+// of the step's three stages (beside the cells' blocks) instead of a launch of its own in front, which held the
+// stream for 28.8 us at ny = 75 and 58.7 us at ny = 256.
+struct CnTabArgs {
+  double *tab;
+  const double *coef;
+  int m;
+  double al[3];
+};
+static_assert(5 * 512 <= 4 * 3 * MP_N, "the tables' scratch fits the ring (ny <= 512)");
 template <int MODE>
 __global__ void __launch_bounds__(MC_X *MC_Y, 3)
-    k_momentum_march(Geo g, Fields3 q, CFields3 u, Fields3 out, const double *__restrict__ p,
+    k_momentum_march(Geo g, Fields3 q, CFields3 u, Fields3 out, const double *p,
                      double A, double dt, double B, double adt, int readq,
                      const double2 *__restrict__ ymet, double theta, int planes,
-                     const double *__restrict__ dtp) {
+                     const double *__restrict__ dtp, CnTabArgs ct, int dep) {
   __shared__ __align__(16) double ring[4][3][MP_N];
+  pdl_trigger(dep);
+  pdl_wait(dep);
   if (dtp) dt = *dtp;  // the step size from device memory (a step inside a CUDA graph)
+  if (MODE == MOM_IMPLICIT && ct.tab && blockIdx.z == 0) {
+    // the layer in front: the step's Crank-Nicolson tables
+    for (int seq = blockIdx.x + gridDim.x * blockIdx.y; seq < 6; seq += gridDim.x * gridDim.y) {
+      __syncthreads();
+      cn_table_seq(seq, g.ny, ct.m, CN_CHUNKS, ct.coef, ct.tab, dt, g.visc, ct.al[seq / 2], ring[0][0]);
+    }
+    return;
+  }
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int tid = tx + MC_X * ty;
   const int I0 = blockIdx.x * MC_X + 1, J0 = blockIdx.y * MC_Y + 1;
-  const int K0 = blockIdx.z * planes + 1, K1 = min(g.nz, K0 + planes - 1);
+  const int bz = blockIdx.z - (MODE == MOM_IMPLICIT && ct.tab ? 1 : 0);
+  const int K0 = bz * planes + 1, K1 = min(g.nz, K0 + planes - 1);
   constexpr int CH = MP_X / 2;  // 16-byte chunks per halo row
   static_assert(MP_Y * CH <= MC_X * MC_Y, "one staging chunk per thread and field plane");
   // this thread's chunk of every staged plane (the same in-plane offset for
@@ -303,10 +325,10 @@ __global__ void __launch_bounds__(MC_X *MC_Y, 3)
     nb.qz0 = (inside && readq) ? q.z[c0] : 0.0;
     nb.p0 = nb.pE = nb.pN = nb.pT = 0.0;
     if (MODE == MOM_IMPLICIT && inside) {
-      nb.p0 = __ldg(p + c0);
-      nb.pE = __ldg(p + c0 + 1);
-      nb.pN = __ldg(p + c0 + sy);
-      nb.pT = __ldg(p + c0 + sz);
+      nb.p0 = p[c0];
+      nb.pE = p[c0 + 1];
+      nb.pN = p[c0 + sy];
+      nb.pT = p[c0 + sz];
     }
     cp_async_wait<0>();  // planes up to K+1 have landed (this thread's copies)
     __syncthreads();     // ... everyone's, and plane K-2's slot is free
@@ -344,12 +366,14 @@ __device__ __forceinline__ unsigned long long dbits(double v) {
 // folded into umax[c] (as ordered bit patterns of non-negative doubles).
 template <int MODE>
 __global__ void __launch_bounds__(256) k_grad(Geo g, Fields3 u, CFields3 W,
-                                              const double *__restrict__ psi, double *p,
-                                              double radt, unsigned long long *umax) {
+                                              const double *psi, double *p,
+                                              double radt, unsigned long long *umax, int dep) {
   const int I = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int J = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int K = blockIdx.z + 1;
   double m0 = 0, m1 = 0, m2 = 0;
+  pdl_trigger(dep);
+  pdl_wait(dep);
   if (I <= g.nx && J <= g.ny) {
     const int sy = g.NX, sz = g.NX * g.NY;
     const int c0 = gidx(g, I, J, K);

@@ -23,6 +23,7 @@
 // needed.  Algebraically this is the reference's Thomas algorithm.
 #pragma once
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace dnsb {
 
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(TY_LINES *TY_CHUNKS, MR <= 8 ? 3 : 1)
     k_ythomas(Geo g, double2 *__restrict__ S, const double *__restrict__ cin,
               const double *__restrict__ ay, const double *__restrict__ by,
               const double *__restrict__ cy, const double *__restrict__ lam1,
-              const double *__restrict__ lam3) {
+              const double *__restrict__ lam3, int dep) {
   // chunk maps, one row of lines per chunk padded by one entry so that the
   // scan's lane-per-chunk reads spread over all banks
   __shared__ double4 za[TY_CHUNKS][TY_LINES + 1];  // forward (Z.re, Z.im, G)
@@ -113,7 +114,9 @@ __global__ void __launch_bounds__(TY_LINES *TY_CHUNKS, MR <= 8 ? 3 : 1)
   const int i = threadIdx.x, ck = threadIdx.y;
   const int ny = g.ny, nz = g.nz;
   const long long nl = (long long)nz * g.nkx;
-  const long long t = (long long)blockIdx.x * TY_LINES + i;
+  // last kx plane first: it is still in L2 from the z-transform, and this
+  // kernel's last planes, the lowest kx, are where the inverse one starts
+  const long long t = (long long)(gridDim.x - 1 - blockIdx.x) * TY_LINES + i;
   const bool act = t < nl;
   const int kz = act ? (int)(t % nz) : 0, kx = act ? (int)(t / nz) : 0;
   const double lam = __ldg(lam1 + kx) + __ldg(lam3 + kz);
@@ -133,6 +136,9 @@ __global__ void __launch_bounds__(TY_LINES *TY_CHUNKS, MR <= 8 ? 3 : 1)
       c = __ldg(cy + j);
     }
   };
+  double cprev = act ? __ldg(cin + t * TY_CHUNKS + ck) : 0.0;  // (a table of the context)
+  pdl_trigger(dep);
+  pdl_wait(dep);
   double2 d[MR];
 #pragma unroll
   for (int r = 0; r < MR; r++) {
@@ -140,7 +146,6 @@ __global__ void __launch_bounds__(TY_LINES *TY_CHUNKS, MR <= 8 ? 3 : 1)
     d[r] = (act && j < ny) ? x[j * st] : make_double2(0.0, 0.0);
   }
   if (pin && s0 == 0) d[0] = make_double2(0.0, 0.0);
-  double cprev = act ? __ldg(cin + t * TY_CHUNKS + ck) : 0.0;
   // forward: 1/beta_j of the chunk (kept in shared memory, one column per
   // thread; c'_j = c_j / beta_j is re-formed where needed), its affine map
   // d'_e = Z + G d'_{s-1}

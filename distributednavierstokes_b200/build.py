@@ -24,7 +24,7 @@ INCLUDES = [os.path.join(ROOT, "include", h) for h in ("dnsb.h", "dnsb_cnn.h")]
 HEADERS = {
     "dnsb.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "spectral.cuh", "spectral4.cuh", "stencil.cuh",
                 "tma.cuh", "ysolve.cuh", "gradmom.cuh", "zyz.cuh", "spsolver.cuh", "lowshells.cuh",
-                "cnn_host.h", "fftany.h", "launch.h", "pdl.cuh"],
+                "cnn_host.h", "fftany.h", "launch.h", "pdl.cuh", "xwarp.cuh"],
     "fftany.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "fftany.cuh", "fftany.h", "launch.h", "pdl.cuh"],
     "cnn.cu": ["cnn.cuh", "cnn_host.h"],
 }

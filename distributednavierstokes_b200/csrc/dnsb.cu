@@ -167,11 +167,7 @@ struct dnsb_ctx {
   AnySplit ax, ay_, az;  // run-time splits of nx/2, ny and nz (tier 0: none, the Stockham kernels)
   int Lx_set = 0, Lz_set = 0, Ly_set = 0;  // lines per block asked for (0: the launch rules)
   int L4z = 8;                         // lines per CTA of the z-FFT
-  // divergence x-FFT with its output pass in registers (3 % faster at
-  // 384x256x384 than the separate shared-memory pass)
-  int rx_post = 1;
-  int ix_pairs = 0;  // inverse x-FFT with the pair pre-processing in its first pass
-  size_t smem_rx4 = 0, smem_ix4 = 0, smem_z4 = 0;
+  size_t smem_z4 = 0;
   int nsm = 148;
   size_t smem_zt = 0;
   double *hostred = nullptr;           // pinned, 8 doubles
@@ -647,26 +643,18 @@ int ensure_device(dnsb_ctx *c) {
   return 0;
 }
 
-#define FFT4_SPLITS(X) X(16, 24) X(16, 16) X(16, 12) X(16, 8) X(8, 12) X(8, 8) X(8, 6) X(8, 4)
-constexpr int IRX_L = 16;  // lines per CTA of the four-step inverse x-FFT
-constexpr int RFX_L = 8;   // lines per CTA of the four-step forward x-FFT
 
-// four-step kernel launches for the split chosen at create time
+// four-step x-kernels for the split chosen at create time
 int launch_rfftx4(dnsb_ctx *c, int mode, const double *a, const double *b, const double *cc) {
   const Geo &g = c->g;
-  dim3 grid(g.ny * ((g.nz + RFX_L - 1) / RFX_L));
 #define RF4(A, B)                                                                                  \
   if (c->x1 == A && c->x2 == B) {                                                                  \
-    if (mode == RIN_DIVERGENCE && c->rx_post)                                                      \
-      LAUNCH(c, DNSB_KIND_RFFTX, k_rfftx4<A, B, RFX_L, RIN_DIVERGENCE, true><<<grid, F4_THREADS, c->smem_rx4, c->stream>>>(g, c->S, a, b, cc, c->twM, c->twN)); \
-    else if (mode == RIN_DIVERGENCE)                                                               \
-      LAUNCH(c, DNSB_KIND_RFFTX, k_rfftx4<A, B, RFX_L, RIN_DIVERGENCE><<<grid, F4_THREADS, c->smem_rx4, c->stream>>>(g, c->S, a, b, cc, c->twM, c->twN)); \
-    else if (mode == RIN_REAL)                                                                     \
-      LAUNCH(c, DNSB_KIND_RFFTX, k_rfftx4<A, B, RFX_L, RIN_REAL><<<grid, F4_THREADS, c->smem_rx4, c->stream>>>(g, c->S, a, b, cc, c->twM, c->twN)); \
-    else if (mode == RIN_PRODUCT)                                                                  \
-      LAUNCH(c, DNSB_KIND_RFFTX, k_rfftx4<A, B, RFX_L, RIN_PRODUCT><<<grid, F4_THREADS, c->smem_rx4, c->stream>>>(g, c->S, a, b, cc, c->twM, c->twN)); \
-    else                                                                                           \
-      LAUNCH(c, DNSB_KIND_RFFTX, k_rfftx4<A, B, RFX_L, RIN_FIELD><<<grid, F4_THREADS, c->smem_rx4, c->stream>>>(g, c->S, a, b, cc, c->twM, c->twN)); \
+    const dim3 grid(g.ny * ((g.nz + XWarp<A, B>::LINES - 1) / XWarp<A, B>::LINES));                \
+    auto k = mode == RIN_DIVERGENCE ? k_rfftx4<A, B, RIN_DIVERGENCE>                               \
+             : mode == RIN_REAL     ? k_rfftx4<A, B, RIN_REAL>                                     \
+             : mode == RIN_PRODUCT  ? k_rfftx4<A, B, RIN_PRODUCT>                                  \
+                                    : k_rfftx4<A, B, RIN_FIELD>;                                   \
+    LAUNCH(c, DNSB_KIND_RFFTX, CK(c, launch_pdl(k, grid, dim3(128), XWarp<A, B>::smem, c->stream, g, c->S, a, b, cc, c->twM, c->twN))); \
     return 0;                                                                                      \
   }
   FFT4_SPLITS(RF4)
@@ -676,16 +664,13 @@ int launch_rfftx4(dnsb_ctx *c, int mode, const double *a, const double *b, const
 
 int launch_irfftx4(dnsb_ctx *c, int mode, double *out) {
   const Geo &g = c->g;
-  dim3 grid(g.ny * ((g.nz + IRX_L - 1) / IRX_L));
 #define IF4(A, B)                                                                                  \
   if (c->x1 == A && c->x2 == B) {                                                                  \
-    if (mode == ROUT_INTERIOR)                                                                     \
-      LAUNCH(c, DNSB_KIND_IRFFTX, k_irfftx4<A, B, IRX_L, ROUT_INTERIOR><<<grid, F4_THREADS, c->smem_ix4, c->stream>>>(g, c->S, out, c->twM, c->twN)); \
-    else if (mode == ROUT_IMAGES)                                                                  \
-      { if (c->ix_pairs) LAUNCH(c, DNSB_KIND_IRFFTX, k_irfftx4<A, B, IRX_L, ROUT_IMAGES, true><<<grid, F4_THREADS, c->smem_ix4, c->stream>>>(g, c->S, out, c->twM, c->twN)); \
-        else LAUNCH(c, DNSB_KIND_IRFFTX, k_irfftx4<A, B, IRX_L, ROUT_IMAGES><<<grid, F4_THREADS, c->smem_ix4, c->stream>>>(g, c->S, out, c->twM, c->twN)); } \
-    else                                                                                           \
-      LAUNCH(c, DNSB_KIND_IRFFTX, k_irfftx4<A, B, IRX_L, ROUT_REAL><<<grid, F4_THREADS, c->smem_ix4, c->stream>>>(g, c->S, out, c->twM, c->twN)); \
+    const dim3 grid(g.ny * ((g.nz + XWarp<A, B>::LINES - 1) / XWarp<A, B>::LINES));                \
+    auto k = mode == ROUT_INTERIOR ? k_irfftx4<A, B, ROUT_INTERIOR>                                \
+             : mode == ROUT_IMAGES ? k_irfftx4<A, B, ROUT_IMAGES>                                  \
+                                   : k_irfftx4<A, B, ROUT_REAL>;                                   \
+    LAUNCH(c, DNSB_KIND_IRFFTX, CK(c, launch_pdl(k, grid, dim3(128), XWarp<A, B>::smem, c->stream, g, c->S, out, c->twM, c->twN))); \
     return 0;                                                                                      \
   }
   FFT4_SPLITS(IF4)
@@ -712,15 +697,14 @@ int launch_fftz4(dnsb_ctx *c, bool inv) {
 template <int A, int B>
 int allow_fft4(dnsb_ctx *c) {
   int rc;
-  if ((rc = allow_smem(c, k_rfftx4<A, B, RFX_L, RIN_DIVERGENCE>, c->smem_rx4)) ||
-      (rc = allow_smem(c, k_rfftx4<A, B, RFX_L, RIN_DIVERGENCE, true>, c->smem_rx4)) ||
-      (rc = allow_smem(c, k_rfftx4<A, B, RFX_L, RIN_REAL>, c->smem_rx4)) ||
-      (rc = allow_smem(c, k_rfftx4<A, B, RFX_L, RIN_FIELD>, c->smem_rx4)) ||
-      (rc = allow_smem(c, k_rfftx4<A, B, RFX_L, RIN_PRODUCT>, c->smem_rx4)) ||
-      (rc = allow_smem(c, k_irfftx4<A, B, IRX_L, ROUT_INTERIOR>, c->smem_ix4)) ||
-      (rc = allow_smem(c, k_irfftx4<A, B, IRX_L, ROUT_IMAGES>, c->smem_ix4)) ||
-      (rc = allow_smem(c, k_irfftx4<A, B, IRX_L, ROUT_IMAGES, true>, c->smem_ix4)) ||
-      (rc = allow_smem(c, k_irfftx4<A, B, IRX_L, ROUT_REAL>, c->smem_ix4)) ||
+  constexpr size_t xs = XWarp<A, B>::smem;
+  if ((rc = allow_smem(c, k_rfftx4<A, B, RIN_DIVERGENCE>, xs)) ||
+      (rc = allow_smem(c, k_rfftx4<A, B, RIN_REAL>, xs)) ||
+      (rc = allow_smem(c, k_rfftx4<A, B, RIN_FIELD>, xs)) ||
+      (rc = allow_smem(c, k_rfftx4<A, B, RIN_PRODUCT>, xs)) ||
+      (rc = allow_smem(c, k_irfftx4<A, B, ROUT_INTERIOR>, xs)) ||
+      (rc = allow_smem(c, k_irfftx4<A, B, ROUT_IMAGES>, xs)) ||
+      (rc = allow_smem(c, k_irfftx4<A, B, ROUT_REAL>, xs)) ||
       (rc = allow_smem(c, k_fftz4<A, B, false>, c->smem_z4)) ||
       (rc = allow_smem(c, k_fftz4<A, B, true>, c->smem_z4)))
     return rc;
@@ -1545,14 +1529,9 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
     c->Lz_set = tuned(tun ? tun->lines_z : 0, "DNSB_LZ", 0);
     c->Ly_set = tuned(tun ? tun->lines_y : 0, "DNSB_LY", 0);
     c->L4z = std::max(1, tuned(tun ? tun->lines_z4 : 0, "DNSB_L4Z", 8));
-    c->rx_post = envint("DNSB_RXPOST", c->rx_post) != 0;
-    c->ix_pairs = envint("DNSB_IXPAIRS", c->ix_pairs) != 0;
     if (fft4_split(M, a, b)) {
       c->x1 = a;
       c->x2 = b;
-      const size_t pitch = b % 2 == 0 ? b + 1 : b;
-      c->smem_rx4 = sizeof(double2) * ((size_t)RFX_L * (a * pitch + 1) + (size_t)RFX_L * (M + 1) + M + (M + 1));
-      c->smem_ix4 = sizeof(double2) * ((size_t)IRX_L * (M + 2) + (size_t)IRX_L * (a * pitch + 1) + M + (M + 1));
     }
     if (fft4_split(nz, a, b)) {
       c->z1 = a;

@@ -18,15 +18,17 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(ROOT, "_build")
 OUT = os.path.join(HERE, "libdnsb.so")
-SOURCES = ["dnsb.cu", "fftany.cu", "cnn.cu"]
+SOURCES = ["dnsb.cu", "fftany.cu", "spany.cu", "cnn.cu"]
 INCLUDES = [os.path.join(ROOT, "include", h) for h in ("dnsb.h", "dnsb_cnn.h")]
 # headers each translation unit includes (a change rebuilds its object)
 HEADERS = {
     "dnsb.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "spectral.cuh", "spectral4.cuh", "stencil.cuh",
                 "tma.cuh", "ysolve.cuh", "gradmom.cuh", "zyz.cuh", "spsolver.cuh", "lowshells.cuh",
-                "cnn_host.h", "fftany.h", "launch.h", "pdl.cuh", "xwarp.cuh"],
+                "cnn_host.h", "fftany.h", "launch.h", "pdl.cuh", "spany.h", "xwarp.cuh"],
     "fftany.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "fftany.cuh", "fftany.h", "launch.h", "pdl.cuh"],
-    "cnn.cu": ["cnn.cuh", "cnn_host.h"],
+    "spany.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "fftany.cuh", "fftany.h", "launch.h", "pdl.cuh",
+                 "spany.cuh", "spany.h", "xwarp.cuh"],
+    "cnn.cu": ["cnn.cuh", "cnn_host.h", "launch.h", "pdl.cuh"],
 }
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

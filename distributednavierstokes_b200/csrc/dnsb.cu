@@ -33,6 +33,7 @@
 #include "fft.cuh"
 #include "fftany.h"
 #include "launch.h"
+#include "spany.h"
 #include "spectral.cuh"
 #include "spectral4.cuh"
 #include "ysolve.cuh"
@@ -2773,6 +2774,7 @@ struct dnsb_spectral {
   double *shellbuf = nullptr;                  // [E | factors | eref] x nshell
   double *shellpart = nullptr;                 // RED_BLOCKS x SP_SHELLS partial sums
   std::vector<double> eref_host;
+  SpPlan any;                                  // truncated transforms (ok(): the lengths have a split)
   std::vector<void *> allocs;
   std::string err;
 };
@@ -2854,11 +2856,29 @@ int sp_from_product(dnsb_spectral *p, const double *va, const double *vb) {
   return 0;
 }
 
+// spec_to_phys! of the three components
+int sp_to_phys3(dnsb_spectral *p, const double2 *uh, double *const v[3]) {
+  if (p->any.ok()) {
+    SPK(p, sp_any_phys(p->any, uh, v, p->c->stream));
+    return 0;
+  }
+  int rc;
+  for (int comp = 0; comp < 3; comp++)
+    if ((rc = sp_to_phys(p, uh + comp * p->s.nc, v[comp]))) return rc;
+  return 0;
+}
+
 // spectral_rhs!: du = -i k_j F[v_i v_j] / n^3; leaves v = the physical velocity
 int sp_rhs(dnsb_spectral *p, const double2 *uh, double2 *du) {
   dnsb_ctx *c = p->c;
   const long long n3 = sp_n3(p);
   int rc;
+  if (p->any.ok()) {
+    SPK(p, sp_any_phys(p->any, uh, p->v, c->stream));
+    SPK(p, sp_any_products(p->any, p->v, nullptr, c->stream));
+    SPK(p, sp_any_rhs(p->any, du, c->stream));
+    return 0;
+  }
   for (int comp = 0; comp < 3; comp++)
     if ((rc = sp_to_phys(p, uh + comp * p->s.nc, p->v[comp]))) return rc;
   static const int pa[6] = {0, 1, 2, 0, 1, 2}, pb[6] = {0, 1, 2, 1, 2, 0};
@@ -2949,6 +2969,26 @@ int dnsb_spectral_create(int n, int kcut, double l, double visc, int device, voi
     dnsb_spectral_destroy(p);
     return rc;
   }
+  // The truncated transforms' six buffers of (kcut + 1) n^2 values are the
+  // context's spectrum and the fields that the solver does not use otherwise
+  // (n^3 real values hold them from n = 6 on: (n/3 + 1) n^2 complex).
+  if (c->ax.tier && c->az.tier && n >= 6) {
+    SpPlan &a = p->any;
+    a.s = SpCube{n, kcut, 2 * kcut + 1, p->s.nc, p->s.kfac};
+    a.x = c->ax;
+    a.yz = c->az;
+    a.twM = c->twM;
+    a.twN = c->twN;
+    a.twn = c->twz;
+    double *const real[5] = {c->W[0], c->W[1], c->W[2], c->r, p->r};
+    a.buf[0] = c->S;
+    for (int i = 0; i < 5; i++) a.buf[i + 1] = reinterpret_cast<double2 *>(real[i]);
+    if (sp_any_allow(device, a) != cudaSuccess) {
+      snprintf(g_create_err, sizeof g_create_err, "shared-memory opt-in of the spectral kernels failed");
+      dnsb_spectral_destroy(p);
+      return DNSB_ECUDA;
+    }
+  }
   if (cudaMallocHost(&p->host, 4 * sizeof(double)) != cudaSuccess) {
     snprintf(g_create_err, sizeof g_create_err, "cudaMallocHost failed");
     dnsb_spectral_destroy(p);
@@ -2975,10 +3015,8 @@ int dnsb_spectral_to_phys(dnsb_spectral *p, const double *uh, double *v) {
   int rc = sp_check(p, uh);
   if (rc || (rc = sp_check(p, v))) return rc;
   const long long n3 = sp_n3(p);
-  for (int comp = 0; comp < 3; comp++)
-    if ((rc = sp_to_phys(p, reinterpret_cast<const double2 *>(uh) + comp * p->s.nc, v + comp * n3)))
-      return rc;
-  return 0;
+  double *const vc[3] = {v, v + n3, v + 2 * n3};
+  return sp_to_phys3(p, reinterpret_cast<const double2 *>(uh), vc);
 }
 
 int dnsb_spectral_from_phys(dnsb_spectral *p, const double *v, double *uh) {
@@ -3017,10 +3055,17 @@ int dnsb_spectral_step(dnsb_spectral *p, double *uh, double dt, double *vmax_out
   double2 *u2 = reinterpret_cast<double2 *>(uh);
   static const double A[3] = {8.0 / 15, 5.0 / 12, 3.0 / 4}, B[3] = {1.0 / 4, 0.0, 0.0},
                       DC[3] = {8.0 / 15, 2.0 / 15, 1.0 / 3};
-  SPK(p, cudaMemcpyAsync(p->ustart, u2, sizeof(double2) * 3 * (size_t)p->s.nc,
-                         cudaMemcpyDeviceToDevice, c->stream));
   SPK(p, cudaMemsetAsync(p->umax, 0, sizeof(unsigned long long), c->stream));
-  for (int i = 0; i < 3; i++) {
+  for (int i = 0; p->any.ok() && i < 3; i++) {
+    SPK(p, sp_any_phys(p->any, u2, p->v, c->stream));
+    SPK(p, sp_any_products(p->any, p->v, i == 0 ? p->umax : nullptr, c->stream));
+    SPK(p, sp_any_stage(p->any, u2, i == 0 ? u2 : p->ustart, i < 2 ? p->ustart : nullptr, A[i], B[i],
+                        p->visc * DC[i] * dt, dt, c->stream));
+  }
+  if (!p->any.ok())
+    SPK(p, cudaMemcpyAsync(p->ustart, u2, sizeof(double2) * 3 * (size_t)p->s.nc,
+                           cudaMemcpyDeviceToDevice, c->stream));
+  for (int i = 0; !p->any.ok() && i < 3; i++) {
     if ((rc = sp_rhs(p, u2, p->du))) return rc;
     if (i == 0) {
       k_sp_vsummax<<<RED_BLOCKS, 256, 0, c->stream>>>(sp_n3(p), p->v[0], p->v[1], p->v[2], p->umax);
@@ -3044,9 +3089,7 @@ int dnsb_spectral_vsummax(dnsb_spectral *p, const double *uh, double *out) {
   int rc = sp_check(p, uh);
   if (rc || (rc = sp_check(p, out))) return rc;
   dnsb_ctx *c = p->c;
-  for (int comp = 0; comp < 3; comp++)
-    if ((rc = sp_to_phys(p, reinterpret_cast<const double2 *>(uh) + comp * p->s.nc, p->v[comp])))
-      return rc;
+  if ((rc = sp_to_phys3(p, reinterpret_cast<const double2 *>(uh), p->v))) return rc;
   SPK(p, cudaMemsetAsync(p->umax, 0, sizeof(unsigned long long), c->stream));
   k_sp_vsummax<<<RED_BLOCKS, 256, 0, c->stream>>>(sp_n3(p), p->v[0], p->v[1], p->v[2], p->umax);
   SPKL(p);

@@ -141,7 +141,7 @@ struct dnsb_ctx {
   // scratch
   double2 *S = nullptr;
   double2 *Sx[2] = {nullptr, nullptr};  // spectra of u.y, u.z during a shell clamp
-  double2 *lsA = nullptr, *lsB = nullptr, *lsG = nullptr, *lsH = nullptr;  // low-shell clamp scratch
+  double2 *lsA = nullptr, *lsB = nullptr, *lsG = nullptr;  // low-shell clamp scratch
   // e^{2 pi i r / n}, r = 0..n-1, per direction, for the clamp's partial sums
   double2 *lsX = nullptr, *lsY = nullptr, *lsZ = nullptr;
   double *work = nullptr;
@@ -1299,7 +1299,6 @@ int upload_eref(dnsb_ctx *c, const double *eref, int nb) {
       if ((rc = dalloc(c, &c->lsA, (size_t)3 * LS_KX * g.ny * g.nz)) ||
           (rc = dalloc(c, &c->lsB, (size_t)3 * LS_KX * g.nz * LS_KY)) ||
           (rc = dalloc(c, &c->lsG, (size_t)3 * LS_KX * LS_KY * LS_KY)) ||
-          (rc = dalloc(c, &c->lsH, (size_t)3 * LS_KX * LS_KY * g.nz)) ||
           (rc = dalloc(c, &c->lsX, (size_t)g.nx)) || (rc = dalloc(c, &c->lsY, (size_t)g.ny)) ||
           (rc = dalloc(c, &c->lsZ, (size_t)g.nz)))
         return rc;
@@ -2351,17 +2350,17 @@ int dnsb_shell_clamp(dnsb_ctx *c, double *ux, double *uy, double *uz, const doub
   if (clamp_direct(c, nb)) {
     const Geo &g = c->g;
     const int KM = nb - 1;
+    const int H = KM + 1, W = 2 * KM + 1;
     const unsigned lines = (unsigned)(((long long)g.ny * g.nz + LS_LINES - 1) / LS_LINES);
-    k_ls_xsums<<<lines, 32 * LS_LINES, 0, c->stream>>>(g, cf(ux, uy, uz), KM, c->lsX, c->lsA);
-    CKL(c);
-    k_ls_ysums<<<(unsigned)(3 * (KM + 1) * g.nz), 128, 0, c->stream>>>(g, c->lsA, KM, c->lsY, c->lsB);
-    CKL(c);
-    k_ls_zsums<<<(unsigned)(3 * (KM + 1) * (2 * KM + 1)), 128, 0, c->stream>>>(g, c->lsB, KM, c->lsZ, c->lsG);
-    CKL(c);
-    k_ls_modes<<<1, 1024, 0, c->stream>>>(g, KM, c->lsG, c->lsH, E, er, f, nb, c->lsZ);
-    CKL(c);
-    k_ls_correct<<<lines, 32 * LS_LINES, 0, c->stream>>>(g, ff(ux, uy, uz), KM, c->lsH, c->lsX, c->lsY);
-    CKL(c);
+    CK(c, launch_pdl(k_ls_xsums, dim3(lines), dim3(128), 0, c->stream, g, cf(ux, uy, uz), KM, c->lsX,
+                     c->lsA));
+    CK(c, launch_pdl(k_ls_sums<8, 4>, dim3((3 * H * g.nz + 7) / 8), dim3(LS_STHREADS), 0, c->stream,
+                     3 * H * g.nz, g.ny, 1, (long long)g.ny, 1, c->lsA, KM, c->lsY, c->lsB));
+    CK(c, launch_pdl(k_ls_sums<1, 32>, dim3(3 * H * W), dim3(LS_STHREADS), 0, c->stream, 3 * H * W, g.nz, W,
+                     (long long)g.nz * W, W, c->lsB, KM, c->lsZ, c->lsG));
+    CK(c, launch_pdl(k_ls_modes, dim3(1), dim3(256), 0, c->stream, g, KM, c->lsG, E, er, f, nb));
+    CK(c, launch_pdl(k_ls_correct, dim3((g.ny + LS_CLINES - 1) / LS_CLINES, g.nz), dim3(256), 0,
+                           c->stream, g, ff(ux, uy, uz), KM, c->lsG, c->lsX, c->lsY, c->lsZ));
     c->umax_for[0] = c->umax_for[1] = c->umax_for[2] = nullptr;
     return 0;
   }

@@ -5,27 +5,37 @@
 // floor(|k|) < nb, nb <= 4: at most 4 x 7 x 7 of the half spectrum.  Their
 // coefficients u_hat(k) = sum_x u(x) e^{-i k.x} (the unnormalised FFT of the
 // interior, as the transform path computes them) are formed separably:
-//   1. per (y, z) line, the x-sums for kx = 0..KM (one read of the field;
-//      a warp per line, lanes striding x, shuffle reduction in a fixed order);
-//   2. the y-sums (ky = -KM..KM) and z-sums (kz = -KM..KM), a block per
-//      output row with fixed-order tree reductions;
+//   1. per (y, z) line, the x-sums for kx = 0..KM (one read of the field; a
+//      thread per line and component, the tile staged in shared memory);
+//   2. the y-sums (ky = -KM..KM), then the z-sums (kz = -KM..KM), a thread per
+//      row, output and part of the row (PARTS), the parts added in order;
 //   3. one block: the shell energies (1/2 w |u_hat|^2 / N^2, w the rfft
-//      double count), the clamp factors f = sqrt(eref / E), the corrections
-//      G(k) = (f(shell) - 1) u_hat(k) / N and their z-sums back to physical z;
-//   4. per (y, z) line, u += Re sum_k w G(k) e^{i k.x} (the y-sum of 2KM+1
-//      terms per line, then the x-sum per point) and the periodic ghost
-//      images are rewritten.
+//      double count; a warp per shell), the clamp factors f = sqrt(eref / E),
+//      the corrections G(k) = (f(shell) - 1) u_hat(k) / N;
+//   4. per block of 16 lines of one plane, the z- and y-sums of G back to
+//      physical space (cooperatively, in shared memory), then
+//      u += Re sum_kx w P(kx) e^{i kx x} per point with the periodic ghost
+//      images.
 // Two passes over each component instead of three forward and three
 // inverse 3-D transforms.  KM = nb - 1 <= 3 and 2 KM < n in every direction.
+// Every sum has a fixed order.  What bounded the first form was not memory:
+// the x-sums spent 240 shuffles per line on reducing 12 complex partial sums,
+// the correction formed each line's 12 plane sums on 12 lanes of its warp
+// from 7 global loads and 14 integer remainders, the shell sums ran on one
+// thread.  128^3, shells 1-2, before -> now: x-sums 32.0 -> 20.4, y 9.1 -> 8.4,
+// z 4.3 -> 3.2, modes 16.1 -> 3.3, correction 56.5 -> 29.6 us.
 #pragma once
 #include "common.cuh"
 #include "fft.cuh"
+#include "pdl.cuh"
 
 namespace dnsb {
 
 constexpr int LS_KX = 4;             // kx = 0..3
 constexpr int LS_KY = 7;             // ky, kz = -3..3
-constexpr int LS_LINES = 8;          // (y, z) lines per CTA of 256 threads
+constexpr int LS_LINES = 32;         // (y, z) lines per block of the x-sums
+constexpr int LS_XT = 32;            // points per staged tile of a line
+constexpr int LS_CLINES = 16;        // lines (one plane) per block of the correction
 
 // the phases e^{+2 pi i r / n} = (cos, sin) for r = 0..n-1 of one direction,
 // formed once per context (the expression the partial sums evaluated per
@@ -49,241 +59,206 @@ __device__ __forceinline__ double2 ls_phase_tab(int m, int n, double sign, const
 }
 
 // A[((c * (KM+1) + kx) * nz + (K-1)) * ny + (J-1)] = sum_i u_c(i, J, K) e^{-2 pi i kx i / nx}
-__global__ void __launch_bounds__(256) k_ls_xsums(Geo g, CFields3 u, int KM, const double2 *__restrict__ xph,
-                                                  double2 *__restrict__ A) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long line = (long long)blockIdx.x * LS_LINES + warp;
-  if (line >= (long long)g.ny * g.nz) return;
-  const int J = (int)(line % g.ny) + 1, K = (int)(line / g.ny) + 1;
-  double2 acc[3][LS_KX];
+__global__ void __launch_bounds__(128) k_ls_xsums(Geo g, CFields3 u, int KM, const double2 *__restrict__ xph,
+                                                  double2 *__restrict__ A, int dep) {
+  constexpr int ROWS = 3 * LS_LINES;
+  __shared__ double tile[ROWS][LS_XT + 1];
+  __shared__ double2 ph[LS_KX][LS_XT];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int line0 = blockIdx.x * LS_LINES, nlines = g.ny * g.nz;
+  // the first cell of each staged line
+  __shared__ int first[LS_LINES];
+  if (tid < LS_LINES) {
+    const int line = min(line0 + tid, nlines - 1);
+    first[tid] = gidx(g, 1, line % g.ny + 1, line / g.ny + 1);
+  }
+  pdl_trigger(dep);
+  pdl_wait(dep);
+  __syncthreads();
+  double a0 = 0.0;
+  double2 acc[LS_KX] = {};
+  for (int x0 = 0; x0 < g.nx; x0 += LS_XT) {
+    const int x = x0 + lane;
+    const bool in = x < g.nx;
 #pragma unroll
-  for (int c = 0; c < 3; c++)
+    for (int c = 0; c < 3; c++) {
+      const double *f = c == 0 ? u.x : c == 1 ? u.y : u.z;
+      double v[LS_LINES / 4];
 #pragma unroll
-    for (int kx = 0; kx < LS_KX; kx++) acc[c][kx] = make_double2(0.0, 0.0);
-  const int row = gidx(g, 1, J, K);
-  for (int i = lane; i < g.nx; i += 32) {
-    const double2 e = xph[i];
-    const double2 z1 = make_double2(e.x, -e.y);
-    const double v[3] = {u.x[row + i], u.y[row + i], u.z[row + i]};
-    double2 zk = make_double2(1.0, 0.0);
+      for (int r = 0; r < LS_LINES / 4; r++) v[r] = in ? f[first[warp + 4 * r] + x] : 0.0;
 #pragma unroll
-    for (int kx = 0; kx < LS_KX; kx++) {
-      if (kx <= KM) {
+      for (int r = 0; r < LS_LINES / 4; r++) tile[c * LS_LINES + warp + 4 * r][lane] = v[r];
+    }
+    if (warp == 0) {
+      const double2 e = in ? xph[x] : make_double2(1.0, 0.0);
+      const double2 z1 = make_double2(e.x, -e.y), z2 = cmul(z1, z1);
+      ph[1][lane] = z1;
+      ph[2][lane] = z2;
+      ph[3][lane] = cmul(z2, z1);
+    }
+    __syncthreads();
+    if (tid < ROWS) {
+#pragma unroll 8
+      for (int i = 0; i < LS_XT; i++) {
+        const double v = tile[tid][i];
+        a0 += v;
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          acc[c][kx].x = fma(v[c], zk.x, acc[c][kx].x);
-          acc[c][kx].y = fma(v[c], zk.y, acc[c][kx].y);
+        for (int kx = 1; kx < LS_KX; kx++) {
+          acc[kx].x = fma(v, ph[kx][i].x, acc[kx].x);
+          acc[kx].y = fma(v, ph[kx][i].y, acc[kx].y);
         }
       }
-      zk = cmul(zk, z1);
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < 3; c++)
-#pragma unroll
-    for (int kx = 0; kx < LS_KX; kx++) {
-      double2 a = acc[c][kx];
-      for (int o = 16; o > 0; o >>= 1) {
-        a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
-        a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
-      }
-      if (lane == 0 && kx <= KM) A[((long long)(c * (KM + 1) + kx) * g.nz + (K - 1)) * g.ny + (J - 1)] = a;
-    }
-}
-
-// y-sums, one block of 128 per (c, kx, z-row): B[((c H + kx) nz + k) W + ky + KM]
-// = sum_j A[...][j] e^{-2 pi i ky j / ny}, each thread over a stride of j,
-// then a fixed-order tree reduction
-__global__ void __launch_bounds__(128) k_ls_ysums(Geo g, const double2 *__restrict__ A, int KM,
-                                                  const double2 *__restrict__ yph, double2 *__restrict__ B) {
-  const int W = 2 * KM + 1;
-  const long long r = blockIdx.x;  // (c H + kx) nz + k
-  const double2 *a = A + r * g.ny;
-  double2 acc[LS_KY];
-#pragma unroll
-  for (int q = 0; q < LS_KY; q++) acc[q] = make_double2(0.0, 0.0);
-  for (int j = threadIdx.x; j < g.ny; j += blockDim.x) {
-    const double2 v = a[j];
-    const double2 e = yph[j];
-    const double2 z1 = make_double2(e.x, -e.y);  // e^{-2 pi i j / ny}
-    double2 zp = v, zm = v;                      // v e^{-+2 pi i ky j / ny}, ky = 0, 1, ..
-    acc[KM] = cadd(acc[KM], v);
-#pragma unroll
-    for (int ky = 1; ky < LS_KX; ky++) {
-      if (ky <= KM) {
-        zp = cmul(zp, z1);
-        zm = cmul(zm, cconj(z1));
-        acc[KM + ky] = cadd(acc[KM + ky], zp);
-        acc[KM - ky] = cadd(acc[KM - ky], zm);
-      }
-    }
-  }
-  __shared__ double2 red[LS_KY][128];
-#pragma unroll
-  for (int q = 0; q < LS_KY; q++) red[q][threadIdx.x] = acc[q];
-  __syncthreads();
-  for (int o = 64; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-#pragma unroll
-      for (int q = 0; q < LS_KY; q++) red[q][threadIdx.x] = cadd(red[q][threadIdx.x], red[q][threadIdx.x + o]);
     }
     __syncthreads();
   }
-  if ((int)threadIdx.x < W) B[r * W + threadIdx.x] = red[threadIdx.x][0];
+  acc[0] = make_double2(a0, 0.0);
+  if (tid < ROWS && line0 + tid % LS_LINES < nlines) {
+    const int c = tid / LS_LINES, line = line0 + tid % LS_LINES;
+#pragma unroll
+    for (int kx = 0; kx < LS_KX; kx++)
+      if (kx <= KM) A[(long long)(c * (KM + 1) + kx) * nlines + line] = acc[kx];
+  }
 }
 
-// z-sums, one block of 128 per (c, kx, ky): Gm[((c H + kx) W + ky + KM) W + kz + KM]
-// = sum_k B[...][k] e^{-2 pi i kz k / nz} (the modes u_hat), fixed-order tree
-__global__ void __launch_bounds__(128) k_ls_zsums(Geo g, const double2 *__restrict__ B, int KM,
-                                                  const double2 *__restrict__ zph, double2 *__restrict__ Gm) {
+// out[r W + q] = sum_i in[base(r) + i stride] e^{-2 pi i (q - KM) i / n}, with
+// base(r) = (r / inner) outer + r % inner: the y-sums (rows of A: inner 1)
+// and the z-sums (rows of B, k strided by W: inner W).  Thread (row, output
+// q < W, part of the row): 8 rows in quarters for the many y-rows, one row in
+// 32 parts for the at most 84 z-rows.
+constexpr int LS_STHREADS = 8 * LS_KY * 4;
+template <int ROWS, int PARTS>
+__global__ void __launch_bounds__(LS_STHREADS)
+    k_ls_sums(int rows, int n, int inner, long long outer, int stride, const double2 *in, int KM,
+              const double2 *__restrict__ ph, double2 *__restrict__ out, int dep) {
   const int W = 2 * KM + 1;
-  const int r = blockIdx.x;  // (c H + kx) W + ky + KM
-  const int ckx = r / W, kyi = r % W;
-  double2 acc[LS_KY];
-#pragma unroll
-  for (int q = 0; q < LS_KY; q++) acc[q] = make_double2(0.0, 0.0);
-  for (int k = threadIdx.x; k < g.nz; k += blockDim.x) {
-    const double2 v = B[((long long)ckx * g.nz + k) * W + kyi];
-    const double2 e = zph[k];
-    const double2 z1 = make_double2(e.x, -e.y);  // e^{-2 pi i k / nz}
-    double2 zp = v, zm = v;
-    acc[KM] = cadd(acc[KM], v);
-#pragma unroll
-    for (int kz = 1; kz < LS_KX; kz++) {
-      if (kz <= KM) {
-        zp = cmul(zp, z1);
-        zm = cmul(zm, cconj(z1));
-        acc[KM + kz] = cadd(acc[KM + kz], zp);
-        acc[KM - kz] = cadd(acc[KM - kz], zm);
-      }
+  static_assert(ROWS * PARTS * LS_KY == LS_STHREADS, "one thread per row, part and output");
+  __shared__ double2 part[PARTS][ROWS][LS_KY];
+  const int tid = threadIdx.x;
+  const int q = tid % LS_KY, p = (tid / LS_KY) % PARTS, rl = tid / (LS_KY * PARTS);
+  const int r = blockIdx.x * ROWS + rl;
+  pdl_trigger(dep);
+  pdl_wait(dep);
+  if (r < rows && q < W) {
+    const double2 *a = in + (r / inner) * outer + r % inner;
+    const int per = (n + PARTS - 1) / PARTS, i0 = p * per, i1 = min(n, i0 + per);
+    // phase index ky i mod n, advanced by ky mod n per term
+    const int ky = q - KM, step = ky < 0 ? ky + n : ky;
+    int m = (int)((long long)step * i0 % n);
+    double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int i = i0; i < i1; i++) {
+      acc = cadd(acc, cmul(a[(long long)i * stride], cconj(ph[m])));
+      m += step;
+      if (m >= n) m -= n;
     }
+    part[p][rl][q] = acc;
   }
-  __shared__ double2 red[LS_KY][128];
-#pragma unroll
-  for (int q = 0; q < LS_KY; q++) red[q][threadIdx.x] = acc[q];
   __syncthreads();
-  for (int o = 64; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-#pragma unroll
-      for (int q = 0; q < LS_KY; q++) red[q][threadIdx.x] = cadd(red[q][threadIdx.x], red[q][threadIdx.x + o]);
-    }
-    __syncthreads();
+  if (r < rows && q < W && p == 0) {
+    double2 sum = part[0][rl][q];
+    for (int i = 1; i < PARTS; i++) sum = cadd(sum, part[i][rl][q]);
+    out[(long long)r * W + q] = sum;
   }
-  if ((int)threadIdx.x < W) Gm[(long long)r * W + threadIdx.x] = red[threadIdx.x][0];
 }
 
-// One block: the shell energies of the modes in Gm into E[0..nb), clamp
-// factors into f, the corrections G = (f(shell) - 1) u_hat / N in place, and
-// Hz[((c H + kx) W + ky + KM) nz + k] = sum_kz G e^{+2 pi i kz k / nz};
+// floor(sqrt(k2)) for the small integers here
+__device__ __forceinline__ int ls_shell(int k2) {
+  int sh = (int)sqrtf((float)k2);
+  while (sh * sh > k2) sh--;
+  while ((sh + 1) * (sh + 1) <= k2) sh++;
+  return sh;
+}
+
+// One block: the shell energies of the modes u_hat in Gm into E[0..nb), clamp
+// factors into f, the corrections G = (f(shell) - 1) u_hat / N in place;
 // eref[s] < 0 leaves shell s unforced.
-__global__ void __launch_bounds__(1024) k_ls_modes(Geo g, int KM, double2 *__restrict__ Gm,
-                                                   double2 *__restrict__ Hz, double *__restrict__ E,
-                                                   const double *__restrict__ eref,
-                                                   double *__restrict__ f, int nb,
-                                                   const double2 *__restrict__ zph) {
+__global__ void __launch_bounds__(256) k_ls_modes(Geo g, int KM, double2 *Gm, double *E,
+                                                  const double *__restrict__ eref, double *f, int nb, int dep) {
   const int W = 2 * KM + 1, H = KM + 1;
   const double N = (double)g.nx * g.ny * g.nz;
   const int nM = 3 * H * W * W;
-  // per-mode energies in shared memory (shell in the low bits), then the
-  // shell sums by one thread in a fixed order, the factors, the corrections
   __shared__ double em[3 * LS_KX * LS_KY * LS_KY];
-  __shared__ int sm[3 * LS_KX * LS_KY * LS_KY];
+  __shared__ signed char sm[3 * LS_KX * LS_KY * LS_KY];
+  __shared__ double fs[LS_KX];
+  pdl_trigger(dep);
+  pdl_wait(dep);
   for (int t = threadIdx.x; t < nM; t += blockDim.x) {
-    const int kzi = t % W;
-    const int r = t / W;
-    const int kyi = r % W, kx = (r / W) % H;
-    const int ky = kyi - KM, kz = kzi - KM;
-    const int k2 = kx * kx + ky * ky + kz * kz;
-    int sh = (int)sqrt((double)k2);
-    while (sh * sh > k2) sh--;
-    while ((sh + 1) * (sh + 1) <= k2) sh++;
+    const int kzi = t % W, r = t / W;
+    const int kx = (r / W) % H, ky = r % W - KM, kz = kzi - KM;
     const double2 a = Gm[t];
     em[t] = (kx > 0 ? 2.0 : 1.0) * (a.x * a.x + a.y * a.y) / 2 / (N * N);
-    sm[t] = sh;
+    sm[t] = (signed char)ls_shell(kx * kx + ky * ky + kz * kz);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double acc[LS_KX] = {0.0, 0.0, 0.0, 0.0};
-    for (int t = 0; t < nM; t++) {
-      const int sh = sm[t];
-#pragma unroll
-      for (int q = 0; q < LS_KX; q++) acc[q] += (sh == q) ? em[t] : 0.0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < nb) {
+    double acc = 0.0;
+    for (int t = lane; t < nM; t += 32) acc += sm[t] == warp ? em[t] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) {
+      const double fac = (eref[warp] >= 0 && acc > 0) ? sqrt(eref[warp] / acc) : 1.0;
+      E[warp] = acc;
+      f[warp] = fac;
+      fs[warp] = fac;
     }
-    for (int q = 0; q < nb; q++) {
-      E[q] = acc[q];
-      f[q] = (eref[q] >= 0 && acc[q] > 0) ? sqrt(eref[q] / acc[q]) : 1.0;
-    }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < nM; t += blockDim.x) {
-    const int kzi = t % W;
-    const int r = t / W;
-    const int kyi = r % W, kx = (r / W) % H;
-    const int ky = kyi - KM, kz = kzi - KM;
-    const int k2 = kx * kx + ky * ky + kz * kz;
-    int sh = (int)sqrt((double)k2);
-    while (sh * sh > k2) sh--;
-    while ((sh + 1) * (sh + 1) <= k2) sh++;
-    const double fac = sh < nb ? f[sh] - 1.0 : 0.0;
-    Gm[t] = cscale(Gm[t], fac / N);
-  }
-  __syncthreads();
-  const int nH = 3 * H * W * g.nz;
-  for (int t = threadIdx.x; t < nH; t += blockDim.x) {
-    const int k = t % g.nz, r = t / g.nz;  // r = (c H + kx) W + ky + KM
-    double2 sacc = make_double2(0.0, 0.0);
-    for (int kzi = 0; kzi < W; kzi++)
-      sacc = cadd(sacc, cmul(Gm[r * W + kzi], ls_phase_tab((kzi - KM) * k, g.nz, 1.0, zph)));
-    Hz[t] = sacc;
-  }
+  for (int t = threadIdx.x; t < nM; t += blockDim.x)
+    Gm[t] = cscale(Gm[t], sm[t] < nb ? (fs[sm[t]] - 1.0) / N : 0.0);
 }
 
 // u_c(i, J, K) += Re sum_{kx, ky, kz} w(kx) G e^{+2 pi i (kx i/nx + ky j/ny + kz k/nz)},
-// then the periodic ghost images of the updated cells
-__global__ void __launch_bounds__(256) k_ls_correct(Geo g, Fields3 u, int KM,
-                                                    const double2 *__restrict__ Hz,
+// then the periodic ghost images of the updated cells.  grid (groups of
+// LS_CLINES rows, nz)
+__global__ void __launch_bounds__(256, 4) k_ls_correct(Geo g, Fields3 u, int KM, const double2 *Gm,
                                                     const double2 *__restrict__ xph,
-                                                    const double2 *__restrict__ yph) {
+                                                    const double2 *__restrict__ yph,
+                                                    const double2 *__restrict__ zph, int dep) {
   const int W = 2 * KM + 1, H = KM + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long line = (long long)blockIdx.x * LS_LINES + warp;
-  if (line >= (long long)g.ny * g.nz) return;
-  const int j = (int)(line % g.ny), k = (int)(line / g.ny);
-  const int J = j + 1, K = k + 1;
-  // P[c][kx] = sum_{ky, kz} G e^{i (ky j / ny + kz k / nz)}: lane t < 3 H forms one
-  double2 P = make_double2(0.0, 0.0);
-  if (lane < 3 * H) {
-    const int c = lane / H, kx = lane % H;
-    for (int kyi = 0; kyi < W; kyi++)
-      P = cadd(P, cmul(Hz[((long long)(c * H + kx) * W + kyi) * g.nz + k],
-                       ls_phase_tab((kyi - KM) * j, g.ny, 1.0, yph)));
-    if (kx > 0) P = cscale(P, 2.0);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int k = blockIdx.y, j0 = blockIdx.x * LS_CLINES;
+  __shared__ double2 Hz[3 * LS_KX * LS_KY];          // [c H + kx][ky]: sum over kz at this k
+  __shared__ double2 P[LS_CLINES][3][LS_KX];         // sum over ky at each line, w(kx) applied
+  pdl_trigger(dep);
+  pdl_wait(dep);
+  if (tid < 3 * H * W) {
+    double2 a = make_double2(0.0, 0.0);
+    for (int kzi = 0; kzi < W; kzi++)
+      a = cadd(a, cmul(Gm[tid * W + kzi], ls_phase_tab((kzi - KM) * k, g.nz, 1.0, zph)));
+    Hz[tid] = a;
   }
-  double2 Pc[3][LS_KX];
-#pragma unroll
-  for (int c = 0; c < 3; c++)
-#pragma unroll
-    for (int kx = 0; kx < LS_KX; kx++) {
-      const int src = c * H + kx;
-      const double px = __shfl_sync(0xffffffffu, P.x, src < 32 ? src : 0);
-      const double py = __shfl_sync(0xffffffffu, P.y, src < 32 ? src : 0);
-      Pc[c][kx] = kx <= KM ? make_double2(px, py) : make_double2(0.0, 0.0);
+  __syncthreads();
+  if (tid < LS_CLINES * 3 * LS_KX) {
+    const int kx = tid % LS_KX, c = (tid / LS_KX) % 3, l = tid / (3 * LS_KX), j = j0 + l;
+    double2 a = make_double2(0.0, 0.0);
+    if (kx <= KM && j < g.ny) {
+      for (int kyi = 0; kyi < W; kyi++)
+        a = cadd(a, cmul(Hz[(c * H + kx) * W + kyi], ls_phase_tab((kyi - KM) * j, g.ny, 1.0, yph)));
+      if (kx > 0) a = cscale(a, 2.0);
     }
+    P[l][c][kx] = a;
+  }
+  __syncthreads();
   double *fc[3] = {u.x, u.y, u.z};
-  const int row = gidx(g, 1, J, K);
   for (int i = lane; i < g.nx; i += 32) {
-    const double2 z1 = xph[i];
-    double d[3] = {0.0, 0.0, 0.0};
-    double2 zk = make_double2(1.0, 0.0);
+    const double2 z1 = xph[i], z2 = cmul(z1, z1), z3 = cmul(z2, z1);
 #pragma unroll
-    for (int kx = 0; kx < LS_KX; kx++) {
+    for (int q = 0; q < LS_CLINES / 8; q++) {
+      const int l = warp + 8 * q, J = j0 + l + 1;
+      if (J > g.ny) continue;
+      const int c0 = gidx(g, i + 1, J, k + 1);
+      double v[3];
 #pragma unroll
-      for (int c = 0; c < 3; c++) d[c] += Pc[c][kx].x * zk.x - Pc[c][kx].y * zk.y;
-      zk = cmul(zk, z1);
-    }
+      for (int c = 0; c < 3; c++) v[c] = fc[c][c0];
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-      store_img(fc[c], g, i + 1, J, K, fc[c][row + i] + d[c], STAG_P);
+      for (int c = 0; c < 3; c++) {
+        const double2 *p = P[l][c];
+        const double d = p[0].x + ((p[1].x * z1.x - p[1].y * z1.y) +
+                                   ((p[2].x * z2.x - p[2].y * z2.y) + (p[3].x * z3.x - p[3].y * z3.y)));
+        fc[c][c0] = v[c] + d;
+        if (img_edge(g, i + 1, J, k + 1))
+          store_images_of(fc[c], g.nx, g.ny, g.nz, g.NX, g.NY, g.wall, i + 1, J, k + 1, v[c] + d, STAG_P);
+      }
     }
   }
 }

@@ -25,6 +25,8 @@
 #include "../../include/dnsb_cnn.h"
 #include "cnn.cuh"
 #include "cnn_host.h"
+#include "launch.h"
+#include "pdl.cuh"
 
 using namespace dnsb::cnn;
 
@@ -111,74 +113,91 @@ struct Packs {
   __nv_bfloat16 *d[NL];  // transposed (backward-data) B operands, L >= 1
 };
 
-// which parameter index p is: layer, and (t, co, ci) or bias co
-__device__ inline void locate(const KernelLayout &k, long p, int &L, int &t, int &co, int &ci,
-                              bool &bias) {
-  L = 0;
-  while (L < NL - 1 && p >= k.w[L + 1]) L++;
-  if (p >= k.b[L]) {
-    bias = true;
-    co = (int)(p - k.b[L]);
-    t = ci = 0;
-  } else {
-    bias = false;
-    long r = p - k.w[L];
-    ci = (int)(r % k.cin[L]);
-    r /= k.cin[L];
-    co = (int)(r % k.cout[L]);
-    t = (int)(r / k.cout[L]);
-  }
-}
+// the split-K partials of the four weight gradients (k_wgrad's layout)
+struct Partials {
+  const float *part[NL];
+  int nsplit[NL];
+};
 
-// Adam update (when lr > 0 or adam != 0) and BF16 packing of every weight.
-__global__ void k_adam_pack(KernelLayout k, float *params, const float *grads, float *m, float *v,
-                            int adam, float lr, const long long *step, Packs packs) {
-  const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= k.total) return;
-  float w = params[p];
+// With `reduce` every parameter's gradient from the split-K partials of its
+// layer, with `adam` the Adam update, and the BF16 packing of every weight.
+// Threads run over (tap, ci, co) with co fastest, the partials' order; eight
+// threads share a parameter's splits (each adds every eighth, the eight sums
+// are added in order).  One launch at the step's end: as four reductions
+// between the backward kernels (5.2 us each, ordinary launches that kept the
+// next convolution from starting early) and an Adam launch (5.9 us, two double
+// pow per thread) they were 27 us of a 545 us training step.
+constexpr int UP_PARTS = 8, UP_PARAMS = 32;
+__global__ void __launch_bounds__(UP_PARTS *UP_PARAMS)
+    k_update(KernelLayout k, Partials pt, int reduce, float *params, float *grads, float *m, float *v, int adam,
+             float lr, const long long *step, Packs packs) {
+  __shared__ float corr[2];
+  __shared__ float sums[UP_PARTS][UP_PARAMS];
+  const int lp = threadIdx.x % UP_PARAMS, part = threadIdx.x / UP_PARAMS;
+  if (adam && threadIdx.x < 2) {  // 1 - beta^(step + 1), by squaring
+    double b = threadIdx.x ? (double)0.999f : (double)0.9f, q = 1.0;
+    for (unsigned long long n = (unsigned long long)*step + 1; n; n >>= 1, b *= b)
+      if (n & 1) q *= b;
+    corr[threadIdx.x] = (float)(1.0 - q);
+  }
+  long i = (long)blockIdx.x * UP_PARAMS + lp;
+  const bool in = i < k.total;
+  int L = 0, t = 0, ci = 0, co = 0;
+  bool bias = false;
+  long p = 0;
+  if (in) {
+    while (L < NL - 1 && i >= k.w[L + 1]) L++;
+    i -= k.w[L];
+    const int cin = k.cin[L], cout = k.cout[L], nw = 27 * cin * cout;
+    bias = i >= nw;
+    if (bias) {
+      co = (int)(i - nw);
+    } else {
+      const int r = (int)i / cout;
+      co = (int)i - r * cout;
+      t = r / cin;
+      ci = r - t * cin;
+    }
+    p = bias ? k.b[L] + co : k.w[L] + ((long)t * cout + co) * cin + ci;
+  }
+  if (reduce) {
+    float g = 0.f;
+    if (in) {
+      const int cich = L == 0 ? 2 : 4, N = 3 * 8 * (L == 3 ? 2 : 4);
+      const int dz = bias ? 0 : t / 9, row = bias ? 3 * 8 * cich : (t % 3) * 8 * cich + ci;
+      const int n = bias ? co : (t / 3) % 3 * (N / 3) + co;
+      const float *q = pt.part[L] + ((long)dz * 128 + row) * N + n;
+      const long stride = 3L * 128 * N;
+      const int ns = pt.nsplit[L];
+#pragma unroll 8
+      for (int sp = part; sp < ns; sp += UP_PARTS) g += q[sp * stride];
+    }
+    sums[part][lp] = g;
+  }
+  __syncthreads();
+  if (part || !in) return;
+  float w = params[p], g;
+  if (reduce) {
+    g = 0.f;
+#pragma unroll
+    for (int q = 0; q < UP_PARTS; q++) g += sums[q][lp];
+    grads[p] = g;
+  } else {
+    g = grads[p];
+  }
   if (adam) {
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const double tt = (double)(*step + 1);
-    const float c1 = (float)(1.0 - pow((double)b1, tt));
-    const float c2 = (float)(1.0 - pow((double)b2, tt));
-    const float g = grads[p];
     const float mm = b1 * m[p] + (1.f - b1) * g;
     const float vv = b2 * v[p] + (1.f - b2) * g * g;
     m[p] = mm;
     v[p] = vv;
-    w = w - lr * ((mm / c1) / (sqrtf(vv / c2) + eps));
+    w = w - lr * ((mm / corr[0]) / (sqrtf(vv / corr[1]) + eps));
     params[p] = w;
   }
-  int L, t, co, ci;
-  bool bias;
-  locate(k, p, L, t, co, ci, bias);
   if (bias) return;
   const __nv_bfloat16 wb = __float2bfloat16_rn(w);
   packs.f[L][pack_fwd(L, t, co, ci)] = wb;
   if (L > 0) packs.d[L][pack_bwd(L, t, co, ci)] = wb;
-}
-
-// split-K partials of one layer's weight gradient -> grads (fixed order)
-__global__ void k_wgrad_reduce(const float *partial, int ngroups, int nsplit, int N, int G,
-                               int cipad, int cin, int cout, int ones_slot, float *gw, float *gb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nw = 27 * cout * cin;
-  if (i >= nw + cout) return;
-  int gi, m, n;
-  if (i < nw) {
-    const int ci = i % cin, co = (i / cin) % cout, t = i / (cin * cout);
-    gi = t / G;
-    m = (t % G) * cipad + ci;
-    n = co;
-  } else {
-    gi = ngroups - 1;
-    m = ones_slot * cipad;
-    n = i - nw;
-  }
-  float s = 0.f;
-  for (int sp = 0; sp < nsplit; sp++) s += partial[(((long)sp * ngroups + gi) * 128 + m) * N + n];
-  if (i < nw) gw[i] = s;
-  else gb[n] = s;
 }
 
 __device__ inline unsigned long long splitmix(unsigned long long x) {
@@ -194,35 +213,41 @@ __device__ inline uint4 chunk3(float a, float b, float c) {
 }
 
 // random crops of the dataset: input with its halo (chunk 0 of x0) and the
-// normalised targets of the crop
-__global__ void k_crops(const float *data, int nsnap, int n, int B, int crop, int P,
-                        unsigned long long seed, const long long *step, uint4 *x0, float4 *tgt) {
-  const long P3 = (long)P * P * P, c3 = (long)crop * crop * crop;
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long)B * (P3 + c3)) return;
-  const bool tpart = i >= (long)B * P3;
-  const long r = tpart ? i - (long)B * P3 : i;
-  const int b = (int)(tpart ? r / c3 : r / P3);
-  long v = tpart ? r % c3 : r % P3;
-  const int side = tpart ? crop : P;
-  const int x = (int)(v % side), y = (int)((v / side) % side), z = (int)(v / ((long)side * side));
-  const unsigned long long key = (unsigned long long)(*step) * 64ull + (unsigned long long)b;
-  const unsigned long long h0 = splitmix(seed ^ splitmix(4 * key));
-  const int snap = (int)(h0 % (unsigned long long)nsnap);
-  const int ox = (int)(splitmix(h0 + 1) % (unsigned long long)n);
-  const int oy = (int)(splitmix(h0 + 2) % (unsigned long long)n);
-  const int oz = (int)(splitmix(h0 + 3) % (unsigned long long)n);
-  const long n3 = (long)n * n * n;
-  const float *s = data + (long)snap * 9 * n3;
-  const int h = tpart ? 0 : HALO;
-  const int gx = ((ox + x - h) % n + n) % n, gy = ((oy + y - h) % n + n) % n, gz = ((oz + z - h) % n + n) % n;
-  const long gi = ((long)gz * n + gy) * n + gx;
-  if (!tpart) {
-    x0[(long)b * 2 * P3 + v] = chunk3(s[gi], s[n3 + gi], s[2 * n3 + gi]);
-  } else {
-    const long o = (((long)b * P + z) * P + y) * P + x;
-    tgt[2 * o] = make_float4(s[3 * n3 + gi], s[4 * n3 + gi], s[5 * n3 + gi], s[6 * n3 + gi]);
-    tgt[2 * o + 1] = make_float4(s[7 * n3 + gi], s[8 * n3 + gi], 0.f, 0.f);
+// normalised targets of the crop.  A block takes one z plane of one sample
+// (grid z: 0 input, 1 targets), draws the crop once and walks its rows; one
+// thread per voxel with the draw's four 64-bit remainders and the index
+// divisions of its own took 22.2 us per batch of 8 crops of 32^3.
+__global__ void __launch_bounds__(256) k_crops(const float *data, int nsnap, int n, int crop, int P,
+                                               unsigned long long seed, const long long *step, uint4 *x0,
+                                               float4 *tgt) {
+  const int b = blockIdx.y, z = blockIdx.x;
+  const bool tpart = blockIdx.z;
+  const int side = tpart ? crop : P, h = tpart ? 0 : HALO;
+  if (z >= side) return;
+  __shared__ int draw[4];  // snapshot, origin x, y, z
+  if (threadIdx.x < 4) {
+    const unsigned long long key = (unsigned long long)(*step) * 64ull + (unsigned long long)b;
+    const unsigned long long h0 = splitmix(seed ^ splitmix(4 * key));
+    const int i = threadIdx.x;
+    draw[i] = i == 0 ? (int)(h0 % (unsigned long long)nsnap)
+                     : (int)(splitmix(h0 + i) % (unsigned long long)n);
+  }
+  __syncthreads();
+  const long n3 = (long)n * n * n, P3 = (long)P * P * P;
+  const float *s = data + (long)draw[0] * 9 * n3;
+  // (crop + 2 HALO may exceed n: the box wraps as often as it takes)
+  auto wrap = [n](int a) { return a >= 0 && a < n ? a : ((a % n) + n) % n; };
+  const float *plane = s + (long)wrap(draw[3] + z - h) * n * n;
+  for (int i = threadIdx.x; i < side * side; i += blockDim.x) {
+    const int y = i / side, x = i - y * side;
+    const int gi = wrap(draw[2] + y - h) * n + wrap(draw[1] + x - h);
+    if (!tpart) {
+      x0[(long)b * 2 * P3 + ((long)z * P + y) * P + x] = chunk3(plane[gi], plane[n3 + gi], plane[2 * n3 + gi]);
+    } else {
+      const long o = (((long)b * P + z) * P + y) * P + x;
+      tgt[2 * o] = make_float4(plane[3 * n3 + gi], plane[4 * n3 + gi], plane[5 * n3 + gi], plane[6 * n3 + gi]);
+      tgt[2 * o + 1] = make_float4(plane[7 * n3 + gi], plane[8 * n3 + gi], 0.f, 0.f);
+    }
   }
 }
 
@@ -255,7 +280,9 @@ __global__ void k_batch_in(const float *x, const float *t, int B, int crop, int 
 // grid (ceil(P / blockDim.x), P, P): x along the threads, y and z from the
 // block (no division per voxel); the halo (HALO < n) wraps by one correction
 __global__ void k_infer_in(const double *v, const double *ux, const double *uy, const double *uz,
-                           int n, int P, const float *in_scale, uint4 *x0) {
+                           int n, int P, const float *in_scale, uint4 *x0, int dep) {
+  dnsb::pdl_trigger(dep);
+  dnsb::pdl_wait(dep);
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
   if (x >= P) return;
   const long i = ((long)z * P + y) * P + x;
@@ -308,7 +335,7 @@ struct Volume {
   CUtensorMap fwd[NL], bwd[NL], flatA[NL], flatB[NL];
   int Rf = 0, Rb = 0;          // patch rows of forward / transposed reads
   int subf = 1, subb = 1;      // 126-output sub-tiles per plane load (1-4), forward / transposed
-  int Rw = 0, wstages = 0;     // weight gradient: rows per K-block, K-blocks in flight
+  int Rw[NL] = {};             // weight gradient: rows per K-block
 };
 
 struct Prof {
@@ -330,6 +357,7 @@ struct dnsb_cnn {
   bool have_tr = false, have_inf = false;
   float *params = nullptr, *grads = nullptr, *m = nullptr, *v = nullptr;
   Packs packs{};
+  Partials parts{};            // of the last backward pass
   float *scales = nullptr;     // in[3] (pad 4), out[6]
   float *partial[NL] = {};
   long partial_n[NL] = {};
@@ -428,13 +456,14 @@ int patch_rows(int P, int s, int e, int sub) {
 // copy is byte-exact (no conversion; out-of-bounds elements read as zero).
 // Conv plane: dims {2P (x and 8 channels), P (y), P (z), chunks * B}, box
 // {2P, R, 1, chunks} -> shared memory [chunk][row][x][16 B] (one ring slot).
-int make_map_patch(dnsb_cnn *c, CUtensorMap *m, void *base, int P, int chunks, int B, int R) {
+// The weight gradient takes R rows of one box of all chunks, or of one.
+int make_map_patch(dnsb_cnn *c, CUtensorMap *m, void *base, int P, int chunks, int B, int R, int boxch) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cfail(c, DNSB_ECUDA, "cuTensorMapEncodeTiled is not available");
   if (2 * P > 256 || R > 256 || chunks > 256) return cfail(c, DNSB_EUNSUP, "TMA box beyond 256 (P %d, R %d)", P, R);
   const cuuint64_t dims[4] = {2ull * P, (cuuint64_t)P, (cuuint64_t)P, (cuuint64_t)chunks * B};
   const cuuint64_t strides[3] = {16ull * P, 16ull * P * P, 16ull * P * P * P};
-  const cuuint32_t box[4] = {(cuuint32_t)(2 * P), (cuuint32_t)R, 1, (cuuint32_t)chunks};
+  const cuuint32_t box[4] = {(cuuint32_t)(2 * P), (cuuint32_t)R, 1, (cuuint32_t)boxch};
   const cuuint32_t es[4] = {1, 1, 1, 1};
   const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, base, dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -465,6 +494,29 @@ int setup_conv_attr(dnsb_cnn *c, size_t smem) {
   if (smem > (size_t)MAX_SMEM) return cfail(c, DNSB_EUNSUP, "convolution needs %zu bytes of shared memory", smem);
   CC(c, cudaFuncSetAttribute(k_conv<CI, CO, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   return 0;
+}
+
+// Weight gradient: shared memory of K-blocks of R rows, and the rows with the
+// least estimated time: a plane's Do + 2 rows in ceil((Do + 2) / R) blocks of
+// R P positions padded to 16, about 48 positions' worth of waits per block, and
+// 15 % where the padding needs a copy per chunk (crop 32: 4 rows of 40).
+size_t wgrad_smem(int P, int R, int ci, int co) {
+  const size_t chunk = (size_t)((R * P + 15) / 16 * 16) * 16;
+  return WG_PLANES * 4 * ci * chunk + WG_GRADS * 3 * co * chunk + 256 + 1024;
+}
+int wgrad_rows(int P, int Do, int ci, int co) {
+  int best = 0;
+  double least = 0;
+  for (int r = 1; r <= std::min(16, P); r++) {
+    if (wgrad_smem(P, r, ci, co) > (size_t)MAX_SMEM) break;
+    const int kb = r * P, kbp = (kb + 15) / 16 * 16;
+    const double t = (Do + 2 + r - 1) / r * (kbp + 48) * (kb == kbp ? 1.0 : 1.15);
+    if (!best || t <= least) {
+      best = r;
+      least = t;
+    }
+  }
+  return best;
 }
 
 int alloc_volume(dnsb_cnn *c, Volume &V, int side, int B, bool training) {
@@ -513,49 +565,17 @@ int alloc_volume(dnsb_cnn *c, Volume &V, int side, int B, bool training) {
       return cfail(c, DNSB_EUNSUP, "side %d too large: a convolution's plane ring (%d slots of %u bytes) "
                    "does not fit in shared memory", side, RING_MIN, sl);
   }
-  if (training) {
-    // weight-gradient K-blocks of R whole rows (R P positions, a multiple of
-    // 16): the most rows with at least two blocks in flight (up to four when
-    // they fit), at most 16 rows and P -- fewer, larger copies win (crop 32:
-    // 8 rows x 2 blocks 0.289 ms, 6 x 3 0.305, 4 x 4 0.358 per training
-    // step); DNSB_WGROWS / DNSB_WGSTAGES override
-    int best = 0, bstages = 0;
-    for (int r = 1; r <= std::min(16, P); r++) {
-      if ((r * P) % 16) continue;
-      // 16 chunks of taps + 4 of g, 16 bytes each, per position
-      const size_t stage = ((size_t)320 * r * P + 1023) & ~(size_t)1023;
-      const int ns = (int)std::min<size_t>(WG_STAGES, ((size_t)MAX_SMEM - 1280) / stage);
-      if (ns >= 2) {
-        best = r;
-        bstages = ns;
-      }
-    }
-    const char *er = getenv("DNSB_WGROWS"), *es = getenv("DNSB_WGSTAGES");
-    if (er) {
-      const int r = atoi(er);
-      const size_t stage = (((size_t)320 * r * P) + 1023) & ~(size_t)1023;
-      if (r >= 1 && r <= std::min(16, P) && (r * P) % 16 == 0 && 2 * stage + 1280 <= (size_t)MAX_SMEM) {
-        best = r;
-        bstages = (int)std::min<size_t>(WG_STAGES, ((size_t)MAX_SMEM - 1280) / stage);
-      }
-    }
-    if (es && best) {
-      const size_t stage = (((size_t)320 * best * P) + 1023) & ~(size_t)1023;
-      const int ns = atoi(es);
-      if (ns >= 2 && ns <= WG_STAGES && ns * stage + 1280 <= (size_t)MAX_SMEM) bstages = ns;
-    }
-    if (!best)
-      return cfail(c, DNSB_EUNSUP, "crop side %d: no weight-gradient block of whole rows fits (side + 8 must "
-                   "allow r (side + 8) to be a multiple of 16 with r <= 16)", side);
-    V.Rw = best;
-    V.wstages = bstages;
-  }
+  if (training)
+    for (int L = 0; L < NL; L++)
+      if (!(V.Rw[L] = wgrad_rows(P, P - 2 * (L + 1), CICH[L], COCH[L])))
+        return cfail(c, DNSB_EUNSUP, "crop side %d: no weight-gradient block of whole rows fits", side);
   for (int L = 0; L < NL; L++) {
-    if ((rc = make_map_patch(c, &V.fwd[L], V.in[L], P, CICH[L], B, V.Rf))) return rc;
+    if ((rc = make_map_patch(c, &V.fwd[L], V.in[L], P, CICH[L], B, V.Rf, CICH[L]))) return rc;
     if (training) {
-      if ((rc = make_map_patch(c, &V.flatA[L], V.in[L], P, CICH[L], B, V.Rw))) return rc;
-      if ((rc = make_map_patch(c, &V.flatB[L], V.gz[L], P, COCH[L], B, V.Rw))) return rc;
-      if (L > 0 && (rc = make_map_patch(c, &V.bwd[L], V.gz[L], P, COCH[L], B, V.Rb))) return rc;
+      const bool whole = V.Rw[L] * P % 16 == 0;
+      if ((rc = make_map_patch(c, &V.flatA[L], V.in[L], P, CICH[L], B, V.Rw[L], whole ? CICH[L] : 1))) return rc;
+      if ((rc = make_map_patch(c, &V.flatB[L], V.gz[L], P, COCH[L], B, V.Rw[L], whole ? COCH[L] : 1))) return rc;
+      if (L > 0 && (rc = make_map_patch(c, &V.bwd[L], V.gz[L], P, COCH[L], B, V.Rb, COCH[L]))) return rc;
     }
   }
   return 0;
@@ -660,31 +680,21 @@ template <int CI, int CO>
 int run_wgrad(dnsb_cnn *c, Volume &V, int L) {
   WgradArgs a{};
   a.P = V.P;
-  a.Pz = V.P;
   a.B = V.B;
   a.Do = V.P - 2 * (L + 1);
-  a.R = V.Rw;
-  a.KB = V.Rw * V.P;
-  a.stages = V.wstages;
-  a.kpp = (a.Do + a.R - 1) / a.R;
-  a.nk = V.B * a.Do * a.kpp;
-  constexpr int G = 16 / CI;
-  a.ngroups = (NTAPS + G - 1) / G;
-  a.ones_slot = NTAPS - (a.ngroups - 1) * G;
-  a.a_bytes = (uint32_t)G * CI * a.KB * 16;
-  a.stage_bytes = ((a.a_bytes + (uint32_t)CO * a.KB * 16) + 1023) & ~1023u;
+  a.R = V.Rw[L];
+  a.KB = a.R * V.P;
+  a.KBp = (a.KB + 15) / 16 * 16;
+  a.whole = a.KB == a.KBp;
+  a.kpp = (a.Do + 2 + a.R - 1) / a.R;
+  a.h_bytes = 4u * CI * a.KBp * 16;
+  a.g_bytes = 3u * CO * a.KBp * 16;
   a.wait_limit = WAIT_LIMIT;
   a.err = c->deverr;
-  const size_t smem = (size_t)a.stages * a.stage_bytes + 256 + 1024;
-  if (smem > (size_t)MAX_SMEM) return cfail(c, DNSB_EUNSUP, "weight gradient needs %zu bytes", smem);
-  CC(c, cudaFuncSetAttribute(k_wgrad<CI, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_wgrad<CI, CO>, NTHREADS, smem) != cudaSuccess || per < 1) {
-    cudaGetLastError();
-    per = 1;
-  }
-  a.nsplit = std::max(1, std::min(a.nk, (c->nsm * per) / a.ngroups));
-  const long need = (long)a.nsplit * a.ngroups * 128 * (8 * CO);
+  const size_t smem = wgrad_smem(V.P, a.R, CI, CO);
+  CC(c, dnsb::raise_smem(c->device, k_wgrad<CI, CO>, smem));
+  a.nsplit = (int)std::max(1LL, std::min<long long>(c->nsm, (long long)a.B * a.kpp * a.Do));
+  const long need = (long)a.nsplit * 3 * 128 * (3 * 8 * CO);
   if (need > c->partial_n[L]) return cfail(c, DNSB_EUNSUP, "weight-gradient partials: %ld > %ld", need, c->partial_n[L]);
   a.partial = c->partial[L];
   const double flops = 2.0 * 27 * CIN[L] * COUT[L] * V.B * pow((double)a.Do, 3);
@@ -693,7 +703,7 @@ int run_wgrad(dnsb_cnn *c, Volume &V, int L) {
   {
     // programmatic dependent launch (the kernel waits before any memory access)
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(a.ngroups * a.nsplit));
+    cfg.gridDim = dim3((unsigned)a.nsplit);
     cfg.blockDim = dim3(NTHREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c->stream;
@@ -706,19 +716,13 @@ int run_wgrad(dnsb_cnn *c, Volume &V, int L) {
   }
   prof_end(c, p);
   CC(c, cudaGetLastError());
-  const int N = 8 * CO;
-  const int nout = 27 * COUT[L] * CIN[L] + COUT[L];
-  Prof p2;
-  prof_begin(c, p2, 3, 0);
-  k_wgrad_reduce<<<(nout + 255) / 256, 256, 0, c->stream>>>(
-      c->partial[L], a.ngroups, a.nsplit, N, G, 8 * CI, CIN[L], COUT[L], a.ones_slot,
-      c->grads + LAYOUT.w[L], c->grads + LAYOUT.b[L]);
-  prof_end(c, p2);
-  CC(c, cudaGetLastError());
+  c->parts.part[L] = c->partial[L];
+  c->parts.nsplit[L] = a.nsplit;
   return 0;
 }
 
-// forward with the loss, backward, gradients reduced (training volume)
+// forward with the loss, backward, weight gradients as split-K partials
+// (training volume)
 int fwd_bwd(dnsb_cnn *c) {
   Volume &V = c->tr;
   int rc;
@@ -738,12 +742,13 @@ int fwd_bwd(dnsb_cnn *c) {
   return 0;
 }
 
-int adam_pack(dnsb_cnn *c, bool adam, float lr) {
+// gradients from the partials (reduce), Adam (adam), BF16 weights
+int update(dnsb_cnn *c, bool reduce, bool adam, float lr) {
   const KernelLayout kl = kernel_layout();
   Prof p;
   prof_begin(c, p, 3, 0);
-  k_adam_pack<<<(unsigned)((kl.total + 255) / 256), 256, 0, c->stream>>>(
-      kl, c->params, c->grads, c->m, c->v, adam ? 1 : 0, lr, c->step, c->packs);
+  k_update<<<(unsigned)((kl.total + UP_PARAMS - 1) / UP_PARAMS), UP_PARTS * UP_PARAMS, 0, c->stream>>>(
+      kl, c->parts, reduce ? 1 : 0, c->params, c->grads, c->m, c->v, adam ? 1 : 0, lr, c->step, c->packs);
   prof_end(c, p);
   CC(c, cudaGetLastError());
   return 0;
@@ -825,9 +830,7 @@ int dnsb_cnn_create(int device, void *stream, int batch, int crop, int nfield, d
     if ((rc = alloc_volume(c, c->tr, crop, batch, true))) return bail(rc);
     c->have_tr = true;
     for (int L = 0; L < NL; L++) {
-      const int G = 16 / CICH[L];
-      const int ngroups = (NTAPS + G - 1) / G;
-      c->partial_n[L] = (long)c->nsm * 2 * 128 * 8 * COCH[L] + (long)ngroups * 128 * 32;
+      c->partial_n[L] = (long)c->nsm * 3 * 128 * 3 * 8 * COCH[L];
       if ((rc = dal(c, &c->partial[L], c->partial_n[L]))) return bail(rc);
     }
   }
@@ -888,7 +891,7 @@ int dnsb_cnn_set_params(dnsb_cnn *c, const float *params) {
   CC(c, cudaMemsetAsync(c->v, 0, LAYOUT.total * sizeof(float), c->stream));
   CC(c, cudaMemsetAsync(c->step, 0, sizeof(long long), c->stream));
   c->h_steps = 0;
-  if ((rc = adam_pack(c, false, 0.f))) return rc;
+  if ((rc = update(c, false, false, 0.f))) return rc;
   CC(c, cudaStreamSynchronize(c->stream));
   return 0;
 }
@@ -945,16 +948,14 @@ int dnsb_cnn_train(dnsb_cnn *c, int nsteps, float lr, unsigned long long seed) {
   int rc;
   if ((rc = ensure_dev(c))) return rc;
   Volume &V = c->tr;
-  const long P3 = (long)V.P * V.P * V.P, c3 = (long)V.side * V.side * V.side;
-  const long work = (long)V.B * (P3 + c3);
   for (int s = 0; s < nsteps; s++) {
     Prof p;
     prof_begin(c, p, 3, 0);
-    k_crops<<<(unsigned)((work + 255) / 256), 256, 0, c->stream>>>(
-        c->data, c->nsnap, c->ndata, V.B, V.side, V.P, seed, c->step, V.in[0], V.tgt);
+    k_crops<<<dim3(V.P, V.B, 2), 256, 0, c->stream>>>(c->data, c->nsnap, c->ndata, V.side, V.P, seed,
+                                                      c->step, V.in[0], V.tgt);
     prof_end(c, p);
     CC(c, cudaGetLastError());
-    if ((rc = fwd_bwd(c)) || (rc = adam_pack(c, true, lr)) || (rc = tail(c, true))) return rc;
+    if ((rc = fwd_bwd(c)) || (rc = update(c, true, true, lr)) || (rc = tail(c, true))) return rc;
     c->h_steps++;
   }
   return 0;
@@ -1004,7 +1005,7 @@ int dnsb_cnn_batch(dnsb_cnn *c, const float *x, const float *t, int nadam, float
   prof_end(c, p);
   CC(c, cudaGetLastError());
   for (int i = 0; i < std::max(1, nadam); i++) {
-    if ((rc = fwd_bwd(c))) return rc;
+    if ((rc = fwd_bwd(c)) || (rc = update(c, true, false, 0.f))) return rc;
     if (i == 0) {
       if ((rc = tail(c, false))) return rc;
       if (grads_out)
@@ -1017,7 +1018,7 @@ int dnsb_cnn_batch(dnsb_cnn *c, const float *x, const float *t, int nadam, float
       }
     }
     if (nadam > 0) {
-      if ((rc = adam_pack(c, true, lr)) || (rc = tail(c, true))) return rc;
+      if ((rc = update(c, false, true, lr)) || (rc = tail(c, true))) return rc;
       c->h_steps++;
     }
   }
@@ -1037,8 +1038,8 @@ static int infer_common(dnsb_cnn *c, const double *v, const double *ux, const do
   prof_begin(c, p, 3, 0);
   {
     const unsigned bx = std::min(256u, (unsigned)(V.P + 31) / 32 * 32);
-    k_infer_in<<<dim3((V.P + bx - 1) / bx, V.P, V.P), bx, 0, c->stream>>>(v, ux, uy, uz, V.side, V.P, c->scales,
-                                                                         V.in[0]);
+    CC(c, dnsb::launch_as(c->pdl, k_infer_in, dim3((V.P + bx - 1) / bx, V.P, V.P), dim3(bx), 0, c->stream, v, ux,
+                          uy, uz, V.side, V.P, c->scales, V.in[0], c->pdl ? 1 : 0));
   }
   prof_end(c, p);
   CC(c, cudaGetLastError());

@@ -35,14 +35,19 @@
 // B (the weights) is resident in shared memory for the whole persistent
 // CTA, packed in the K-major core-matrix order.
 //
-// Weight gradient (k_wgrad): D[(tap slot j, ci)][co] = sum_o h[o + t_j][ci]
-// g[o][co] over the output positions o (the GEMM's K).  Both operands are
+// Weight gradient (k_wgrad): dW[dz, dy, dx][ci][co] = sum_o h[o + (dz, dy,
+// dx)][ci] g[o][co] over the output positions o (the GEMM's K).  With o' = o
+// + (0, dy, 0) the taps split over both operands: the GEMM's rows are (dx,
+// ci) of h shifted by dx, its columns (dy, co) of g shifted by -dy, and one
+// accumulator per dz takes h's plane z + dz against g's plane z.  Both are
 // MN-major canonical layouts without swizzle, straight from the chunked
-// activations: a K-block of R whole rows of one plane (R P positions) is one
-// TMA box [chunk][R rows][x] per tap, the tap's x shift running past the row
-// end into zeros where g is zero anyway; 128 / (8 CI) taps fill the 128 rows (the slot
-// after the last real tap holds ones, which makes that row the bias
-// gradient).  Split-K partials are reduced in a fixed order.
+// activations: a K-block of R whole rows of one plane (R P positions, padded
+// to a multiple of 16) is one TMA box [chunk][R rows][x] per shift; an x
+// shift runs past the row end into zeros where g is zero anyway, a y shift
+// starts above or below the volume in zeros.  A CTA marches up z, so that
+// each plane of h is copied once for its three dz.  The row slot after the
+// three dx holds ones, which makes that row of dz = 0 the bias gradient.
+// Split-K partials are reduced in a fixed order.
 //
 // Warp roles: warp 0 issues the TMA copies, warp 1 owns the tensor memory
 // and issues the MMAs (one thread), the other warps run the epilogue (warp
@@ -70,7 +75,6 @@ constexpr int TILE_M = 128;      // GEMM rows (positions) of a convolution tile
 constexpr int TILE_OUT = 126;    // outputs of a convolution tile (rows m, m + 1, m + 2 feed output m)
 constexpr int CONV_BARS = 512;   // bytes of barriers and flags after the plane ring
 constexpr int CONV_XBUF = CONV_GROUPS * 2 * 3 * 2 * 32 * 4;  // lane-quarter boundary exchange, bytes
-constexpr int WG_STAGES = 4;
 constexpr int CV_STAGES = 2;
 enum { DEVERR_CNN_TIMEOUT = 2 };
 
@@ -738,66 +742,80 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
 
 // ------------------------------------------------------ weight gradient --
 
+constexpr int WG_PLANES = 4;  // planes of h in shared memory: three in use, one ahead
+constexpr int WG_GRADS = 2;   // planes of g
+
 struct WgradArgs {
-  int P, Pz, B;     // volume geometry
+  int P, B;         // volume geometry
   int Do;           // output box side (of g)
-  int R, KB;        // rows per K-block and its positions R * P (a multiple of 16)
-  int stages;       // K-blocks in flight (<= WG_STAGES)
-  int kpp;          // K-blocks per plane: ceil(Do / R)
-  int nk;           // B * Do * kpp
-  int ngroups;      // ceil(27 / G) tap groups
-  int nsplit;       // K splits (grid = ngroups * nsplit)
-  int ones_slot;    // slot of the last group holding ones (bias row)
-  uint32_t a_bytes, stage_bytes;
+  int R, KB, KBp;   // rows per K-block, its positions R P, padded to a multiple of 16
+  int whole;        // one TMA box per shift holds all chunks (KB == KBp), else one per chunk
+  int kpp;          // K-blocks per plane: ceil((Do + 2) / R)
+  int nsplit;       // K splits = CTAs
+  uint32_t h_bytes, g_bytes;  // one plane of h (four row slots) and of g (three shifts)
   unsigned wait_limit;
-  float *partial;   // [split][group][128][N]
+  float *partial;   // [split][dz][128][N]
   int *err;
 };
 
-// h: CI chunks (A operand, tap-shifted), g: CO chunks (B operand).
+// h: CI chunks (A operand, shifted in x), g: CO chunks (B operand, shifted in
+// y).  Bound by the L2-to-SM copies and the MMAs about alike: per step (one
+// plane of one row block) six boxes of 64-byte positions and 3 KBp / 16 MMAs of
+// N = 96 (56 cycles each) for 27 taps.  With the taps stacked four at a time
+// on the rows (N = 32) every position was copied 34 times and took 7 MMAs of 52
+// cycles per 16 positions: 85.6 us for a 32 x 32-channel layer of 8 crops of
+// 32^3 (959 MB of copies, 11.7 TB/s).
 template <int CI, int CO>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_wgrad(const __grid_constant__ CUtensorMap th, const __grid_constant__ CUtensorMap tg,
             const WgradArgs a) {
-  constexpr int N = 8 * CO;
-  constexpr int G = 16 / CI;             // tap slots per group (M = 128 rows)
-  constexpr uint32_t NCOLS = N < 32 ? 32 : N;
-  const uint32_t SLOT = (uint32_t)CI * a.KB * 16;  // bytes of one tap slot
+  constexpr int N = 3 * 8 * CO;
+  constexpr uint32_t ACC = 128, NCOLS = 512;  // columns between the dz accumulators, allocated
+  const uint32_t chunk = (uint32_t)a.KBp * 16;  // bytes of one chunk of a K-block
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *smem = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + a.stages * a.stage_bytes);
-  uint64_t *full = bars, *empty = bars + WG_STAGES, *done = bars + 2 * WG_STAGES;
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 2 * WG_STAGES + 1);
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * WG_STAGES + 2);
+  unsigned char *gs = smem + WG_PLANES * a.h_bytes;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(gs + WG_GRADS * a.g_bytes);
+  uint64_t *hfull = bars, *hempty = hfull + WG_PLANES, *gfull = hempty + WG_PLANES,
+           *gempty = gfull + WG_GRADS, *done = gempty + WG_GRADS;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(done + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = blockIdx.x % a.ngroups, split = blockIdx.x / a.ngroups;
-  const int tap0 = grp * G;
-  const int ntap = min(G, NTAPS - tap0);
-  const bool ones = grp == a.ngroups - 1 && a.ones_slot < G;
-  const int k0 = (int)((long long)a.nk * split / a.nsplit);
-  const int k1 = (int)((long long)a.nk * (split + 1) / a.nsplit);
+  const int split = blockIdx.x;
+  // steps (sample, row block, z), z fastest
+  const long long nsteps = (long long)a.B * a.kpp * a.Do;
+  const int s0 = (int)(nsteps * split / a.nsplit), s1 = (int)(nsteps * (split + 1) / a.nsplit);
   // programmatic dependent launch: dependents may launch once every block
   // of this grid has started; they wait for its completion before memory
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < a.stages; i++) {
-      mb_init(&full[i], 1);
-      mb_init(&empty[i], 1);
+    for (int i = 0; i < WG_PLANES; i++) {
+      mb_init(&hfull[i], 1);
+      mb_init(&hempty[i], 1);
+    }
+    for (int i = 0; i < WG_GRADS; i++) {
+      mb_init(&gfull[i], 1);
+      mb_init(&gempty[i], 1);
     }
     mb_init(done, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (ones) {
-    // the slot after the last tap: BF16 ones, in every stage, never copied over
-    const uint32_t one2 = 0x3F803F80u;
-    for (int st = 0; st < a.stages; st++) {
-      uint32_t *p = reinterpret_cast<uint32_t *>(smem + st * a.stage_bytes + a.ones_slot * SLOT);
-      for (int i = threadIdx.x; i < (int)(SLOT / 4); i += NTHREADS) p[i] = one2;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  if (!a.whole) {
+    // the padding positions of every chunk stay zero
+    uint4 *z = reinterpret_cast<uint4 *>(smem);
+    const int n = (int)((WG_PLANES * a.h_bytes + WG_GRADS * a.g_bytes) / 16);
+    for (int i = threadIdx.x; i < n; i += NTHREADS) z[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
   }
+  // the row slot after the three dx: BF16 ones in every plane slot, never copied over
+  for (int st = 0; st < WG_PLANES; st++) {
+    uint4 *p = reinterpret_cast<uint4 *>(smem + st * a.h_bytes + 3 * CI * chunk);
+    const uint32_t one2 = 0x3F803F80u;
+    for (int i = threadIdx.x; i < (int)(CI * chunk / 16); i += NTHREADS) p[i] = make_uint4(one2, one2, one2, one2);
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (warp == 1) tmem_alloc(tslot, NCOLS);
   // the previous kernel's outputs (activations, gradients) complete and
   // visible past this (a no-op for an ordinary launch)
@@ -809,64 +827,87 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      const uint32_t bytes = (uint32_t)ntap * SLOT + (uint32_t)CO * a.KB * 16;
-      int i = 0, issued = 0;
-      for (int k = k0; k < k1; k++, i++) {
-        const int s = i % a.stages, ph = (i / a.stages) & 1;
-        if (*abort_flag || !mb_wait(&empty[s], ph ^ 1, a.wait_limit, abort_flag)) {
-          *abort_flag = 1;
-          atomicExch(a.err, DEVERR_CNN_TIMEOUT);
-          break;
+      const uint32_t hb = 3u * CI * a.KB * 16, gb = 3u * CO * a.KB * 16;
+      int pl = 0, gi = 0;  // planes of h and of g issued
+      bool ok = true;
+      for (int s = s0; ok && s < s1; s++) {
+        const int col = s / a.Do, z = s - col * a.Do;
+        const int b = col / a.kpp, y0 = (col - b * a.kpp) * a.R;
+        // the first step of a column loads three planes, the others one
+        for (int pz = s == s0 || z == 0 ? z : z + 2; ok && pz <= z + 2; pz++) {
+          const int sl = pl % WG_PLANES;
+          ok = !*abort_flag && mb_wait(&hempty[sl], ((pl / WG_PLANES) & 1) ^ 1, a.wait_limit, abort_flag);
+          if (!ok) break;
+          mb_expect(&hfull[sl], hb);
+          unsigned char *d = smem + sl * a.h_bytes;
+          for (int dx = 0; dx < 3; dx++)
+            for (int c = 0; c < (a.whole ? 1 : CI); c++)
+              tma4(d + (dx * CI + c) * chunk, &th, 2 * dx, y0, pz, b * CI + c, &hfull[sl]);
+          pl++;
         }
-        const int jb = k % a.kpp, rest = k / a.kpp;
-        const int z = rest % a.Do, b = rest / a.Do;
-        const int y0 = jb * a.R;
-        unsigned char *st = smem + s * a.stage_bytes;
-        mb_expect(&full[s], bytes);
-        // R whole rows per box; a tap's x shift runs past the row end into
-        // zeros, where g (zero outside its output box) takes nothing
-        for (int j = 0; j < ntap; j++) {
-          const int tap = tap0 + j;
-          const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-          tma4(st + j * SLOT, &th, 2 * dx, y0 + dy, z + dz, b * CI, &full[s]);
+        if (ok) {
+          const int st = gi % WG_GRADS;
+          ok = !*abort_flag && mb_wait(&gempty[st], ((gi / WG_GRADS) & 1) ^ 1, a.wait_limit, abort_flag);
+          if (!ok) break;
+          mb_expect(&gfull[st], gb);
+          unsigned char *d = gs + st * a.g_bytes;
+          for (int dy = 0; dy < 3; dy++)
+            for (int c = 0; c < (a.whole ? 1 : CO); c++)
+              tma4(d + (dy * CO + c) * chunk, &tg, 0, y0 - dy, z, b * CO + c, &gfull[st]);
+          gi++;
         }
-        tma4(st + a.a_bytes, &tg, 0, y0, z, b * CO, &full[s]);
-        issued = i + 1;
-      }
-      // let the last copies of every stage land before leaving
-      for (int i2 = issued - a.stages < 0 ? 0 : issued - a.stages; i2 < issued; i2++)
-        mb_wait(&full[i2 % a.stages], (i2 / a.stages) & 1, a.wait_limit, abort_flag);
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_bf16(N, true, true);
-      int i = 0;
-      bool ok = true, any = false;
-      for (int k = k0; k < k1; k++, i++) {
-        const int s = i % a.stages, ph = (i / a.stages) & 1;
-        if (*abort_flag || !mb_wait(&full[s], ph, a.wait_limit, abort_flag)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t sa = saddr(smem + s * a.stage_bytes);
-        const uint32_t sb = sa + a.a_bytes;
-        const int nkk = a.KB / 16;
-        for (int kk = 0; kk < nkk; kk++) {
-          // MN-major, no swizzle: SBO = stride of 8-element MN groups (one
-          // chunk's K-block, 16 KB bytes), LBO = stride of 8-row K groups (128 B)
-          const uint64_t ad = sdesc(sa + kk * 256, 128, (uint32_t)a.KB * 16);
-          const uint64_t bd = sdesc(sb + kk * 256, 128, (uint32_t)a.KB * 16);
-          mma_bf16(tbase, ad, bd, idesc, (i | kk) != 0);
-        }
-        mma_commit(&empty[s]);
-        any = true;
       }
       if (!ok) {
         *abort_flag = 1;
         atomicExch(a.err, DEVERR_CNN_TIMEOUT);
       }
-      if (any) mma_commit(done);
+      // let the last copies of every slot land before leaving
+      for (int i = pl < WG_PLANES ? 0 : pl - WG_PLANES; i < pl; i++)
+        mb_wait(&hfull[i % WG_PLANES], (i / WG_PLANES) & 1, a.wait_limit, abort_flag);
+      for (int i = gi < WG_GRADS ? 0 : gi - WG_GRADS; i < gi; i++)
+        mb_wait(&gfull[i % WG_GRADS], (i / WG_GRADS) & 1, a.wait_limit, abort_flag);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = idesc_bf16(N, true, true);
+      const int nkk = a.KBp / 16;
+      int pc = 0, have = 0, gi = 0;  // plane of dz = 0, planes waited for, planes of g
+      bool ok = true;
+      for (int s = s0; s < s1; s++) {
+        const bool last = s + 1 == s1 || (s + 1) % a.Do == 0;  // of its column here
+        for (; ok && have < pc + 3; have++)
+          ok = !*abort_flag &&
+               mb_wait(&hfull[have % WG_PLANES], (have / WG_PLANES) & 1, a.wait_limit, abort_flag);
+        const int st = gi % WG_GRADS;
+        ok = ok && !*abort_flag && mb_wait(&gfull[st], (gi / WG_GRADS) & 1, a.wait_limit, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        // MN-major, no swizzle: SBO = stride of 8-element MN groups (one
+        // chunk), LBO = stride of 8-row K groups (128 B)
+        const uint64_t bd = sdesc(saddr(gs + st * a.g_bytes), 128, chunk);
+        uint64_t ad[3];
+#pragma unroll
+        for (int dz = 0; dz < 3; dz++)
+          ad[dz] = sdesc(saddr(smem + (pc + dz) % WG_PLANES * a.h_bytes), 128, chunk);
+        for (int kk = 0; kk < nkk; kk++) {
+#pragma unroll
+          for (int dz = 0; dz < 3; dz++)  // 16 positions: 256 bytes on, 16 in the address field
+            mma_bf16(tbase + dz * ACC, ad[dz] + 16 * kk, bd + 16 * kk, idesc, (gi | kk) != 0);
+        }
+        mma_commit(&gempty[st]);
+        mma_commit(&hempty[pc % WG_PLANES]);
+        if (last) {
+          mma_commit(&hempty[(pc + 1) % WG_PLANES]);
+          mma_commit(&hempty[(pc + 2) % WG_PLANES]);
+        }
+        pc += last ? 3 : 1;
+        gi++;
+      }
+      if (!ok) {
+        *abort_flag = 1;
+        atomicExch(a.err, DEVERR_CNN_TIMEOUT);
+      }
+      if (gi > 0) mma_commit(done);
       else mb_arrive(done);
     }
   } else {
@@ -878,15 +919,21 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       atomicExch(a.err, DEVERR_CNN_TIMEOUT);
     }
     tc_fence_after();
-    float v[N];
-    tmem_ld<N>(tbase + ((uint32_t)(q * 32) << 16), v);
-    float *dst = a.partial + (((long long)split * a.ngroups + grp) * 128 + m) * N;
-    const bool empty_range = k1 <= k0;
+    const bool none = s1 <= s0 || !ok;
+    constexpr int W = N % 32 == 0 ? 32 : 16;
+    for (int dz = 0; dz < 3; dz++) {
+      float *dst = a.partial + (((long long)split * 3 + dz) * 128 + m) * N;
+#pragma unroll 1
+      for (int c0 = 0; c0 < N; c0 += W) {
+        float v[W];
+        tmem_ld<W>(tbase + ((uint32_t)(q * 32) << 16) + dz * ACC + c0, v);
+        if (m > 3 * 8 * CI) continue;  // rows beyond the ones: nothing reads them
 #pragma unroll
-    for (int c = 0; c < N; c += 4)
-      *reinterpret_cast<float4 *>(dst + c) =
-          empty_range || !ok ? make_float4(0.f, 0.f, 0.f, 0.f)
-                             : make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        for (int c = 0; c < W; c += 4)
+          *reinterpret_cast<float4 *>(dst + c0 + c) =
+              none ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+      }
+    }
   }
   tc_fence_before();
   __syncthreads();

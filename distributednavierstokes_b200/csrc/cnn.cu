@@ -121,66 +121,94 @@ struct Partials {
 
 // With `reduce` every parameter's gradient from the split-K partials of its
 // layer, with `adam` the Adam update, and the BF16 packing of every weight.
-// Threads run over (tap, ci, co) with co fastest, the partials' order; eight
-// threads share a parameter's splits (each adds every eighth, the eight sums
-// are added in order).  One launch at the step's end: as four reductions
-// between the backward kernels (5.2 us each, ordinary launches that kept the
-// next convolution from starting early) and an Adam launch (5.9 us, two double
-// pow per thread) they were 27 us of a 545 us training step.
-constexpr int UP_PARTS = 8, UP_PARAMS = 32;
-__global__ void __launch_bounds__(UP_PARTS *UP_PARAMS)
-    k_update(KernelLayout k, Partials pt, int reduce, float *params, float *grads, float *m, float *v, int adam,
-             float lr, const long long *step, Packs packs) {
+// Work is numbered over quads of the partials' columns (dy, co), so that a
+// thread reads 16 bytes of each split; 16 threads share a quad's splits (each
+// adds every 16th, the sums are added in order), all loads in flight at once.
+// One launch at the step's end: as four reductions between the backward kernels
+// (5.2 us each, ordinary launches that kept the next convolution from starting
+// early) and an Adam launch (5.9 us, two double pow per thread) they were 27 us
+// of a 545 us training step.  26 us: the splits' sums are read once (49 MB).
+constexpr int UP_PARTS = 16, UP_QUADS = 16;
+__host__ __device__ inline int up_quads(int L, int cin) {  // of layer L: weights, then biases
+  const int coch = L == 3 ? 2 : 4;
+  return 3 * 3 * cin * (3 * 2 * coch) + 2 * coch;
+}
+__global__ void __launch_bounds__(UP_PARTS *UP_QUADS)
+    k_update(const __grid_constant__ KernelLayout k, const __grid_constant__ Partials pt, int reduce, float *params,
+             float *grads, float *m, float *v, int adam, float lr, const long long *step,
+             const __grid_constant__ Packs packs) {
   __shared__ float corr[2];
-  __shared__ float sums[UP_PARTS][UP_PARAMS];
-  const int lp = threadIdx.x % UP_PARAMS, part = threadIdx.x / UP_PARAMS;
-  if (adam && threadIdx.x < 2) {  // 1 - beta^(step + 1), by squaring
-    double b = threadIdx.x ? (double)0.999f : (double)0.9f, q = 1.0;
+  __shared__ float4 sums[UP_PARTS][UP_QUADS];
+  const int tid = threadIdx.x;
+  if (adam && tid < 2) {  // 1 - beta^(step + 1), by squaring
+    double b = tid ? (double)0.999f : (double)0.9f, q = 1.0;
     for (unsigned long long n = (unsigned long long)*step + 1; n; n >>= 1, b *= b)
       if (n & 1) q *= b;
-    corr[threadIdx.x] = (float)(1.0 - q);
+    corr[tid] = (float)(1.0 - q);
   }
-  long i = (long)blockIdx.x * UP_PARAMS + lp;
-  const bool in = i < k.total;
-  int L = 0, t = 0, ci = 0, co = 0;
-  bool bias = false;
-  long p = 0;
-  if (in) {
-    while (L < NL - 1 && i >= k.w[L + 1]) L++;
-    i -= k.w[L];
-    const int cin = k.cin[L], cout = k.cout[L], nw = 27 * cin * cout;
-    bias = i >= nw;
-    if (bias) {
-      co = (int)(i - nw);
-    } else {
-      const int r = (int)i / cout;
-      co = (int)i - r * cout;
-      t = r / cin;
-      ci = r - t * cin;
+  // quad -> layer, tap, ci, first co and its place in a split's partials
+  struct Quad {
+    int L, t, ci, co;  // t < 0: bias; L = NL: none
+    long at;
+  };
+  auto locate = [&](int lq) {
+    Quad q{NL, -1, 0, 0, 0};
+    int r = blockIdx.x * UP_QUADS + lq;
+    for (int L = 0; L < NL; L++) {
+      const int n = up_quads(L, k.cin[L]);
+      if (r >= n) {
+        r -= n;
+        continue;
+      }
+      const int cich = L == 0 ? 2 : 4, coch = L == 3 ? 2 : 4, cin = k.cin[L], N = 24 * coch, N4 = N / 4;
+      q.L = L;
+      if (r >= 9 * cin * N4) {
+        q.co = 4 * (r - 9 * cin * N4);
+        q.at = 24L * cich * N + q.co;
+      } else {
+        const int n4 = r % N4, row = r / N4, dz = row / (3 * cin), dx = row / cin % 3;
+        q.ci = row % cin;
+        q.co = 4 * n4 % (8 * coch);
+        q.t = (dz * 3 + 4 * n4 / (8 * coch)) * 3 + dx;
+        q.at = (128L * dz + 8 * cich * dx + q.ci) * N + 4 * n4;
+      }
+      break;
     }
-    p = bias ? k.b[L] + co : k.w[L] + ((long)t * cout + co) * cin + ci;
-  }
+    return q;
+  };
   if (reduce) {
-    float g = 0.f;
-    if (in) {
-      const int cich = L == 0 ? 2 : 4, N = 3 * 8 * (L == 3 ? 2 : 4);
-      const int dz = bias ? 0 : t / 9, row = bias ? 3 * 8 * cich : (t % 3) * 8 * cich + ci;
-      const int n = bias ? co : (t / 3) % 3 * (N / 3) + co;
-      const float *q = pt.part[L] + ((long)dz * 128 + row) * N + n;
-      const long stride = 3L * 128 * N;
-      const int ns = pt.nsplit[L];
-#pragma unroll 8
-      for (int sp = part; sp < ns; sp += UP_PARTS) g += q[sp * stride];
+    const int lq = tid % UP_QUADS, part = tid / UP_QUADS;
+    const Quad q = locate(lq);
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (q.L < NL) {
+      const long stride = 3L * 128 * (24 * (q.L == 3 ? 2 : 4));
+      const int ns = pt.nsplit[q.L];
+      const float *src = pt.part[q.L] + q.at;
+#pragma unroll 10
+      for (int sp = part; sp < ns; sp += UP_PARTS) {
+        const float4 x = *reinterpret_cast<const float4 *>(src + sp * stride);
+        g.x += x.x;
+        g.y += x.y;
+        g.z += x.z;
+        g.w += x.w;
+      }
     }
-    sums[part][lp] = g;
+    sums[part][lq] = g;
   }
   __syncthreads();
-  if (part || !in) return;
+  // one thread per parameter
+  if (tid >= 4 * UP_QUADS) return;
+  const Quad q = locate(tid / 4);
+  if (q.L == NL) return;
+  const int L = q.L, co = q.co + tid % 4;
+  if (co >= k.cout[L]) return;
+  const bool bias = q.t < 0;
+  const long p = bias ? k.b[L] + co : k.w[L] + ((long)q.t * k.cout[L] + co) * k.cin[L] + q.ci;
   float w = params[p], g;
   if (reduce) {
     g = 0.f;
 #pragma unroll
-    for (int q = 0; q < UP_PARTS; q++) g += sums[q][lp];
+    for (int i = 0; i < UP_PARTS; i++) g += reinterpret_cast<const float *>(&sums[i][tid / 4])[tid % 4];
     grads[p] = g;
   } else {
     g = grads[p];
@@ -196,8 +224,8 @@ __global__ void __launch_bounds__(UP_PARTS *UP_PARAMS)
   }
   if (bias) return;
   const __nv_bfloat16 wb = __float2bfloat16_rn(w);
-  packs.f[L][pack_fwd(L, t, co, ci)] = wb;
-  if (L > 0) packs.d[L][pack_bwd(L, t, co, ci)] = wb;
+  packs.f[L][pack_fwd(L, q.t, co, q.ci)] = wb;
+  if (L > 0) packs.d[L][pack_bwd(L, q.t, co, q.ci)] = wb;
 }
 
 __device__ inline unsigned long long splitmix(unsigned long long x) {
@@ -208,8 +236,7 @@ __device__ inline unsigned long long splitmix(unsigned long long x) {
 }
 
 __device__ inline uint4 chunk3(float a, float b, float c) {
-  const float v[8] = {a, b, c, 0.f, 0.f, 0.f, 0.f, 0.f};
-  return pack8(v);
+  return make_uint4(pack2(make_float2(a, b)), pack2(make_float2(c, 0.f)), 0u, 0u);
 }
 
 // random crops of the dataset: input with its halo (chunk 0 of x0) and the
@@ -281,8 +308,8 @@ __global__ void k_batch_in(const float *x, const float *t, int B, int crop, int 
 // block (no division per voxel); the halo (HALO < n) wraps by one correction
 __global__ void k_infer_in(const double *v, const double *ux, const double *uy, const double *uz,
                            int n, int P, const float *in_scale, uint4 *x0, int dep) {
-  dnsb::pdl_trigger(dep);
   dnsb::pdl_wait(dep);
+  dnsb::pdl_trigger(dep);  // past the wait: the convolution reads the weights before its own
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
   if (x >= P) return;
   const long i = ((long)z * P + y) * P + x;
@@ -472,7 +499,7 @@ int make_map_patch(dnsb_cnn *c, CUtensorMap *m, void *base, int P, int chunks, i
   return 0;
 }
 
-constexpr int RING_MAX = 12, RING_MIN = 4;
+constexpr int RING_MAX = 12, RING_GOOD = 6, RING_MIN = 4;
 constexpr size_t CONV_EXTRA = CONV_BARS + CONV_XBUF + 1024;  // barriers, exchange, alignment slack
 
 // shared memory of a convolution with the largest plane ring that fits
@@ -537,16 +564,20 @@ int alloc_volume(dnsb_cnn *c, Volume &V, int side, int B, bool training) {
     if ((rc = dal(c, &V.tgt, (size_t)B * P3 * 2))) return rc;
   }
   // up to four 126-output sub-tiles per plane load (fewer copies per
-  // output): the most whose wider patch fits the plane and a ring of at
-  // least RING_MIN planes
+  // output): the most whose wider patch fits the plane and a ring of
+  // RING_GOOD planes, else of at least RING_MIN.  Three planes are in use; with
+  // one ahead (3 sub-tiles, 4 slots at side 64) the next plane's copy is not
+  // done in time: 85.7 us an inference of 64^3, 81.6 with 6 slots and 1 or 2
+  // sub-tiles (training on 8 crops of 32^3 about the same, 358 and 360 us)
   {
     auto most = [&](int s, int e) {
-      for (int sub = 4; sub > 1; sub--) {
-        int ns;
-        uint32_t sl, st, wb;
-        const int r = patch_rows(P, s, e, sub);
-        if (r <= P && conv_smem(4, 4, P, r, &ns, &sl, &st, &wb)) return sub;
-      }
+      for (int want : {RING_GOOD, RING_MIN})
+        for (int sub = 4; sub > (want == RING_GOOD ? 0 : 1); sub--) {
+          int ns;
+          uint32_t sl, st, wb;
+          const int r = patch_rows(P, s, e, sub);
+          if (r <= P && conv_smem(4, 4, P, r, &ns, &sl, &st, &wb) && ns >= want) return sub;
+        }
       return 1;
     };
     V.subf = most(0, 0);
@@ -631,8 +662,9 @@ int run_conv(dnsb_cnn *c, Volume &V, int L, const CUtensorMap &map, bool transpo
   // output box of a forward layer L: P - 2 (L+1); of the transposed one: the
   // box of layer L's input (layer L-1's output)
   a.Do = transposed ? V.P - 2 * L : V.P - 2 * (L + 1);
-  a.tpp = (a.Do * a.P + a.sub * TILE_OUT - 1) / (a.sub * TILE_OUT);
-  a.ntiles = V.B * a.Do * a.tpp;
+  a.spp = (a.Do * a.P + TILE_OUT - 1) / TILE_OUT;
+  a.tpp = (a.spp + a.sub - 1) / a.sub;
+  a.nsub = V.B * a.Do * a.spp;
   const size_t smem = conv_smem(CI, CO, a.P, a.R, &a.nslot, &a.slot_bytes, &a.slot_stride, &a.w_bytes);
   if (!smem) return cfail(c, DNSB_EUNSUP, "convolution plane ring does not fit in shared memory");
   a.wait_limit = WAIT_LIMIT;
@@ -649,7 +681,7 @@ int run_conv(dnsb_cnn *c, Volume &V, int L, const CUtensorMap &map, bool transpo
   a.err = c->deverr;
   int rc = setup_conv_attr<CI, CO, MODE>(c, smem);
   if (rc) return rc;
-  const int grid = grid_for(c, (const void *)k_conv<CI, CO, MODE>, smem, a.ntiles, CONV_THREADS);
+  const int grid = grid_for(c, (const void *)k_conv<CI, CO, MODE>, smem, a.nsub, CONV_THREADS);
   if (MODE == FWD_LOSS) {
     if (grid > c->loss_nparts) return cfail(c, DNSB_EUNSUP, "loss partials: grid %d > %d", grid, c->loss_nparts);
     c->loss_nparts_used = grid;
@@ -747,7 +779,9 @@ int update(dnsb_cnn *c, bool reduce, bool adam, float lr) {
   const KernelLayout kl = kernel_layout();
   Prof p;
   prof_begin(c, p, 3, 0);
-  k_update<<<(unsigned)((kl.total + UP_PARAMS - 1) / UP_PARAMS), UP_PARTS * UP_PARAMS, 0, c->stream>>>(
+  int quads = 0;
+  for (int L = 0; L < NL; L++) quads += up_quads(L, CIN[L]);
+  k_update<<<(quads + UP_QUADS - 1) / UP_QUADS, UP_PARTS * UP_QUADS, 0, c->stream>>>(
       kl, c->parts, reduce ? 1 : 0, c->params, c->grads, c->m, c->v, adam ? 1 : 0, lr, c->step, c->packs);
   prof_end(c, p);
   CC(c, cudaGetLastError());

@@ -49,11 +49,12 @@
 // three dx holds ones, which makes that row of dz = 0 the bias gradient.
 // Split-K partials are reduced in a fixed order.
 //
-// Warp roles: warp 0 issues the TMA copies, warp 1 owns the tensor memory
-// and issues the MMAs (one thread), the other warps run the epilogue (warp
-// w reads TMEM lanes 32 (w % 4) .. + 31): warps 2-5 of the weight gradient
-// (192 threads), two groups of four (warps 2-5, 6-9) taking alternate tiles
-// of the convolution (320 threads).  Every
+// Warp roles: warp 0 issues the TMA copies; warps 1 and 2 of the convolution,
+// 1 to 3 of the weight gradient issue the MMAs (the whole warp runs the loop,
+// one elected lane issues) and warp 1 owns the tensor memory; the other warps
+// run the epilogue (a warp reads TMEM lanes 32 (w % 4) .. + 31): four groups of
+// four taking the convolution's sub-tiles in turn (608 threads), warps 4-7 of
+// the weight gradient (256 threads).  Every
 // mbarrier wait is bounded; a wait that runs out raises the CTA's abort flag
 // and the global error word, every role leaves its loop, the copies and MMAs
 // in flight are waited for (bounded), the tensor memory is freed and the CTA
@@ -67,7 +68,7 @@
 namespace dnsb {
 namespace cnn {
 
-constexpr int NTHREADS = 192;       // weight gradient: TMA, MMA, 4 epilogue warps
+constexpr int NTHREADS = 256;       // weight gradient: TMA, three MMA, four epilogue warps
 constexpr int CONV_GROUPS = 4;      // convolution epilogue: groups of 4 warps taking tiles in turn
 constexpr int CONV_THREADS = 96 + 128 * CONV_GROUPS;  // TMA, two MMA, epilogue warps
 constexpr int NTAPS = 27;
@@ -75,7 +76,6 @@ constexpr int TILE_M = 128;      // GEMM rows (positions) of a convolution tile
 constexpr int TILE_OUT = 126;    // outputs of a convolution tile (rows m, m + 1, m + 2 feed output m)
 constexpr int CONV_BARS = 512;   // bytes of barriers and flags after the plane ring
 constexpr int CONV_XBUF = CONV_GROUPS * 2 * 3 * 2 * 32 * 4;  // lane-quarter boundary exchange, bytes
-constexpr int CV_STAGES = 2;
 enum { DEVERR_CNN_TIMEOUT = 2 };
 
 enum Mode { FWD_GELU = 0, FWD_LOSS = 1, FWD_INFER = 2, DGRAD = 3 };
@@ -94,15 +94,6 @@ __device__ __forceinline__ void mb_expect(uint64_t *b, uint32_t bytes) {
 }
 __device__ __forceinline__ void mb_arrive(uint64_t *b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
-}
-__device__ __forceinline__ bool mb_try(uint64_t *b, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(saddr(b)), "r"(parity)
-      : "memory");
-  return ok != 0;
 }
 // try_wait that may suspend the thread for up to `ns` nanoseconds while the
 // phase is incomplete (returns as soon as it completes)
@@ -139,6 +130,23 @@ __device__ __forceinline__ bool mb_wait(uint64_t *b, uint32_t parity, unsigned l
   }
   return false;
 }
+// The same by a whole warp, with one answer for all its lanes (so that the
+// loops around it stay uniform)
+__device__ __forceinline__ bool warp_wait(uint64_t *b, uint32_t parity, unsigned limit,
+                                          volatile int *abort_flag) {
+  if (__all_sync(0xffffffffu, mb_test(b, parity))) return true;
+  for (unsigned it = 0; it < limit; it++) {
+    if (__all_sync(0xffffffffu, mb_try_sleep(b, parity, 1000))) return true;
+    if ((it & 15) == 15 && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+  }
+  return false;
+}
+// one lane of a converged warp, the same every time
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(r));
+  return r != 0;
+}
 // named barrier over `n` threads that also ORs a predicate across them
 __device__ __forceinline__ bool bar_or(int id, int n, bool pred) {
   uint32_t r;
@@ -148,14 +156,6 @@ __device__ __forceinline__ bool bar_or(int id, int n, bool pred) {
       : "r"((uint32_t)pred), "r"(id), "r"(n)
       : "memory");
   return r != 0;
-}
-__device__ __forceinline__ void tma3(void *dst, const CUtensorMap *m, int c0, int c1, int c2,
-                                     uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-          saddr(dst)),
-      "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(saddr(bar))
-      : "memory");
 }
 __device__ __forceinline__ void tma4(void *dst, const CUtensorMap *m, int c0, int c1, int c2, int c3,
                                      uint64_t *bar) {
@@ -272,39 +272,59 @@ __device__ __forceinline__ float tanh_hw(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float gelu_f(float z) {
-  const float u = z * fmaf(GELU_C * GELU_A, z * z, GELU_C);
-  const float h = 0.5f * z;
-  return fmaf(h, tanh_hw(u), h);
+// Two FP32 values per instruction (fma / mul / add .rn.f32x2, each rounded as
+// the scalar operation): the convolutions' epilogue is bound by its
+// instructions.
+__device__ __forceinline__ unsigned long long bits2(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
 }
-// d/dz [0.5 z (1 + t)] = 0.5 (1 + t) + 0.5 z (1 - t^2) u'(z)
-__device__ __forceinline__ float gelu_grad_f(float z) {
-  const float z2 = z * z;
-  const float t = tanh_hw(z * fmaf(GELU_C * GELU_A, z2, GELU_C));
-  const float du = fmaf(3.f * GELU_C * GELU_A, z2, GELU_C);
-  return fmaf(0.5f * z * fmaf(-t, t, 1.f), du, fmaf(0.5f, t, 0.5f));
+__device__ __forceinline__ float2 float2_of(unsigned long long r) {
+  float2 a;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+  return a;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
+  return float2_of(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
+  return float2_of(d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)));
+  return float2_of(d);
+}
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 tanh2(float2 u) { return make_float2(tanh_hw(u.x), tanh_hw(u.y)); }
+__device__ __forceinline__ float2 gelu2(float2 z) {
+  const float2 u = mul2(z, fma2(both(GELU_C * GELU_A), mul2(z, z), both(GELU_C)));
+  const float2 h = mul2(both(0.5f), z);
+  return fma2(h, tanh2(u), h);
+}
+// d/dz [0.5 z (1 + t)] = s + s (1 - t) z u'(z) with s = 0.5 (1 + t)
+__device__ __forceinline__ float2 gelu_grad2(float2 z) {
+  const float2 z2 = mul2(z, z);
+  const float2 t = tanh2(mul2(z, fma2(both(GELU_C * GELU_A), z2, both(GELU_C))));
+  const float2 zdu = mul2(z, fma2(both(3.f * GELU_C * GELU_A), z2, both(GELU_C)));
+  const float2 s = fma2(both(0.5f), t, both(0.5f));
+  return fma2(mul2(s, fma2(both(-1.f), t, both(1.f))), zdu, s);
 }
 
-__device__ __forceinline__ uint4 pack8(const float *v) {
-  uint4 o;
-  __nv_bfloat162 t;
-  t = __floats2bfloat162_rn(v[0], v[1]);
-  o.x = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2bfloat162_rn(v[2], v[3]);
-  o.y = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2bfloat162_rn(v[4], v[5]);
-  o.z = *reinterpret_cast<uint32_t *>(&t);
-  t = __floats2bfloat162_rn(v[6], v[7]);
-  o.w = *reinterpret_cast<uint32_t *>(&t);
-  return o;
+__device__ __forceinline__ uint32_t pack2(float2 v) {
+  const __nv_bfloat162 t = __floats2bfloat162_rn(v.x, v.y);
+  return *reinterpret_cast<const uint32_t *>(&t);
 }
-__device__ __forceinline__ void unpack8(uint4 q, float *v) {
-  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    v[2 * i] = __uint_as_float(w[i] << 16);
-    v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
+__device__ __forceinline__ uint4 pack8(const float2 *v) {
+  return make_uint4(pack2(v[0]), pack2(v[1]), pack2(v[2]), pack2(v[3]));
+}
+__device__ __forceinline__ float2 unpack2(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
 }
 
 // ------------------------------------------------------------ geometry --
@@ -314,8 +334,9 @@ struct ConvArgs {
   int Do;              // output box side
   int s, e, R;         // input offset (0 / -2), extra patch row, patch rows
   int sub;             // 126-output sub-tiles per tile (1 to 4), one plane load each tile
-  int tpp;             // tiles per plane: ceil(Do * P / (126 sub))
-  int ntiles;          // B * tpp * Do output tiles, z fastest
+  int spp;             // sub-tiles per plane: ceil(Do * P / 126)
+  int tpp;             // tiles per plane: ceil(spp / sub), the last with the sub-tiles left over
+  int nsub;            // B * Do * spp sub-tiles, z fastest (see SubWalk)
   int nslot;           // input planes held in the shared-memory ring
   uint32_t slot_bytes;   // one input plane: CI * R * P * 16 (one TMA box)
   uint32_t slot_stride;  // slot_bytes rounded up to 1 KB
@@ -334,6 +355,46 @@ struct ConvArgs {
   int *err;
 };
 
+// A CTA's sub-tiles, in order: tile (b, j) of a plane marches up z, and a
+// tile is up to `sub` sub-tiles of one plane.  The CTAs' ranges are cut at
+// sub-tiles: cut at whole tiles, the busiest CTA had 21 sub-tiles of an average
+// 18.9 (side 64, three a tile).  tile() gives the sub-tiles [lo, hi) of the
+// next tile, `fresh` where its first two planes are not in the ring yet, `last`
+// where all three are used for the last time.
+struct SubWalk {
+  int b, j, z;       // the tile given last
+  int lo, hi;        // its sub-tiles
+  bool fresh, last;
+  int left, n;       // sub-tiles to come; sub-tiles of a whole tile of column j
+  bool first;
+  __device__ __forceinline__ void start(const ConvArgs &a, int s0, int s1) {
+    b = s0 / (a.spp * a.Do);
+    int r = s0 - b * a.spp * a.Do;
+    j = r / (a.sub * a.Do);
+    r -= j * a.sub * a.Do;
+    n = min(a.sub, a.spp - j * a.sub);
+    z = r / n - 1;
+    lo = r - (z + 1) * n;
+    left = s1 - s0;
+    first = true;
+  }
+  __device__ __forceinline__ bool tile(const ConvArgs &a) {
+    if (left <= 0) return false;
+    if (++z == a.Do) {
+      z = 0;
+      if (++j == a.tpp) j = 0, b++;
+      n = min(a.sub, a.spp - j * a.sub);
+    }
+    if (!first) lo = 0;
+    hi = min(n, lo + left);
+    left -= hi - lo;
+    fresh = first || z == 0;
+    last = left == 0 || z == a.Do - 1;
+    first = false;
+    return true;
+  }
+};
+
 // Forward / transposed convolution, CI input chunks (the GEMM's K, 16
 // channels per MMA), CO output chunks.  One MMA covers the three x-taps of
 // a (dz, dy) pair: its N = 3 * 8 CO columns are (dx, output channel), so
@@ -345,11 +406,19 @@ struct ConvArgs {
 // through shared memory; a tile of 128 rows thus yields TILE_OUT = 126
 // outputs and costs 9 CI / 2 MMAs of N = 24 CO instead of 27 CI / 2 of N =
 // 8 CO (the tensor core takes about as long for N = 96 as for N = 32).
-// Tiles are numbered z fastest (tile = ((b tpp) + j) Do + z) and every CTA
-// takes one contiguous range of them, marching up z: the input planes
+// Tiles are numbered z fastest and every CTA takes one contiguous range of
+// their sub-tiles (SubWalk), marching up z: the input planes
 // z+s .. z+s+2 of a tile sit in a ring of nslot shared-memory slots, so a
 // tile loads one new plane (three at the start of a column) and the planes
 // are released to the producer after their last use.
+// Bound by the issue of the MMAs and the epilogue's instructions about alike
+// (32 -> 32 channels, per sub-tile: 18 MMAs of about 50 cycles; 16 epilogue warps,
+// 2.3k cycles of arithmetic and stores and 1.1k of tensor-memory reads and
+// shuffles each, every fourth sub-tile).  64^3 inference, four layers, before ->
+// now 90.3 -> 81.6 us: ranges cut at sub-tiles and six ring slots (86.2 -> 81.6),
+// MMAs issued by a whole warp's uniform loop (88.5 -> 86.2), packed FP32 pairs, two
+// shuffles per output instead of three and the weights ahead of the wait
+// (90.2 -> 88.5).  Training on 8 crops of 32^3: with these 428 -> 360 us a step.
 template <int CI, int CO, int MODE>
 __global__ void __launch_bounds__(CONV_THREADS, 1)
     k_conv(const __grid_constant__ CUtensorMap tin, const ConvArgs a) {
@@ -363,6 +432,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
   constexpr uint32_t ACC_STRIDE = N <= 64 ? 64 : 128;   // TMEM columns per accumulator
   constexpr uint32_t NCOLS = NACC * ACC_STRIDE;         // 256 or 512 columns
   constexpr int MAXSLOT = 12;
+  constexpr int CU = MODE == FWD_LOSS || MODE == FWD_INFER ? 1 : CO;  // chunks used: 6 components there
+  constexpr int NU = 8 * CU;
   constexpr int XB = 3 * 2 * NW;                        // exchange floats per group and buffer
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // 1 KB-aligned base (TMA destinations; the host adds 1 KB of slack)
@@ -377,13 +448,14 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
   float *lsum = reinterpret_cast<float *>(bars + 2 * MAXSLOT + 2 * NACC + 3);  // 16 floats
   float *bsm = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(bars) + 352);  // 32 biases
   // boundary rows handed between TMEM lane quarters: [group][buffer][quarter
-  // 1..3][2][NW] (row 32q's x-shift 2 for lane 30 of the quarter below; row
-  // 32q's x-shift 1 + row 32q + 1's x-shift 2 for its lane 31)
+  // 1..3][2][NW] (for lanes 30 and 31 of the quarter below: row 32q's x-shift
+  // 2; row 32q's x-shift 1 + row 32q + 1's x-shift 2)
   float *xbuf = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(bars) + CONV_BARS);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // this CTA's tiles
-  const int t0 = (int)((long long)a.ntiles * blockIdx.x / gridDim.x);
-  const int t1 = (int)((long long)a.ntiles * (blockIdx.x + 1) / gridDim.x);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform
+  // this CTA's sub-tiles
+  SubWalk w;
+  w.start(a, (int)((long long)a.nsub * blockIdx.x / gridDim.x),
+          (int)((long long)a.nsub * (blockIdx.x + 1) / gridDim.x));
   // the next convolution may launch now: its blocks start once this grid's
   // blocks have all started (this grid is one wave: grid_for) and wait for
   // its completion before touching memory
@@ -403,44 +475,44 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(tslot, NCOLS);
-  // programmatic dependent launch: the barrier set-up and the tensor-memory
-  // allocation above overlap the tail of the previous convolution; every
-  // read of global memory (biases, weights, input planes, zin, targets) and
-  // every write follows the wait (a no-op for an ordinary launch)
+  // The weights, by the lane that set the barriers.  They are written by an
+  // ordinary launch (k_update), and the kernel that follows it in the chain is
+  // an ordinary launch too or lets its dependents start only past its own wait
+  // (k_infer_in), so this kernel starts with them complete and visible
+  if (threadIdx.x == 0) {
+    mb_expect(wbar, a.w_bytes);
+    bulk_load(wsm, a.wpack, a.w_bytes, wbar);
+  }
+  // programmatic dependent launch: the barrier set-up, the tensor-memory
+  // allocation and the weights above overlap the tail of the previous
+  // convolution; every other read of global memory (biases, input planes,
+  // zin, targets) and every write follows the wait (a no-op for an ordinary
+  // launch)
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (warp == 2) bsm[lane] = MODE != DGRAD && lane < (CO == 4 ? 32 : 6) ? __ldg(a.bias + lane) : 0.f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tbase = *tslot;
+  const uint32_t tbase = __shfl_sync(0xffffffffu, *tslot, 0);
   const int P2 = a.P * a.P;
 
   if (warp == 0) {
     if (lane == 0) {
-      // weights once, then the input planes of the tiles in order
-      mb_expect(wbar, a.w_bytes);
-      bulk_load(wsm, a.wpack, a.w_bytes, wbar);
-      // one lane runs this loop serially: the tile coordinates and the
-      // ring slot advance by increments (no division per plane)
+      // the input planes of the tiles in order; one lane runs this loop
+      // serially: the ring slot advances by increments (no division per plane)
       int g = 0, sl = 0, ph = 0;  // planes issued; slot and phase of the next
-      int z = t0 % a.Do, j = (t0 / a.Do) % a.tpp, b = t0 / (a.Do * a.tpp);
-      int y0 = (j * a.sub * TILE_OUT) / a.P;
+      int y0 = 0;
       bool ok = true;
-      for (int t = t0; ok && t < t1; t++) {
-        const bool fresh = t == t0 || z == 0;
-        for (int zp = fresh ? 0 : 2; zp < 3; zp++, g++) {
+      while (ok && w.tile(a)) {
+        if (w.fresh) y0 = (w.j * a.sub * TILE_OUT) / a.P;
+        for (int zp = w.fresh ? 0 : 2; zp < 3; zp++, g++) {
           if (*abort_flag || !mb_wait(&empty[sl], ph ^ 1, a.wait_limit, abort_flag)) {
             ok = false;
             break;
           }
           mb_expect(&full[sl], a.slot_bytes);
-          tma4(ring + sl * a.slot_stride, &tin, 0, y0 + a.s - a.e, z + a.s + zp, b * CI, &full[sl]);
+          tma4(ring + sl * a.slot_stride, &tin, 0, y0 + a.s - a.e, w.z + a.s + zp, w.b * CI, &full[sl]);
           if (++sl == a.nslot) sl = 0, ph ^= 1;
-        }
-        if (++z == a.Do) {  // next column of tiles
-          z = 0;
-          if (++j == a.tpp) j = 0, b++;
-          y0 = (j * a.sub * TILE_OUT) / a.P;
         }
       }
       if (!ok) {
@@ -453,103 +525,105 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
       mb_wait(wbar, 0, a.wait_limit, abort_flag);
     }
   } else if (warp == 1 || warp == 2) {
-    if (lane == 0) {
-      // Two issuing lanes (warps 1 and 2) take the sub-tiles in turn (sub-tile
-      // i on lane i % 2): while one does its waits and bookkeeping, the
-      // other's MMAs keep the tensor pipe fed.  Both wait for every plane and
-      // both release it (the empty barriers count two arrivals: a commit
-      // arrives once that lane's earlier MMAs are done).
-      const int r = warp - 1;
-      constexpr uint32_t idesc = idesc_bf16(N, false, false);
-      // Descriptors are built once; per MMA only the start-address field
-      // (bits 0-13, 16-byte units) moves, by an offset added to the whole
-      // 64-bit word (starts stay below 256 KB, so the field never carries).
-      const uint32_t cstride_u = (uint32_t)a.R * a.P;  // chunk stride in a slot, 16-byte units
-      const uint64_t bdesc0 = sdesc(saddr(wsm), 3 * CO * 128u, 128);
-      const uint64_t adesc_st = sdesc(0, cstride_u * 16u, 128);  // start 0
-      const uint32_t ring_u = saddr(ring) >> 4, stride_u = a.slot_stride >> 4;
-      uint32_t yrow[3];  // (dy + e) P, 16-byte units
+    // Two issuing warps (1 and 2) take the sub-tiles in turn (sub-tile
+    // i on warp i % 2): while one does its waits and bookkeeping, the
+    // other's MMAs keep the tensor pipe fed.  Both wait for every plane and
+    // both release it (the empty barriers count two arrivals: a commit
+    // arrives once that warp's earlier MMAs are done).  The whole warp runs
+    // the loop with warp-uniform values and one elected lane issues: the
+    // descriptors then stay in uniform registers.  Run by a single lane, an
+    // MMA took 71-130 cycles to issue for 18-36 of the tensor pipe.
+    const int r = warp - 1;
+    constexpr uint32_t idesc = idesc_bf16(N, false, false);
+    // Descriptors are built once; per MMA only the start-address field
+    // (bits 0-13, 16-byte units) moves, by an offset added to the whole
+    // 64-bit word (starts stay below 256 KB, so the field never carries).
+    const uint32_t cstride_u = (uint32_t)a.R * a.P;  // chunk stride in a slot, 16-byte units
+    const uint64_t bdesc0 = sdesc(saddr(wsm), 3 * CO * 128u, 128);
+    const uint64_t adesc_st = sdesc(0, cstride_u * 16u, 128);  // start 0
+    const uint32_t ring_u = saddr(ring) >> 4, stride_u = a.slot_stride >> 4;
+    uint32_t yrow[3];  // (dy + e) P, 16-byte units
 #pragma unroll
-      for (int q = 0; q < 3; q++) yrow[q] = (uint32_t)((q + a.e) * a.P);
-      // each lane runs this loop serially: plane slots, tile coordinates and
-      // accumulators advance by increments (no division per tile)
-      int i = 0, last_a = -1, last_aph = 0;
-      int gs = 0, gph = 0;  // slot and phase of the next plane to arrive
-      int ac = r, aph = 0;  // accumulator (i % NACC) of this lane's next sub-tile and its phase
-      int z = t0 % a.Do, j = (t0 / a.Do) % a.tpp;
-      int x0 = (j * a.sub * TILE_OUT) % a.P;  // the tile's first position in patch row y0
-      // phases seen complete ahead of their wait, by tests placed among the
-      // MMAs (the issue is throttled by the tensor pipe, so the tests cost
-      // nothing there): the next accumulator's release, the next plane
-      bool acc_ready = false, plane_ready = false;
-      bool ok = mb_wait(wbar, 0, a.wait_limit, abort_flag);
-      for (int t = t0; ok && t < t1; t++) {
-        const bool fresh = t == t0 || z == 0;
-        const bool last = t == t1 - 1 || z == a.Do - 1;
-        const bool more = t + 1 < t1;
-        for (int q = fresh ? 0 : 2; q < 3 && ok; q++) {
-          if (!plane_ready) ok = !*abort_flag && mb_wait(&full[gs], gph, a.wait_limit, abort_flag);
-          plane_ready = false;
-          if (++gs == a.nslot) gs = 0, gph ^= 1;
+    for (int q = 0; q < 3; q++) yrow[q] = (uint32_t)((q + a.e) * a.P);
+    // plane slots, tile coordinates and accumulators advance by increments
+    // (no division per tile)
+    int i = 0, last_a = -1, last_aph = 0;
+    int gs = 0, gph = 0;  // slot and phase of the next plane to arrive
+    int ac = r, aph = 0;  // accumulator (i % NACC) of this warp's next sub-tile and its phase
+    // phases seen complete ahead of their wait, by tests placed among the
+    // MMAs: the next accumulator's release, the next plane
+    bool acc_ready = false, plane_ready = false;
+    int x0 = 0;  // the tile's first position in patch row y0
+    bool ok = warp_wait(wbar, 0, a.wait_limit, abort_flag);
+    while (ok && w.tile(a)) {
+      if (w.fresh) x0 = (w.j * a.sub * TILE_OUT) % a.P;
+      for (int q = w.fresh ? 0 : 2; q < 3 && ok; q++) {
+        if (!plane_ready) ok = warp_wait(&full[gs], gph, a.wait_limit, abort_flag);
+        plane_ready = false;
+        if (++gs == a.nslot) gs = 0, gph ^= 1;
+      }
+      if (!ok) break;
+      // slots of the last three planes loaded: planes z+s, z+s+1, z+s+2
+      int sz[3];
+      sz[2] = gs == 0 ? a.nslot - 1 : gs - 1;
+      sz[1] = sz[2] == 0 ? a.nslot - 1 : sz[2] - 1;
+      sz[0] = sz[1] == 0 ? a.nslot - 1 : sz[1] - 1;
+      uint64_t ab[3];
+#pragma unroll
+      for (int dz = 0; dz < 3; dz++)
+        ab[dz] = adesc_st + (uint64_t)(ring_u + (uint32_t)sz[dz] * stride_u + (uint32_t)(x0 + a.s));
+      for (int sb = w.lo; sb < w.hi; sb++, i++) {
+        if ((i & 1) != r) continue;
+        if (!acc_ready && !warp_wait(&tempty[ac], aph ^ 1, a.wait_limit, abort_flag)) {
+          ok = false;
+          break;
         }
-        if (!ok) break;
-        // slots of the last three planes loaded: planes z+s, z+s+1, z+s+2
-        int sz[3];
-        sz[2] = gs == 0 ? a.nslot - 1 : gs - 1;
-        sz[1] = sz[2] == 0 ? a.nslot - 1 : sz[2] - 1;
-        sz[0] = sz[1] == 0 ? a.nslot - 1 : sz[1] - 1;
-        uint64_t ab[3];
+        tc_fence_after();
+        const uint32_t dacc = tbase + (uint32_t)ac * ACC_STRIDE;
+        const uint64_t so = (uint64_t)(sb * TILE_OUT);  // the sub-tile's rows, 16-byte units
+        const int nac = ac + 2 >= NACC ? ac + 2 - NACC : ac + 2, naph = ac + 2 >= NACC ? aph ^ 1 : aph;
+        auto taps = [&](int zy) {
+          const uint64_t at = ab[zy / 3] + so + (uint64_t)yrow[zy % 3];
 #pragma unroll
-        for (int dz = 0; dz < 3; dz++)
-          ab[dz] = adesc_st + (uint64_t)(ring_u + (uint32_t)sz[dz] * stride_u + (uint32_t)(x0 + a.s));
-        for (int sb = 0; sb < a.sub; sb++, i++) {
-          if ((i & 1) != r) continue;
-          if (!acc_ready && (*abort_flag || !mb_wait(&tempty[ac], aph ^ 1, a.wait_limit, abort_flag))) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t dacc = tbase + (uint32_t)ac * ACC_STRIDE;
-          const uint64_t so = (uint64_t)(sb * TILE_OUT);  // the sub-tile's rows, 16-byte units
-          const int nac = ac + 2 >= NACC ? ac + 2 - NACC : ac + 2, naph = ac + 2 >= NACC ? aph ^ 1 : aph;
+          for (int k = 0; k < CI / 2; k++)
+            mma_bf16(dacc, at + (uint64_t)(2 * k) * cstride_u,
+                     bdesc0 + (uint64_t)((zy * CI + 2 * k) * 3 * CO * 8), idesc, (zy | k) != 0 ? 1u : 0u);
+        };
+        if (elect_one()) {
 #pragma unroll
-          for (int zy = 0; zy < 9; zy++) {
-            if (zy == 5) {
-              acc_ready = mb_test(&tempty[nac], naph ^ 1);
-              if (sb + 2 >= a.sub && more) plane_ready = mb_test(&full[gs], gph);
-            }
-            const uint64_t at = ab[zy / 3] + so + (uint64_t)yrow[zy % 3];
+          for (int zy = 0; zy < 6; zy++) taps(zy);
+        }
+        __syncwarp();
+        acc_ready = __all_sync(0xffffffffu, mb_test(&tempty[nac], naph ^ 1));
+        if (sb + 2 >= w.hi && w.left > 0) plane_ready = __all_sync(0xffffffffu, mb_test(&full[gs], gph));
+        if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < CI / 2; k++)
-              mma_bf16(dacc, at + (uint64_t)(2 * k) * cstride_u,
-                       bdesc0 + (uint64_t)((zy * CI + 2 * k) * 3 * CO * 8), idesc, (zy | k) != 0 ? 1u : 0u);
-          }
+          for (int zy = 6; zy < 9; zy++) taps(zy);
           mma_commit(&tfull[ac]);
-          last_a = ac;
-          last_aph = aph;
-          ac = nac;
-          aph = naph;
         }
-        if (!ok) break;
-        // release the planes this tile used for the last time
+        __syncwarp();
+        last_a = ac;
+        last_aph = aph;
+        ac = nac;
+        aph = naph;
+      }
+      if (!ok) break;
+      // release the planes this tile used for the last time
+      if (elect_one()) {
         mma_commit(&empty[sz[0]]);
-        if (last) {
+        if (w.last) {
           mma_commit(&empty[sz[1]]);
           mma_commit(&empty[sz[2]]);
         }
-        if (++z == a.Do) {  // next column of tiles
-          z = 0;
-          if (++j == a.tpp) j = 0;
-          x0 = (j * a.sub * TILE_OUT) % a.P;
-        }
       }
-      if (!ok) {
-        *abort_flag = 1;
-        atomicExch(a.err, DEVERR_CNN_TIMEOUT);
-      }
-      // the MMAs issued last complete before the tensor memory is freed
-      if (last_a >= 0) mb_wait(&tfull[last_a], last_aph, a.wait_limit, abort_flag);
+      __syncwarp();
     }
+    if (!ok && lane == 0) {
+      *abort_flag = 1;
+      atomicExch(a.err, DEVERR_CNN_TIMEOUT);
+    }
+    // the MMAs issued last complete before the tensor memory is freed
+    if (last_a >= 0) warp_wait(&tfull[last_a], last_aph, a.wait_limit, abort_flag);
   } else {
     // epilogue: CONV_GROUPS groups of 4 warps take the tiles in turn (group
     // e / 4 the tiles with local index i % CONV_GROUPS == e / 4); warp w
@@ -557,46 +631,57 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
     // tile), 8 columns of each x-shift at a time
     const int e = warp - 3, q = warp & 3, grp = e >> 2;
     const int m = q * 32 + lane;
-    const float keep1 = lane < 31 ? 1.f : 0.f, keep2 = lane < 30 ? 1.f : 0.f;
+    const float2 keep = both(lane < 31 ? 1.f : 0.f);
     float osc[6];
 #pragma unroll
     for (int k = 0; k < 6; k++) osc[k] = MODE == FWD_INFER ? __ldg(a.oscale + k) : 0.f;
     const bool store_z = a.zout != nullptr;
     float *xg = xbuf + grp * 2 * XB;
     float lacc = 0.f;
-    // the tile's (b, j, z) and this thread's positions in its sub-tiles,
-    // updated as z marches
-    int z = t0 % a.Do, j = (t0 / a.Do) % a.tpp, b = t0 / (a.Do * a.tpp);
+    // this thread's positions in the tile's sub-tiles, updated as z marches
     int fA = 0, xA = 0, yA = 0;  // this thread's row in sub-tile 0: offset, x, y
     // a sub-tile further: TILE_OUT = q126 rows of P + r126
     const int q126 = TILE_OUT / a.P, r126 = TILE_OUT - q126 * a.P;
     const long long cstr = (long long)a.Pz * P2;  // one chunk of 8 channels further
-    const float4 *bias4 = reinterpret_cast<const float4 *>(bsm);
-    bool fresh = true, stop = false;
+    const float2 *bias2 = reinterpret_cast<const float2 *>(bsm);
+    bool stop = false;
     int i = 0, own = 0;
-    for (int t = t0; t < t1 && !stop; t++) {
-      if (fresh) {
-        fA = j * a.sub * TILE_OUT + m;
+    while (!stop && w.tile(a)) {
+      if (w.fresh) {
+        fA = w.j * a.sub * TILE_OUT + m;
         yA = fA / a.P;
         xA = fA - yA * a.P;
-        fresh = false;
-      }
-      const int zc = z, bc = b;
-      if (++z == a.Do) {  // next column
-        z = 0;
-        fresh = true;
-        if (++j == a.tpp) {
-          j = 0;
-          b++;
-        }
       }
       int x = xA, y = yA;
-      for (int sb = 0; sb < a.sub; sb++, i++, x += r126, y += q126) {
+      for (int sb = 0; sb < w.lo; sb++) {  // a range that starts inside a tile
+        x += r126;
+        y += q126;
+        if (x >= a.P) x -= a.P, y++;
+      }
+      for (int sb = w.lo; sb < w.hi; sb++, i++, x += r126, y += q126) {
         if (x >= a.P) x -= a.P, y++;
         const bool mine = (i % CONV_GROUPS) == grp;
         const int ac = i % NACC, aph = (i / NACC) & 1;
-        float v[NW];
-        if (mine) {
+        if (!mine) continue;
+        const int f = fA + sb * TILE_OUT;
+        const bool inside = m < TILE_OUT && f < P2;
+        const bool valid = inside && x < a.Do && y < a.Do;
+        const long long vox = (long long)w.z * P2 + f;
+        const long long o0 = (long long)w.b * CO * cstr + vox;
+        // what the tile's outputs need from memory is on its way while the MMAs run
+        uint4 zq[CO];
+        float4 tq[2];
+        if (MODE == DGRAD) {
+#pragma unroll
+          for (int c = 0; c < CO; c++) zq[c] = valid ? a.zin[o0 + c * cstr] : make_uint4(0, 0, 0, 0);
+        }
+        if (MODE == FWD_LOSS) {
+          const float4 *tp = a.target + ((long long)w.b * a.Pz * P2 + vox) * 2;
+#pragma unroll
+          for (int k = 0; k < 2; k++) tq[k] = valid ? tp[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        float2 v[NU / 2];
+        {
           float *xw = xg + (own & 1) * XB;
           bool ok = !*abort_flag && mb_wait(&tfull[ac], aph, a.wait_limit, abort_flag);
           ok = __all_sync(0xffffffffu, ok);
@@ -604,26 +689,29 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
             tc_fence_after();
             const uint32_t ta = tbase + ((uint32_t)(q * 32) << 16) + (uint32_t)ac * ACC_STRIDE;
 #pragma unroll
-            for (int c = 0; c < CO; c++) {
+            for (int c = 0; c < CU; c++) {
               float d[24];  // columns 8c.. of x-shift 0, 1, 2
               tmem_ld3x8(ta + 8 * c, ta + NW + 8 * c, ta + 2 * NW + 8 * c, d);
-              // lane 0: its x-shift 2; lane 1: lane 0's x-shift 1 + its x-shift 2
-              float hx[8];
+              // out[m] = d0[m] + (d1 + d2[. + 1])[m + 1]
+              float2 w[4];
 #pragma unroll
-              for (int k = 0; k < 8; k++) {
-                const float up = __shfl_up_sync(0xffffffffu, d[8 + k], 1);
-                hx[k] = lane == 0 ? d[16 + k] : up + d[16 + k];
+              for (int k = 0; k < 4; k++) {
+                const float2 s2 = make_float2(__shfl_down_sync(0xffffffffu, d[16 + 2 * k], 1),
+                                              __shfl_down_sync(0xffffffffu, d[17 + 2 * k], 1));
+                w[k] = fma2(s2, keep, make_float2(d[8 + 2 * k], d[9 + 2 * k]));
               }
-              if (q > 0 && lane < 2) {
-                float4 *xs = reinterpret_cast<float4 *>(xw + 2 * (q - 1) * NW + lane * NW + 8 * c);
-                xs[0] = make_float4(hx[0], hx[1], hx[2], hx[3]);
-                xs[1] = make_float4(hx[4], hx[5], hx[6], hx[7]);
+              if (q > 0 && lane == 0) {
+                float4 *xs = reinterpret_cast<float4 *>(xw + 2 * (q - 1) * NW + 8 * c);
+                xs[0] = make_float4(d[16], d[17], d[18], d[19]);
+                xs[1] = make_float4(d[20], d[21], d[22], d[23]);
+                xs[NW / 4] = make_float4(w[0].x, w[0].y, w[1].x, w[1].y);
+                xs[NW / 4 + 1] = make_float4(w[2].x, w[2].y, w[3].x, w[3].y);
               }
 #pragma unroll
-              for (int k = 0; k < 8; k++) {
-                const float s1 = __shfl_down_sync(0xffffffffu, d[8 + k], 1);
-                const float s2 = __shfl_down_sync(0xffffffffu, d[16 + k], 2);
-                v[8 * c + k] = fmaf(s2, keep2, fmaf(s1, keep1, d[k]));
+              for (int k = 0; k < 4; k++) {
+                const float2 s1 = make_float2(__shfl_down_sync(0xffffffffu, w[k].x, 1),
+                                              __shfl_down_sync(0xffffffffu, w[k].y, 1));
+                v[4 * c + k] = fma2(s1, keep, make_float2(d[2 * k], d[2 * k + 1]));
               }
             }
             tc_fence_before();
@@ -641,82 +729,61 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
           if (q < 3 && lane >= 30) {
             const float4 *xr = reinterpret_cast<const float4 *>(xw + 2 * q * NW + (lane - 30) * NW);
 #pragma unroll
-            for (int c = 0; c < NW / 4; c++) {  // quarter q + 1's rows
+            for (int c = 0; c < NU / 4; c++) {  // quarter q + 1's rows
               const float4 h = xr[c];
-              v[4 * c] += h.x;
-              v[4 * c + 1] += h.y;
-              v[4 * c + 2] += h.z;
-              v[4 * c + 3] += h.w;
+              v[2 * c] = add2(v[2 * c], make_float2(h.x, h.y));
+              v[2 * c + 1] = add2(v[2 * c + 1], make_float2(h.z, h.w));
             }
           }
           own++;
         }
-        if (!mine || m >= TILE_OUT) continue;
-        const int f = fA + sb * TILE_OUT;
-        if (f >= P2) continue;
-        const bool valid = x < a.Do && y < a.Do;
-        const long long vox = (long long)zc * P2 + f;
+        if (!inside) continue;
         if (MODE == FWD_GELU) {
-          const long long o0 = (long long)bc * CO * cstr + vox;
 #pragma unroll
           for (int c = 0; c < CO; c++) {
-            const float4 b0 = bias4[2 * c], b1 = bias4[2 * c + 1];
-            const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-            float zv[8], hv[8];
+            float2 zv[4], hv[4];
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-              const float zz = valid ? v[8 * c + k] + bb[k] : 0.f;
-              zv[k] = zz;
-              hv[k] = gelu_f(zz);
+            for (int k = 0; k < 4; k++) {
+              zv[k] = add2(v[4 * c + k], bias2[4 * c + k]);
+              hv[k] = gelu2(zv[k]);
             }
+            const uint4 none = make_uint4(0, 0, 0, 0);
             const long long o = o0 + c * cstr;
-            if (store_z) a.zout[o] = pack8(zv);
-            a.out[o] = pack8(hv);
+            if (store_z) a.zout[o] = valid ? pack8(zv) : none;
+            a.out[o] = valid ? pack8(hv) : none;
           }
         } else if (MODE == FWD_LOSS) {
           // 6 output components in chunk 0 (N = 16: chunk 1 stays zero)
-          float tv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+          const float tv[6] = {tq[0].x, tq[0].y, tq[0].z, tq[0].w, tq[1].x, tq[1].y};
+          float2 gv[4] = {both(0.f), both(0.f), both(0.f), both(0.f)};
           if (valid) {
-            const float4 *tp = a.target + ((long long)bc * a.Pz * P2 + vox) * 2;
-            const float4 t0v = tp[0], t1v = tp[1];
-            tv[0] = t0v.x; tv[1] = t0v.y; tv[2] = t0v.z; tv[3] = t0v.w;
-            tv[4] = t1v.x; tv[5] = t1v.y;
-          }
-          float gv[8];
 #pragma unroll
-          for (int k = 0; k < 8; k++) {
-            float g = 0.f;
-            if (valid && k < 6) {
-              const float d = v[k] + bsm[k] - tv[k];
-              lacc += d * d;
-              g = a.loss_scale * d;
+            for (int k = 0; k < 3; k++) {
+              const float2 d = make_float2(v[k].x + bsm[2 * k] - tv[2 * k], v[k].y + bsm[2 * k + 1] - tv[2 * k + 1]);
+              lacc += d.x * d.x;
+              lacc += d.y * d.y;
+              gv[k] = make_float2(a.loss_scale * d.x, a.loss_scale * d.y);
             }
-            gv[k] = g;
           }
-          const long long o = ((long long)(bc * CO) * a.Pz) * P2 + vox;
-          a.out[o] = pack8(gv);
+          a.out[o0] = pack8(gv);
         } else if (MODE == FWD_INFER) {
           if (valid) {
             const long long n3 = (long long)a.Do * a.Do * a.Do;
-            const long long o = ((long long)zc * a.Do + y) * a.Do + x;
+            const long long o = ((long long)w.z * a.Do + y) * a.Do + x;
 #pragma unroll
-            for (int k = 0; k < 6; k++) a.infer_out[k * n3 + o] = (double)((v[k] + bsm[k]) * osc[k]);
+            for (int k = 0; k < 3; k++) {
+              a.infer_out[2 * k * n3 + o] = (double)((v[k].x + bsm[2 * k]) * osc[2 * k]);
+              a.infer_out[(2 * k + 1) * n3 + o] = (double)((v[k].y + bsm[2 * k + 1]) * osc[2 * k + 1]);
+            }
           }
         } else {  // DGRAD: g = dL/dh * gelu'(z) of the output's layer
 #pragma unroll
           for (int c = 0; c < CO; c++) {
-            const long long o = ((long long)(bc * CO + c) * a.Pz) * P2 + vox;
-            float gv[8];
-            if (valid) {
-              float zv[8];
-              unpack8(a.zin[o], zv);
+            const uint32_t zw[4] = {zq[c].x, zq[c].y, zq[c].z, zq[c].w};
+            float2 gv[4];
 #pragma unroll
-              for (int k = 0; k < 8; k++) gv[k] = v[8 * c + k] * gelu_grad_f(zv[k]);
-            } else {
-#pragma unroll
-              for (int k = 0; k < 8; k++) gv[k] = 0.f;
-            }
-            a.out[o] = pack8(gv);
+            for (int k = 0; k < 4; k++) gv[k] = mul2(v[4 * c + k], gelu_grad2(unpack2(zw[k])));
+            a.out[o0 + c * cstr] = valid ? pack8(gv) : make_uint4(0, 0, 0, 0);
           }
         }
       }
@@ -759,12 +826,14 @@ struct WgradArgs {
 };
 
 // h: CI chunks (A operand, shifted in x), g: CO chunks (B operand, shifted in
-// y).  Bound by the L2-to-SM copies and the MMAs about alike: per step (one
+// y).  Bound by the latency of a step's copies (two planes of g in flight),
+// above the L2-to-SM copies and the MMAs themselves: per step (one
 // plane of one row block) six boxes of 64-byte positions and 3 KBp / 16 MMAs of
 // N = 96 (56 cycles each) for 27 taps.  With the taps stacked four at a time
 // on the rows (N = 32) every position was copied 34 times and took 7 MMAs of 52
 // cycles per 16 positions: 85.6 us for a 32 x 32-channel layer of 8 crops of
-// 32^3 (959 MB of copies, 11.7 TB/s).
+// 32^3 (959 MB of copies, 11.7 TB/s); now 53.4 us with one issuing lane for the
+// three dz and 33.6 us with an issuing warp each.
 template <int CI, int CO>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_wgrad(const __grid_constant__ CUtensorMap th, const __grid_constant__ CUtensorMap tg,
@@ -780,7 +849,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
            *gempty = gfull + WG_GRADS, *done = gempty + WG_GRADS;
   uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(done + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // warp-uniform
   const int split = blockIdx.x;
   // steps (sample, row block, z), z fastest
   const long long nsteps = (long long)a.B * a.kpp * a.Do;
@@ -792,13 +861,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (threadIdx.x == 0) {
     for (int i = 0; i < WG_PLANES; i++) {
       mb_init(&hfull[i], 1);
-      mb_init(&hempty[i], 1);
+      mb_init(&hempty[i], 3);  // one arrival per issuing lane
     }
     for (int i = 0; i < WG_GRADS; i++) {
       mb_init(&gfull[i], 1);
-      mb_init(&gempty[i], 1);
+      mb_init(&gempty[i], 3);
     }
-    mb_init(done, 1);
+    mb_init(done, 3);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -823,7 +892,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tbase = *tslot;
+  const uint32_t tbase = __shfl_sync(0xffffffffu, *tslot, 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -867,47 +936,55 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       for (int i = gi < WG_GRADS ? 0 : gi - WG_GRADS; i < gi; i++)
         mb_wait(&gfull[i % WG_GRADS], (i / WG_GRADS) & 1, a.wait_limit, abort_flag);
     }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_bf16(N, true, true);
-      const int nkk = a.KBp / 16;
-      int pc = 0, have = 0, gi = 0;  // plane of dz = 0, planes waited for, planes of g
-      bool ok = true;
-      for (int s = s0; s < s1; s++) {
-        const bool last = s + 1 == s1 || (s + 1) % a.Do == 0;  // of its column here
-        for (; ok && have < pc + 3; have++)
-          ok = !*abort_flag &&
-               mb_wait(&hfull[have % WG_PLANES], (have / WG_PLANES) & 1, a.wait_limit, abort_flag);
-        const int st = gi % WG_GRADS;
-        ok = ok && !*abort_flag && mb_wait(&gfull[st], (gi / WG_GRADS) & 1, a.wait_limit, abort_flag);
+  } else if (warp <= 3) {
+    // One issuing warp per dz, each with its own accumulator: a warp's waits
+    // and commits run beside the others' MMAs.  Warp dz meets plane j of a
+    // column (of n steps here, n + 2 planes) at step j - dz, and releases the
+    // planes it does not use as they arrive.  The loop is the whole warp's and
+    // uniform, one elected lane issues (see k_conv).
+    constexpr uint32_t idesc = idesc_bf16(N, true, true);
+    const int nkk = a.KBp / 16, dz = warp - 1;
+    const uint32_t dacc = tbase + (uint32_t)dz * ACC;
+    // MN-major, no swizzle: SBO = stride of 8-element MN groups (one
+    // chunk), LBO = stride of 8-row K groups (128 B); 16 positions are
+    // 256 bytes on, 16 in the address field
+    const uint64_t ad0 = sdesc(saddr(smem), 128, chunk), bd0 = sdesc(saddr(gs), 128, chunk);
+    const uint32_t h_u = a.h_bytes >> 4, g_u = a.g_bytes >> 4;
+    int sl = 0, ph = 0, g0 = 0;  // slot and phase of the next plane, steps of the columns before
+    bool ok = true, any = false;
+    for (int s = s0; ok && s < s1;) {
+      const int n = min(s1 - s, a.Do - s % a.Do);
+      for (int j = 0; j < n + 2; j++) {
+        ok = warp_wait(&hfull[sl], ph, a.wait_limit, abort_flag);
         if (!ok) break;
-        tc_fence_after();
-        // MN-major, no swizzle: SBO = stride of 8-element MN groups (one
-        // chunk), LBO = stride of 8-row K groups (128 B)
-        const uint64_t bd = sdesc(saddr(gs + st * a.g_bytes), 128, chunk);
-        uint64_t ad[3];
-#pragma unroll
-        for (int dz = 0; dz < 3; dz++)
-          ad[dz] = sdesc(saddr(smem + (pc + dz) % WG_PLANES * a.h_bytes), 128, chunk);
-        for (int kk = 0; kk < nkk; kk++) {
-#pragma unroll
-          for (int dz = 0; dz < 3; dz++)  // 16 positions: 256 bytes on, 16 in the address field
-            mma_bf16(tbase + dz * ACC, ad[dz] + 16 * kk, bd + 16 * kk, idesc, (gi | kk) != 0);
+        if (j < dz || j - dz >= n) {
+          if (elect_one()) mb_arrive(&hempty[sl]);
+        } else {
+          const int gi = g0 + j - dz, st = gi % WG_GRADS;
+          ok = warp_wait(&gfull[st], (gi / WG_GRADS) & 1, a.wait_limit, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            uint64_t ad = ad0 + (uint64_t)(sl * h_u), bd = bd0 + (uint64_t)(st * g_u);
+            for (int kk = 0; kk < nkk; kk++, ad += 16, bd += 16)
+              mma_bf16(dacc, ad, bd, idesc, any || kk != 0);
+            mma_commit(&gempty[st]);
+            mma_commit(&hempty[sl]);
+          }
+          any = true;
         }
-        mma_commit(&gempty[st]);
-        mma_commit(&hempty[pc % WG_PLANES]);
-        if (last) {
-          mma_commit(&hempty[(pc + 1) % WG_PLANES]);
-          mma_commit(&hempty[(pc + 2) % WG_PLANES]);
-        }
-        pc += last ? 3 : 1;
-        gi++;
+        __syncwarp();
+        if (++sl == WG_PLANES) sl = 0, ph ^= 1;
       }
-      if (!ok) {
-        *abort_flag = 1;
-        atomicExch(a.err, DEVERR_CNN_TIMEOUT);
-      }
-      if (gi > 0) mma_commit(done);
+      s += n;
+      g0 += n;
+    }
+    if (!ok && lane == 0) {
+      *abort_flag = 1;
+      atomicExch(a.err, DEVERR_CNN_TIMEOUT);
+    }
+    if (elect_one()) {
+      if (any) mma_commit(done);
       else mb_arrive(done);
     }
   } else {
@@ -927,11 +1004,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       for (int c0 = 0; c0 < N; c0 += W) {
         float v[W];
         tmem_ld<W>(tbase + ((uint32_t)(q * 32) << 16) + dz * ACC + c0, v);
-        if (m > 3 * 8 * CI) continue;  // rows beyond the ones: nothing reads them
+        if (m <= 3 * 8 * CI)  // rows beyond the ones: nothing reads them
 #pragma unroll
-        for (int c = 0; c < W; c += 4)
-          *reinterpret_cast<float4 *>(dst + c0 + c) =
-              none ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+          for (int c = 0; c < W; c += 4)
+            *reinterpret_cast<float4 *>(dst + c0 + c) =
+                none ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        __syncwarp();  // the next tensor-memory load is of the whole warp
       }
     }
   }

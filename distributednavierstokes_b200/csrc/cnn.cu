@@ -122,13 +122,14 @@ struct Partials {
 // With `reduce` every parameter's gradient from the split-K partials of its
 // layer, with `adam` the Adam update, and the BF16 packing of every weight.
 // Work is numbered over quads of the partials' columns (dy, co), so that a
-// thread reads 16 bytes of each split; 16 threads share a quad's splits (each
-// adds every 16th, the sums are added in order), all loads in flight at once.
+// thread reads 16 bytes of each split; 8 threads share a quad's splits (each
+// adds every 8th, the sums are added in order), seven loads in flight at once.
 // One launch at the step's end: as four reductions between the backward kernels
 // (5.2 us each, ordinary launches that kept the next convolution from starting
 // early) and an Adam launch (5.9 us, two double pow per thread) they were 27 us
-// of a 545 us training step.  26 us: the splits' sums are read once (49 MB).
-constexpr int UP_PARTS = 16, UP_QUADS = 16;
+// of a 545 us training step.  23 us for the 49 MB of the splits' sums, in one
+// wave of blocks (26 us with 16 threads a quad and twice the blocks).
+constexpr int UP_PARTS = 8, UP_QUADS = 32;
 __host__ __device__ inline int up_quads(int L, int cin) {  // of layer L: weights, then biases
   const int coch = L == 3 ? 2 : 4;
   return 3 * 3 * cin * (3 * 2 * coch) + 2 * coch;
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(UP_PARTS *UP_QUADS)
       const long stride = 3L * 128 * (24 * (q.L == 3 ? 2 : 4));
       const int ns = pt.nsplit[q.L];
       const float *src = pt.part[q.L] + q.at;
-#pragma unroll 10
+#pragma unroll 7
       for (int sp = part; sp < ns; sp += UP_PARTS) {
         const float4 x = *reinterpret_cast<const float4 *>(src + sp * stride);
         g.x += x.x;
@@ -529,7 +530,7 @@ int setup_conv_attr(dnsb_cnn *c, size_t smem) {
 // 15 % where the padding needs a copy per chunk (crop 32: 4 rows of 40).
 size_t wgrad_smem(int P, int R, int ci, int co) {
   const size_t chunk = (size_t)((R * P + 15) / 16 * 16) * 16;
-  return WG_PLANES * 4 * ci * chunk + WG_GRADS * 3 * co * chunk + 256 + 1024;
+  return WG_PLANES * 3 * ci * chunk + WG_GRADS * 3 * co * chunk + 256 + 1024;
 }
 int wgrad_rows(int P, int Do, int ci, int co) {
   int best = 0;
@@ -719,7 +720,7 @@ int run_wgrad(dnsb_cnn *c, Volume &V, int L) {
   a.KBp = (a.KB + 15) / 16 * 16;
   a.whole = a.KB == a.KBp;
   a.kpp = (a.Do + 2 + a.R - 1) / a.R;
-  a.h_bytes = 4u * CI * a.KBp * 16;
+  a.h_bytes = 3u * CI * a.KBp * 16;
   a.g_bytes = 3u * CO * a.KBp * 16;
   a.wait_limit = WAIT_LIMIT;
   a.err = c->deverr;

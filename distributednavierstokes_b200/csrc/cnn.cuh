@@ -45,9 +45,8 @@
 // to a multiple of 16) is one TMA box [chunk][R rows][x] per shift; an x
 // shift runs past the row end into zeros where g is zero anyway, a y shift
 // starts above or below the volume in zeros.  A CTA marches up z, so that
-// each plane of h is copied once for its three dz.  The row slot after the
-// three dx holds ones, which makes that row of dz = 0 the bias gradient.
-// Split-K partials are reduced in a fixed order.
+// each plane of h is copied once for its three dz.  The bias gradient is the
+// sum of g, formed by the epilogue warps while the MMAs run.  Split-K partials are reduced in a fixed order.
 //
 // Warp roles: warp 0 issues the TMA copies; warps 1 and 2 of the convolution,
 // 1 to 3 of the weight gradient issue the MMAs (the whole warp runs the loop,
@@ -810,7 +809,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
 // ------------------------------------------------------ weight gradient --
 
 constexpr int WG_PLANES = 4;  // planes of h in shared memory: three in use, one ahead
-constexpr int WG_GRADS = 2;   // planes of g
+constexpr int WG_GRADS = 3;   // planes of g
 
 struct WgradArgs {
   int P, B;         // volume geometry
@@ -819,21 +818,21 @@ struct WgradArgs {
   int whole;        // one TMA box per shift holds all chunks (KB == KBp), else one per chunk
   int kpp;          // K-blocks per plane: ceil((Do + 2) / R)
   int nsplit;       // K splits = CTAs
-  uint32_t h_bytes, g_bytes;  // one plane of h (four row slots) and of g (three shifts)
+  uint32_t h_bytes, g_bytes;  // one plane of h and of g (three shifts each)
   unsigned wait_limit;
   float *partial;   // [split][dz][128][N]
   int *err;
 };
 
 // h: CI chunks (A operand, shifted in x), g: CO chunks (B operand, shifted in
-// y).  Bound by the latency of a step's copies (two planes of g in flight),
-// above the L2-to-SM copies and the MMAs themselves: per step (one
+// y).  Bound by the MMAs (about 50 cycles each) and the set-up and stores around them
+// (a third plane of g in flight: 34.1 -> 33.1 us): per step (one
 // plane of one row block) six boxes of 64-byte positions and 3 KBp / 16 MMAs of
 // N = 96 (56 cycles each) for 27 taps.  With the taps stacked four at a time
 // on the rows (N = 32) every position was copied 34 times and took 7 MMAs of 52
 // cycles per 16 positions: 85.6 us for a 32 x 32-channel layer of 8 crops of
 // 32^3 (959 MB of copies, 11.7 TB/s); now 53.4 us with one issuing lane for the
-// three dz and 33.6 us with an issuing warp each.
+// three dz and 33.1 us with an issuing warp each.
 template <int CI, int CO>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_wgrad(const __grid_constant__ CUtensorMap th, const __grid_constant__ CUtensorMap tg,
@@ -865,7 +864,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
     for (int i = 0; i < WG_GRADS; i++) {
       mb_init(&gfull[i], 1);
-      mb_init(&gempty[i], 3);
+      mb_init(&gempty[i], 3 + 4);  // and one per summing warp
     }
     mb_init(done, 3);
     *abort_flag = 0;
@@ -877,12 +876,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int n = (int)((WG_PLANES * a.h_bytes + WG_GRADS * a.g_bytes) / 16);
     for (int i = threadIdx.x; i < n; i += NTHREADS) z[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-  }
-  // the row slot after the three dx: BF16 ones in every plane slot, never copied over
-  for (int st = 0; st < WG_PLANES; st++) {
-    uint4 *p = reinterpret_cast<uint4 *>(smem + st * a.h_bytes + 3 * CI * chunk);
-    const uint32_t one2 = 0x3F803F80u;
-    for (int i = threadIdx.x; i < (int)(CI * chunk / 16); i += NTHREADS) p[i] = make_uint4(one2, one2, one2, one2);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (warp == 1) tmem_alloc(tslot, NCOLS);
@@ -990,7 +983,42 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   } else {
     const int q = warp & 3;
     const int m = q * 32 + lane;
-    const bool ok = mb_wait(done, 0, a.wait_limit, abort_flag) && !*abort_flag;
+    // while the MMAs run, a warp per chunk sums g over the positions of its
+    // unshifted copy: the bias gradient (a row of ones among h's rows gave it
+    // before, in the shared memory that the third plane of g takes now)
+    float2 sum[4] = {both(0.f), both(0.f), both(0.f), both(0.f)};
+    bool ok = true;
+    for (int gi = 0; ok && gi < s1 - s0; gi++) {
+      const int st = gi % WG_GRADS;
+      ok = warp_wait(&gfull[st], (gi / WG_GRADS) & 1, a.wait_limit, abort_flag);
+      if (!ok) break;
+      if (q < CO) {
+        const uint4 *p = reinterpret_cast<const uint4 *>(gs + st * a.g_bytes + q * chunk);
+        for (int i = lane; i < a.KB; i += 32) {
+          const uint4 g = p[i];
+          const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+          for (int k = 0; k < 4; k++) sum[k] = add2(sum[k], unpack2(gw[k]));
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mb_arrive(&gempty[st]);
+    }
+    if (q < CO) {
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          sum[k] = add2(sum[k], make_float2(__shfl_xor_sync(0xffffffffu, sum[k].x, o),
+                                            __shfl_xor_sync(0xffffffffu, sum[k].y, o)));
+      if (lane == 0) {  // the partial row after dz = 0's
+        float4 *dst = reinterpret_cast<float4 *>(a.partial + ((long long)split * 3 * 128 + 24 * CI) * N + 8 * q);
+        dst[0] = make_float4(sum[0].x, sum[0].y, sum[1].x, sum[1].y);
+        dst[1] = make_float4(sum[2].x, sum[2].y, sum[3].x, sum[3].y);
+      }
+    }
+    const bool all = mb_wait(done, 0, a.wait_limit, abort_flag);
+    ok = ok && all && !*abort_flag;
     if (!ok) {
       *abort_flag = 1;
       atomicExch(a.err, DEVERR_CNN_TIMEOUT);
@@ -1004,7 +1032,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       for (int c0 = 0; c0 < N; c0 += W) {
         float v[W];
         tmem_ld<W>(tbase + ((uint32_t)(q * 32) << 16) + dz * ACC + c0, v);
-        if (m <= 3 * 8 * CI)  // rows beyond the ones: nothing reads them
+        if (m < 3 * 8 * CI)  // rows beyond: whatever follows in shared memory, nothing reads them
 #pragma unroll
           for (int c = 0; c < W; c += 4)
             *reinterpret_cast<float4 *>(dst + c0 + c) =

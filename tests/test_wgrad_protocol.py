@@ -1,6 +1,6 @@
 """Barrier protocol of the weight-gradient kernel (cnn.cuh, k_wgrad), simulated
-on the CPU: the copying lane, the three MMA-issuing warps (one per dz), copies that
-land late and in any order, MMAs that finish late (each warp's in order, with
+on the CPU: the copying lane, the three MMA-issuing warps (one per dz), two of the
+warps that sum g, copies that land late and in any order, MMAs that finish late (each warp's in order, with
 their commits), run in random interleavings.  No run may deadlock, overwrite a slot that an
 unfinished MMA reads, or let an MMA read a plane other than its own.
 """
@@ -8,7 +8,7 @@ import random
 
 import pytest
 
-PLANES, GRADS = 4, 2
+PLANES, GRADS = 4, 3
 
 
 class Bar:
@@ -31,7 +31,7 @@ def simulate(B, kpp, Do, nsplit, split, rng):
     n = B * kpp * Do
     s0, s1 = n * split // nsplit, n * (split + 1) // nsplit
     hfull, hempty = [Bar(1) for _ in range(PLANES)], [Bar(3) for _ in range(PLANES)]
-    gfull, gempty = [Bar(1) for _ in range(GRADS)], [Bar(3) for _ in range(GRADS)]
+    gfull, gempty = [Bar(1) for _ in range(GRADS)], [Bar(3 + 2) for _ in range(GRADS)]
     hslot, gslot = [None] * PLANES, [None] * GRADS
     copies = []                                  # in flight
     mmas = [[], [], []]                          # per lane: (slots read, barriers to arrive on)
@@ -91,7 +91,20 @@ def simulate(B, kpp, Do, nsplit, split, rng):
             s += n
             g0 += n
 
-    agents = {"p": producer(), 0: issuer(0), 1: issuer(1), 2: issuer(2)}
+    def summer(out):
+        for gi in range(s1 - s0):
+            st = gi % GRADS
+            while not gfull[st].passed((gi // GRADS) & 1):
+                yield "wait"
+            assert gslot[st] == divmod(s0 + gi, Do)
+            yield "go"                           # reading: nothing may land in the slot meanwhile
+            assert gslot[st] == divmod(s0 + gi, Do)
+            out.append(s0 + gi)
+            gempty[st].complete()
+            yield "go"
+
+    summed = [], []
+    agents = {"p": producer(), 0: issuer(0), 1: issuer(1), 2: issuer(2), "s": summer(summed[0]), "t": summer(summed[1])}
     idle = 0
     while agents or copies or any(mmas):
         acts = list(agents) + (["copy"] if copies else []) + [("mma", d) for d in range(3) if mmas[d]]
@@ -109,7 +122,7 @@ def simulate(B, kpp, Do, nsplit, split, rng):
             except StopIteration:
                 del agents[a]
         assert idle < 2000, "deadlock"
-    assert read == [list(range(s0, s1))] * 3
+    assert read == [list(range(s0, s1))] * 3 and summed == (list(range(s0, s1)),) * 2
 
 
 @pytest.mark.parametrize("B,kpp,Do,nsplit", [(1, 1, 1, 1), (1, 2, 1, 1), (2, 3, 2, 1), (2, 2, 5, 3),

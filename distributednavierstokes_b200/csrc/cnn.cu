@@ -121,14 +121,15 @@ struct Partials {
 
 // With `reduce` every parameter's gradient from the split-K partials of its
 // layer, with `adam` the Adam update, and the BF16 packing of every weight.
-// Work is numbered over quads of the partials' columns (dy, co), so that a
-// thread reads 16 bytes of each split; 8 threads share a quad's splits (each
+// Work is numbered over quads of the partials' columns (dy, co), rows (dx, ci)
+// fastest, so that a thread reads 16 bytes of each split and a warp 512; 8 threads share a quad's splits (each
 // adds every 8th, the sums are added in order), seven loads in flight at once.
 // One launch at the step's end: as four reductions between the backward kernels
 // (5.2 us each, ordinary launches that kept the next convolution from starting
 // early) and an Adam launch (5.9 us, two double pow per thread) they were 27 us
-// of a 545 us training step.  23 us for the 49 MB of the splits' sums, in one
-// wave of blocks (26 us with 16 threads a quad and twice the blocks).
+// of a 545 us training step.  15 us for the 49 MB of the splits' sums, in one
+// wave of blocks (26 us with 16 threads a quad and twice the blocks, 23 us with columns
+// fastest in the partials).
 constexpr int UP_PARTS = 8, UP_QUADS = 32;
 __host__ __device__ inline int up_quads(int L, int cin) {  // of layer L: weights, then biases
   const int coch = L == 3 ? 2 : 4;
@@ -165,13 +166,14 @@ __global__ void __launch_bounds__(UP_PARTS *UP_QUADS)
       q.L = L;
       if (r >= 9 * cin * N4) {
         q.co = 4 * (r - 9 * cin * N4);
-        q.at = 24L * cich * N + q.co;
+        q.at = 128L * q.co + 4 * 24 * cich;
       } else {
-        const int n4 = r % N4, row = r / N4, dz = row / (3 * cin), dx = row / cin % 3;
-        q.ci = row % cin;
+        // rows fastest, as in the partials
+        const int row = r % (3 * cin), n4 = r / (3 * cin) % N4, dz = r / (3 * cin * N4), dx = row / cin;
+        q.ci = row - dx * cin;
         q.co = 4 * n4 % (8 * coch);
         q.t = (dz * 3 + 4 * n4 / (8 * coch)) * 3 + dx;
-        q.at = (128L * dz + 8 * cich * dx + q.ci) * N + 4 * n4;
+        q.at = ((long)(dz * N4 + n4) * 128 + 8 * cich * dx + q.ci) * 4;
       }
       break;
     }

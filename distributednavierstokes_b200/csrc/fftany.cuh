@@ -123,7 +123,7 @@ __device__ __forceinline__ void fa_step2(int N1, int N2, int P, int LS, int L, c
 // Complex FFT along z of L contiguous lines of S, in place (k_fftz).
 template <int TIER, bool INV>
 __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
-    k_fftz_any(int n, int N1, int N2, int L, long long nlines, double2 *__restrict__ S,
+    k_fftz_any(int n, int N1, int N2, int L, long long nlines, double2 *S,
                const double2 *__restrict__ twz, int dep) {
   extern __shared__ double2 smem[];
   const int P = fa_pitch(N2), LS = N1 * P;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
 // here (two passes at the copy rate: 41 us); 32^3: 6.8 -> 5.8 us.
 template <int TIER, int YMODE>
 __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
-    k_y_any(Geo g, int N1, int N2, int L, double2 *__restrict__ S, const double2 *__restrict__ twy,
+    k_y_any(Geo g, int N1, int N2, int L, double2 *S, const double2 *__restrict__ twy,
             const double *__restrict__ lam1, const double *__restrict__ lam2,
             const double *__restrict__ lam3, int dep) {
   extern __shared__ double2 smem[];

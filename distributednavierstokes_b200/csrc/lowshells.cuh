@@ -173,7 +173,7 @@ __device__ __forceinline__ int ls_shell(int k2) {
 // factors into f, the corrections G = (f(shell) - 1) u_hat / N in place;
 // eref[s] < 0 leaves shell s unforced.
 __global__ void __launch_bounds__(256) k_ls_modes(Geo g, int KM, double2 *Gm, double *E,
-                                                  const double *__restrict__ eref, double *f, int nb, int dep) {
+                                                  const double *eref, double *f, int nb, int dep) {
   const int W = 2 * KM + 1, H = KM + 1;
   const double N = (double)g.nx * g.ny * g.nz;
   const int nM = 3 * H * W * W;

@@ -12,7 +12,11 @@ namespace dnsb {
 // memory that another kernel writes or reads, so a chain of dependent
 // launches keeps stream order.  What another kernel of the stream writes is
 // read through plain pointers: __ldg and const __restrict__ allow the compiler
-// to move a load above the wait.
+// to move a load above the wait, and so does a __restrict__ pointer that the
+// kernel also writes through (the compiler may take the wait's assembly not to
+// touch what it points to).  __restrict__ is for the context's tables, which no
+// kernel of a step writes, and for outputs that are only written, from values
+// loaded past the wait (tests/test_dependent_launches.py lists both).
 __device__ __forceinline__ void pdl_wait(int dep) {
   if (dep) asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -17,7 +17,7 @@ constexpr int F4_THREADS = 256;
 // Complex FFT along z of L contiguous lines of S (n = N1*N2 = nz); INV
 // scales by 1/nz.  Shared memory: transpose buffer + n twiddles.
 template <int N1, int N2, bool INV>
-__global__ void __launch_bounds__(F4_THREADS, 2) k_fftz4(Geo g, double2 *__restrict__ S, int L,
+__global__ void __launch_bounds__(F4_THREADS, 2) k_fftz4(Geo g, double2 *S, int L,
                                                          const double2 *__restrict__ twz, int dep) {
   constexpr int n = N1 * N2;
   extern __shared__ double2 smem[];

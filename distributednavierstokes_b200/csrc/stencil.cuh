@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(MC_X *MC_Y, 3)
     k_momentum_march(Geo g, Fields3 q, CFields3 u, Fields3 out, const double *p,
                      double A, double dt, double B, double adt, int readq,
                      const double2 *__restrict__ ymet, double theta, int planes,
-                     const double *__restrict__ dtp, CnTabArgs ct, int dep) {
+                     const double *dtp, CnTabArgs ct, int dep) {
   __shared__ __align__(16) double ring[4][3][MP_N];
   pdl_trigger(dep);
   pdl_wait(dep);

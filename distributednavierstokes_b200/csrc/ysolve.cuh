@@ -103,7 +103,7 @@ constexpr size_t ythomas_smem(int mr) { return sizeof(double) * (size_t)mr * TY_
 
 template <int MR>
 __global__ void __launch_bounds__(TY_LINES *TY_CHUNKS, MR <= 8 ? 3 : 1)
-    k_ythomas(Geo g, double2 *__restrict__ S, const double *__restrict__ cin,
+    k_ythomas(Geo g, double2 *S, const double *__restrict__ cin,
               const double *__restrict__ ay, const double *__restrict__ by,
               const double *__restrict__ cy, const double *__restrict__ lam1,
               const double *__restrict__ lam3, int dep) {

@@ -1,0 +1,83 @@
+"""Source rules of the programmatic dependent launches (csrc/pdl.cuh), read from
+the CUDA sources: a kernel that waits for the grids before it may not let the
+compiler load what they write ahead of the wait.  A latent race of this kind
+shows in no result until a compiler or a register count changes, so the rule is
+checked where it can be broken.
+"""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                    "distributednavierstokes_b200", "csrc")
+
+# tables of a context, written when it is created and by no kernel of a step
+TABLES = {"twz", "twy", "twM", "twN", "twn", "lam1", "lam2", "lam3", "ymet", "cin", "ay", "by", "cy",
+          "xph", "yph", "zph", "ph"}
+# outputs that a kernel only writes, from values loaded past its wait
+OUTPUTS = {"k_rfftx_any": {"S"}, "k_irfftx_any": {"out"}, "k_rfftx4": {"S"}, "k_irfftx4": {"out"},
+           "k_gradmom_pipe": {"p_out"}, "k_ls_xsums": {"A"}, "k_ls_sums": {"out"}}
+# read-only loads of tables, and of a closure's biases and scales (written by
+# ordinary launches before the first convolution of a pass)
+LDG = {"g.rdy", "g.rdyu", "lam1", "lam2", "lam3", "ay", "by", "cy", "cin", "twM", "twN", "a.bias", "a.oscale"}
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def closing(text, i):
+    """Index past the bracket that closes the one at i."""
+    pair = {"(": ")", "{": "}"}[text[i]]
+    depth = 0
+    for j in range(i, len(text)):
+        depth += (text[j] == text[i]) - (text[j] == pair)
+        if depth == 0:
+            return j + 1
+    raise AssertionError("unbalanced source")
+
+
+def kernels(text):
+    """(name, parameters, body) of every __global__ function."""
+    for m in re.finditer(r"__global__\s+void\b", text):
+        i = m.end()
+        bounds = re.match(r"\s*__launch_bounds__\s*", text[i:])
+        if bounds:
+            i = closing(text, i + bounds.end())
+        name = re.match(r"\s*(\w+)\s*", text[i:])
+        i += name.end()
+        j = closing(text, i)
+        k = text.index("{", j)
+        if text[j:k].strip():
+            continue  # a declaration
+        yield name.group(1), text[i + 1:j - 1], text[k:closing(text, k)]
+
+
+def dependents():
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh")):
+            for name, params, body in kernels(source(f)):
+                if "pdl_wait(" in body or "griddepcontrol.wait" in body:
+                    yield name, params, body
+
+
+DEPENDENTS = list(dependents())
+
+
+def test_the_parser_sees_them():
+    names = {k[0] for k in DEPENDENTS}
+    assert {"k_momentum_march", "k_gradmom_pipe", "k_fftz_any", "k_y_any", "k_rfftx_any", "k_irfftx_any",
+            "k_fftz4", "k_rfftx4", "k_irfftx4", "k_ythomas", "k_cn", "k_grad", "k_sfs_stage", "k_les_dt",
+            "k_maxabs3", "k_conv", "k_wgrad", "k_infer_in", "k_sp_stage", "k_ls_modes"} <= names
+
+
+@pytest.mark.parametrize("name,params,body", DEPENDENTS, ids=[k[0] for k in DEPENDENTS])
+def test_what_other_kernels_write_is_read_through_plain_pointers(name, params, body):
+    restricted = set(re.findall(r"__restrict__\s+(\w+)", params))
+    assert restricted <= TABLES | OUTPUTS.get(name, set()), name
+    assert set(re.findall(r"__ldg\(\s*&?([\w.]+)", body)) <= LDG, name
+    # nothing is loaded through an output
+    for out in OUTPUTS.get(name, set()):
+        assert not re.search(rf"=\s*{out}\s*\[", body), (name, out)

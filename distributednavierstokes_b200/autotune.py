@@ -2,21 +2,23 @@
 reference).
 
 For a periodic box of side n it times one RK3 step under candidate launch
-shapes (dnsb_tuning: lines per CTA of the Stockham x-, y- and z-transforms
-and of the four-step z-transform, the per-cell kernels' block shape) by
-coordinate descent from the defaults: each field in turn takes the value
-of its candidates that makes the step fastest (CUDA events over `steps`
-steps after two warm-up steps; the best of `repeats` timings), the others
-held.  The results do not depend on the shapes, only the time does.
-Choices are cached per device name and box in a JSON file.
+shapes (dnsb_tuning: lines per CTA of the x-, y- and z-transforms, the per-cell
+kernels' block shape) by coordinate descent from the defaults: each field in
+turn takes the value of its candidates that makes the step fastest (CUDA events
+over `steps` steps after two warm-up steps; the best of `repeats` timings), the
+others held.  What is returned names the fields that were changed and no others,
+so that the rest keep the library's own rules.  The results do not depend on the
+shapes, only the time does.  Choices are cached per device name and box in a JSON
+file, for the library build that they were timed with.
 """
+import hashlib
 import json
 import os
 import time
 
 import torch
 
-from . import api
+from . import _lib, api
 
 CANDIDATES = {
     "lines_z4": (2, 4, 8, 16),
@@ -24,6 +26,24 @@ CANDIDATES = {
     "lines_x": (2, 4, 8),
     "cell": ((64, 2), (32, 4), (128, 2), (32, 8)),
 }
+# sides whose z-transform is the kernel with a compile-time split, which takes
+# lines_z4 (launch_fftz, csrc/dnsb.cu); every other one takes lines_z
+Z4_SIDES = (32, 48, 64, 96)
+
+
+def candidates(n):
+    """CANDIDATES for an n^3 box: the z-transform's field is the one its kernel
+    reads."""
+    return {("lines_z" if f == "lines_z4" and n not in Z4_SIDES else f): v for f, v in CANDIDATES.items()}
+
+
+def _build_id():
+    """What identifies the library build (a timed choice is its build's)."""
+    try:
+        with open(_lib.LIBPATH, "rb") as f:
+            return hashlib.sha256(f.read()).hexdigest()[:16]
+    except OSError:
+        return None
 
 
 def default_cache():
@@ -56,31 +76,32 @@ def _time_step(n, visc, tuning, steps, repeats, device):
 
 
 def tune(n, visc=1e-3, steps=10, repeats=3, device=None, log=None):
-    """Coordinate descent over CANDIDATES for an n^3 periodic explicit box;
-    returns (tuning dict in effect, ms per step, {candidate: ms})."""
+    """Coordinate descent over candidates(n) for an n^3 periodic explicit box;
+    returns (tuning dict of the changed fields, ms per step, {candidate: ms})."""
     device = device or torch.device("cuda", torch.cuda.current_device())
     cur = {}
-    best_ms, eff = _time_step(n, visc, cur, steps, repeats, device)
+    best_ms, _ = _time_step(n, visc, cur, steps, repeats, device)
     tried = {"default": best_ms}
-    for field, values in CANDIDATES.items():
+    for field, values in candidates(n).items():
         for v in values:
             trial = dict(cur)
             if field == "cell":
                 trial["cell_bx"], trial["cell_by"] = v
             else:
                 trial[field] = v
-            ms, e2 = _time_step(n, visc, trial, steps, repeats, device)
+            ms, _ = _time_step(n, visc, trial, steps, repeats, device)
             tried[f"{field}={v}"] = ms
             if ms < best_ms * 0.99:   # keep a change only if it gains more than 1 %
-                best_ms, cur, eff = ms, trial, e2
+                best_ms, cur = ms, trial
         if log:
             log(f"n={n}: after {field}: {best_ms:.4f} ms {cur}")
-    return eff, best_ms, tried
+    return cur, best_ms, tried
 
 
 def tune_sizes(sizes, visc=1e-3, cache=None, device=None, log=None, refresh=False):
     """{n: tuning dict} for every box side in `sizes`, from the cache file
-    (keyed by device name and side) or measured now and stored."""
+    (keyed by device name and side, of this library build) or measured now and
+    stored."""
     device = device or torch.device("cuda", torch.cuda.current_device())
     cache = cache or default_cache()
     name = torch.cuda.get_device_name(device)
@@ -91,16 +112,16 @@ def tune_sizes(sizes, visc=1e-3, cache=None, device=None, log=None, refresh=Fals
                 data = json.load(f)
         except (OSError, ValueError):
             data = {}
-    out, report = {}, {}
+    out, report, build = {}, {}, _build_id()
     for n in sorted(set(int(v) for v in sizes)):
         key = f"{name}|periodic|{n}"
-        if key in data and not refresh:
+        if key in data and not refresh and data[key].get("build") == build:
             out[n] = data[key]["tuning"]
             report[n] = dict(data[key], cached=True)
             continue
         t0 = time.perf_counter()
         eff, ms, tried = tune(n, visc, device=device, log=log)
-        data[key] = {"tuning": eff, "ms_per_step": ms, "tried": tried,
+        data[key] = {"tuning": eff, "ms_per_step": ms, "tried": tried, "build": build,
                      "seconds": time.perf_counter() - t0}
         out[n] = eff
         report[n] = dict(data[key], cached=False)

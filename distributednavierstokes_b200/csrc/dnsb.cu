@@ -1564,7 +1564,7 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
     const long cols = (long)c->tgrid.x * c->tgrid.y;
     const int mp = envint("DNSB_MOMZ", 0), gp = tuned(tun ? tun->gm_planes : 0, "DNSB_GMZ", 0);
     c->mom_planes = std::max(1, std::min(64, mp > 0 ? mp : march_planes(cols, nz, 8, c->nsm * 17L / 10)));
-    c->gm_planes = std::max(gp > 0 ? 4 : 1, std::min(256, gp > 0 ? gp : march_planes(cols, nz, 22, c->nsm * 257L / 100)));
+    c->gm_planes = std::max(1, std::min(256, gp > 0 ? gp : march_planes(cols, nz, 22, c->nsm * 257L / 100)));
     c->gmgrid = dim3(c->tgrid.x, c->tgrid.y, (nz + c->gm_planes - 1) / c->gm_planes);
     c->tgrid.z = (nz + c->mom_planes - 1) / c->mom_planes;
   }
@@ -1679,9 +1679,10 @@ int dnsb_set_stream(dnsb_ctx *c, void *stream) {
 
 int dnsb_get_tuning(const dnsb_ctx *c, dnsb_tuning *t) {
   if (!c || !t) return DNSB_EINVAL;
-  t->lines_x = c->Lx;
-  t->lines_z = c->Lz;
-  t->lines_y = c->Ly;
+  // what the kernels that run take, so that a context created from it launches alike
+  t->lines_x = c->ax.tier ? any_lines_x(c->g, c->ax, c->Lx_set) : c->Lx;
+  t->lines_z = c->az.tier && !c->use_tma ? any_lines_z(c->g, c->az, c->g.nkx, c->Lz_set) : c->Lz;
+  t->lines_y = c->ay_.tier ? any_lines_y(c->g, c->ay_, c->g.nkx, c->Ly_set) : c->Ly;
   t->lines_z4 = c->L4z;
   t->cell_bx = (int)c->cblock.x;
   t->cell_by = (int)c->cblock.y;

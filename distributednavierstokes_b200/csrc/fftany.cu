@@ -44,20 +44,10 @@ int even(int nz, int L) {
   return (nz + groups - 1) / groups;
 }
 
-int lines_z(const Geo &g, const AnySplit &sp, int nkx, int asked) {
-  const int n = sp.n1 * sp.n2;
-  return lines_for(sp, asked, (long long)g.ny * nkx, 2, sizeof(double2) * sp.n1 * fa_pitch(sp.n2),
-                   sizeof(double2) * n);
-}
 size_t smem_z(const AnySplit &sp, int L) {
   return sizeof(double2) * ((size_t)L * sp.n1 * fa_pitch(sp.n2) + sp.n1 * sp.n2);
 }
 
-int lines_y(const Geo &g, const AnySplit &sp, int nkx, int asked) {
-  const int n = sp.n1 * sp.n2;
-  const int L = lines_for(sp, asked, (long long)nkx * g.nz, 4, sizeof(double2) * n, sizeof(double2) * n);
-  return even(g.nz, std::min(L, 16));
-}
 size_t smem_y(const AnySplit &sp, int L) {
   return sizeof(double2) * (size_t)(L + 1) * sp.n1 * sp.n2;
 }
@@ -66,12 +56,25 @@ size_t line_x(const AnySplit &sp) {
   return sizeof(double2) * ((size_t)sp.n1 * fa_pitch(sp.n2) + sp.n1 * sp.n2 + 1);
 }
 size_t fixed_x(const AnySplit &sp) { return sizeof(double2) * (2 * (size_t)sp.n1 * sp.n2 + 1); }
-int lines_x(const Geo &g, const AnySplit &sp, int asked) {
-  return even(g.nz, std::min(16, lines_for(sp, asked, (long long)g.ny * g.nz, 4, line_x(sp), fixed_x(sp))));
-}
 size_t smem_x(const AnySplit &sp, int L) { return fixed_x(sp) + L * line_x(sp); }
 
 }  // namespace
+
+int any_lines_x(const Geo &g, const AnySplit &sp, int asked) {
+  return even(g.nz, std::min(16, lines_for(sp, asked, (long long)g.ny * g.nz, 4, line_x(sp), fixed_x(sp))));
+}
+
+int any_lines_y(const Geo &g, const AnySplit &sp, int nkx, int asked) {
+  const int n = sp.n1 * sp.n2;
+  const int L = lines_for(sp, asked, (long long)nkx * g.nz, 4, sizeof(double2) * n, sizeof(double2) * n);
+  return even(g.nz, std::min(L, 16));
+}
+
+int any_lines_z(const Geo &g, const AnySplit &sp, int nkx, int asked) {
+  const int n = sp.n1 * sp.n2;
+  return lines_for(sp, asked, (long long)g.ny * nkx, 2, sizeof(double2) * sp.n1 * fa_pitch(sp.n2),
+                   sizeof(double2) * n);
+}
 
 AnySplit any_split(int n) {
 #define FA_LIST(R) R,
@@ -127,7 +130,7 @@ cudaError_t any_allow(int device, const AnySplit &x, const AnySplit &y, const An
 cudaError_t any_fftz(const Geo &g, const AnySplit &sp, int nkx, int lines, bool inv, double2 *S,
                      const double2 *twz, cudaStream_t stream) {
   const long long nlines = (long long)g.ny * nkx;
-  const int L = lines_z(g, sp, nkx, lines);
+  const int L = any_lines_z(g, sp, nkx, lines);
   const dim3 grid((unsigned)((nlines + L - 1) / L)), block(threads_for(L * std::max(sp.n1, sp.n2)));
   return by_tier(sp.tier, [&](auto t) {
     constexpr int T = decltype(t)::value;
@@ -138,7 +141,7 @@ cudaError_t any_fftz(const Geo &g, const AnySplit &sp, int nkx, int lines, bool 
 
 cudaError_t any_y(const Geo &g, const AnySplit &sp, int nkx, int lines, int mode, double2 *S, const double2 *twy,
                   const double *lam1, const double *lam2, const double *lam3, cudaStream_t stream) {
-  const int L = lines_y(g, sp, nkx, lines);
+  const int L = any_lines_y(g, sp, nkx, lines);
   const dim3 grid((unsigned)(nkx * ((g.nz + L - 1) / L))), block(threads_for(L * std::max(sp.n1, sp.n2)));
   return by_tier(sp.tier, [&](auto t) {
     constexpr int T = decltype(t)::value;
@@ -153,7 +156,7 @@ cudaError_t any_rfftx(const Geo &g, const AnySplit &sp, int lines, int mode, dou
                       const double *a,
                       const double *b, const double *c, const double2 *twM, const double2 *twN,
                       cudaStream_t stream) {
-  const int L = lines_x(g, sp, lines);
+  const int L = any_lines_x(g, sp, lines);
   const dim3 grid((unsigned)(g.ny * ((g.nz + L - 1) / L)));
   return by_tier(sp.tier, [&](auto t) {
     constexpr int T = decltype(t)::value;
@@ -168,7 +171,7 @@ cudaError_t any_rfftx(const Geo &g, const AnySplit &sp, int lines, int mode, dou
 
 cudaError_t any_irfftx(const Geo &g, const AnySplit &sp, int lines, int mode, const double2 *S, double *out,
                        const double2 *twM, const double2 *twN, cudaStream_t stream) {
-  const int L = lines_x(g, sp, lines);
+  const int L = any_lines_x(g, sp, lines);
   const dim3 grid((unsigned)(g.ny * ((g.nz + L - 1) / L)));
   return by_tier(sp.tier, [&](auto t) {
     constexpr int T = decltype(t)::value;

@@ -16,6 +16,13 @@ AnySplit any_split(int n);
 // opt in to the shared memory of the kernels of one split
 cudaError_t any_allow(int device, const AnySplit &x, const AnySplit &y, const AnySplit &z);
 
+// lines per block of the transforms along x, y and z (over nkx kx planes): `asked`
+// within what fits, or with 0 the launch's own rule.  What they return gives
+// itself when asked for.
+int any_lines_x(const Geo &g, const AnySplit &sp, int asked);
+int any_lines_y(const Geo &g, const AnySplit &sp, int nkx, int asked);
+int any_lines_z(const Geo &g, const AnySplit &sp, int nkx, int asked);
+
 // Each returns the launch's status; the launches are launch_pdl's.  nkx: kx planes transformed; lines: lines per
 // block (0: the launch's own rule).
 cudaError_t any_fftz(const Geo &g, const AnySplit &sp, int nkx, int lines, bool inv, double2 *S,

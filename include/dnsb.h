@@ -59,12 +59,13 @@ typedef struct dnsb_ctx dnsb_ctx;
 
 /* Launch shapes of a context (no counterpart in the reference; the
  * autotuner of the batched ensemble picks them per grid).  0 keeps the
- * default (or the DNSB_* environment override): lines per CTA of the
- * Stockham x-, z- and y-transforms and of the four-step z-transform, the
- * block shape of the per-cell kernels (cell_bx a multiple of 32,
- * cell_bx * cell_by <= 256), z-planes per CTA of the fused projection +
- * momentum.  Results do not depend on them (every line and cell is computed
- * by the same arithmetic). */
+ * default (or the DNSB_* environment override): lines per CTA of the x-, z-
+ * and y-transforms, of the z-transform with a compile-time split (nz of 32, 48,
+ * 64, 96: lines_z4, elsewhere lines_z), the block shape of the per-cell kernels
+ * (cell_bx a multiple of 32, cell_bx * cell_by <= 256), z-planes per CTA of the
+ * fused projection + momentum.  The x-transforms by warps (a compile-time split
+ * of nx/2 and two CTAs per SM) take no lines_x.  Results do not depend on any of
+ * them (every line and cell is computed by the same arithmetic). */
 typedef struct {
   int lines_x, lines_z, lines_y, lines_z4;
   int cell_bx, cell_by;

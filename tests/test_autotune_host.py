@@ -62,3 +62,32 @@ def test_cache_per_device_and_side(monkeypatch, tmp_path):
     monkeypatch.setattr(torch.cuda, "get_device_name", lambda device=None: "OtherGPU")
     autotune.tune_sizes([32], cache=cache, device="cpu")
     assert calls == [32, 64, 32, 32]
+
+
+def test_an_untouched_default_asks_for_nothing(monkeypatch):
+    """What no candidate improved is left to the library: the fields in effect
+    are not handed back as if they had been asked for."""
+    effect = dict(lines_x=8, lines_z=4, lines_y=8, lines_z4=8, cell_bx=64, cell_by=2, gm_planes=22)
+    monkeypatch.setattr(autotune, "_time_step", lambda *a: (1.0, dict(effect, **a[2])))
+    assert autotune.tune(128, device="cpu")[0] == {}
+    monkeypatch.setattr(autotune, "_time_step",
+                        lambda *a: (0.5 if a[2].get("lines_y") == 4 else 1.0, dict(effect, **a[2])))
+    assert autotune.tune(128, device="cpu")[0] == {"lines_y": 4}
+
+
+def test_a_choice_of_another_build_is_timed_again(monkeypatch, tmp_path):
+    calls = []
+    monkeypatch.setattr(autotune, "tune", lambda n, visc, **kw: (calls.append(n) or {}, 1.0, {}))
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda device=None: "TestGPU")
+    cache = str(tmp_path / "tuning.json")
+    for build in ("a", "a", "b"):
+        monkeypatch.setattr(autotune, "_build_id", lambda: build)
+        autotune.tune_sizes([32], cache=cache, device="cpu")
+    assert calls == [32, 32]
+    with open(cache) as f:            # an entry of before the builds were told apart
+        data = json.load(f)
+    del data["TestGPU|periodic|32"]["build"]
+    with open(cache, "w") as f:
+        json.dump(data, f)
+    autotune.tune_sizes([32], cache=cache, device="cpu")
+    assert calls == [32, 32, 32]

@@ -162,6 +162,24 @@ def test_launch_shapes_do_not_change_results(D):
     s1.close()
 
 
+@pytest.mark.parametrize("n,x,z,y", [
+    ((32, 32, 32), 16, 8, 8),         # nx/2 = 4 x 4: 16 lines keep 64 threads busy
+    ((128, 128, 128), 16, 8, 8),      # 8 x 16 along z and y: 8 lines of 16 columns fill 128 threads
+    ((108, 108, 108), None, None, None),
+    ((60, 45, 10), None, None, None)])
+def test_the_shapes_in_effect_launch_alike(D, n, x, z, y):
+    """setup(tuning=s.tuning()) takes the launch shapes of s: the rules' own
+    where nothing was asked for."""
+    s0 = D.setup(n=n, visc=1e-2)
+    t = s0.tuning()
+    for k, v in (("lines_x", x), ("lines_z", z), ("lines_y", y)):
+        assert v is None or t[k] == v, (k, t)
+    s1 = D.setup(n=n, visc=1e-2, tuning=t)
+    assert s1.tuning() == t
+    s0.close()
+    s1.close()
+
+
 def test_autotuner_picks_valid_shapes(D, tmp_path):
     """The coordinate-descent autotuner on a small box returns shapes that
     the library accepts, caches them, and reads the cache back."""

@@ -206,6 +206,17 @@ __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
                : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
+// The tensor memory of a block, then the programmatic dependents' launch: they
+// may start once every block of this grid (one wave: grid_for) has its columns,
+// and wait for its completion before touching memory.  In the other order a
+// dependent block on the same SM could take the columns first (a kernel takes 256
+// or 512 of the 512) and wait for this grid, one of whose blocks then waits for
+// the columns: no end.  With it a grid that holds tensor memory and waits for
+// another waits for one that holds all of its own, also beside other streams'.
+__device__ __forceinline__ void tmem_alloc_then_trigger(uint32_t *slot, uint32_t ncols) {
+  tmem_alloc(slot, ncols);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void tmem_free(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                : "memory");
@@ -455,10 +466,6 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
   SubWalk w;
   w.start(a, (int)((long long)a.nsub * blockIdx.x / gridDim.x),
           (int)((long long)a.nsub * (blockIdx.x + 1) / gridDim.x));
-  // the next convolution may launch now: its blocks start once this grid's
-  // blocks have all started (this grid is one wave: grid_for) and wait for
-  // its completion before touching memory
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < a.nslot; i++) {
@@ -473,7 +480,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(tslot, NCOLS);
+  if (warp == 1) tmem_alloc_then_trigger(tslot, NCOLS);
   // The weights, by the lane that set the barriers.  They are written by an
   // ordinary launch (k_update), and the kernel that follows it in the chain is
   // an ordinary launch too or lets its dependents start only past its own wait
@@ -854,9 +861,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // steps (sample, row block, z), z fastest
   const long long nsteps = (long long)a.B * a.kpp * a.Do;
   const int s0 = (int)(nsteps * split / a.nsplit), s1 = (int)(nsteps * (split + 1) / a.nsplit);
-  // programmatic dependent launch: dependents may launch once every block
-  // of this grid has started; they wait for its completion before memory
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < WG_PLANES; i++) {
@@ -879,7 +883,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     __syncthreads();
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  if (warp == 1) tmem_alloc(tslot, NCOLS);
+  if (warp == 1) tmem_alloc_then_trigger(tslot, NCOLS);
   // the previous kernel's outputs (activations, gradients) complete and
   // visible past this (a no-op for an ordinary launch)
   asm volatile("griddepcontrol.wait;" ::: "memory");

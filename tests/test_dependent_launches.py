@@ -81,3 +81,20 @@ def test_what_other_kernels_write_is_read_through_plain_pointers(name, params, b
     # nothing is loaded through an output
     for out in OUTPUTS.get(name, set()):
         assert not re.search(rf"=\s*{out}\s*\[", body), (name, out)
+
+
+def test_tensor_memory_is_taken_before_the_dependents_may_start():
+    """A dependent block allocates tensor memory before it waits for the grid
+    ahead of it.  Were it let in before that grid's blocks hold theirs, it could
+    take the columns of an SM that one of them still needs, and neither would end."""
+    text = source("cnn.cuh")
+    helper = text[text.index("void tmem_alloc_then_trigger("):]
+    helper = helper[helper.index("{"):closing(helper, helper.index("{"))]
+    assert 0 <= helper.index("tmem_alloc(") < helper.index("griddepcontrol.launch_dependents")
+    assert text.count("griddepcontrol.launch_dependents") == 1
+    users = {k[0]: k[2] for k in kernels(text) if "tmem_free(" in k[2]}
+    assert set(users) == {"k_conv", "k_wgrad"}
+    for name, body in users.items():
+        assert body.count("tmem_alloc_then_trigger(") == 1 and "tmem_alloc(" not in body, name
+        assert "pdl_trigger(" not in body, name
+        assert body.index("tmem_alloc_then_trigger(") < body.index("griddepcontrol.wait"), name

@@ -522,7 +522,9 @@ size_t conv_smem(int ci, int co, int P, int R, int *nslot, uint32_t *slot, uint3
 template <int CI, int CO, int MODE>
 int setup_conv_attr(dnsb_cnn *c, size_t smem) {
   if (smem > (size_t)MAX_SMEM) return cfail(c, DNSB_EUNSUP, "convolution needs %zu bytes of shared memory", smem);
-  CC(c, cudaFuncSetAttribute(k_conv<CI, CO, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the limit is the kernel's, not this closure's: only ever raised, so that a
+  // closure of another side in another thread cannot lower it before the launch
+  CC(c, dnsb::raise_smem(c->device, k_conv<CI, CO, MODE>, smem));
   return 0;
 }
 

@@ -98,3 +98,13 @@ def test_tensor_memory_is_taken_before_the_dependents_may_start():
         assert body.count("tmem_alloc_then_trigger(") == 1 and "tmem_alloc(" not in body, name
         assert "pdl_trigger(" not in body, name
         assert body.index("tmem_alloc_then_trigger(") < body.index("griddepcontrol.wait"), name
+
+
+def test_shared_memory_limits_are_only_raised():
+    """A kernel's dynamic shared-memory limit belongs to the kernel on the device:
+    set to one context's size, it could drop below another's between that one's
+    own set and its launch.  Only raise_smem (launch.h), which keeps the largest,
+    sets it."""
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh", ".h")) and f != "launch.h":
+            assert "cudaFuncAttributeMaxDynamicSharedMemorySize" not in source(f), f

@@ -47,3 +47,37 @@ def test_gradients(C, batch, crop):  # noqa: F811
         for k in range(2):
             assert l2rel(gd[L][k], gref[L][k]) <= 5e-3 and maxrel(gd[L][k], gref[L][k]) <= 1e-2, (L, k)
     cl.close()
+
+
+def test_sides_from_two_threads(C):  # noqa: F811
+    """Closures of different sides (different shared-memory needs of the same
+    kernels) used at the same time from two threads give what each gives alone."""
+    import threading
+
+    closure, _ = C
+    cls = [closure.Closure(batch=0, crop=0, nfield=n, seed=5) for n in (16, 64)]
+    v = [torch.randn((3, n, n, n), dtype=torch.float64, device="cuda") for n in (16, 64)]
+    alone = [cl.infer_cells(x).clone() for cl, x in zip(cls, v)]
+    torch.cuda.synchronize()
+    bad = []
+
+    def use(i):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for _ in range(100):
+                    got = cls[i].infer_cells(v[i])
+                stream.synchronize()
+                if not torch.equal(got, alone[i]):
+                    bad.append(f"closure {i}: other values")
+        except Exception as e:  # noqa: BLE001
+            bad.append(str(e))
+
+    threads = [threading.Thread(target=use, args=(i,)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
+    for cl in cls:
+        cl.close()

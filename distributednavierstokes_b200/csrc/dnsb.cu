@@ -2361,15 +2361,21 @@ int dnsb_shell_clamp(dnsb_ctx *c, double *ux, double *uy, double *uz, const doub
     const Geo &g = c->g;
     const int KM = nb - 1;
     const int H = KM + 1, W = 2 * KM + 1;
-    const unsigned lines = (unsigned)(((long long)g.ny * g.nz + LS_LINES - 1) / LS_LINES);
-    CK(c, launch_pdl(k_ls_xsums, dim3(lines), dim3(128), 0, c->stream, g, cf(ux, uy, uz), KM, c->lsX,
-                     c->lsA));
-    CK(c, launch_pdl(k_ls_sums<8, 4>, dim3((3 * H * g.nz + 7) / 8), dim3(LS_STHREADS), 0, c->stream,
-                     3 * H * g.nz, g.ny, 1, (long long)g.ny, 1, c->lsA, KM, c->lsY, c->lsB));
+    const long lines = (long)g.ny * g.nz;
+    const bool few = (lines + 31) / 32 < 2L * c->nsm && g.nx >= LS_TILE / 8;
+    CK(c, launch_pdl(few ? k_ls_xsums<8> : k_ls_xsums<32>, dim3((unsigned)(few ? (lines + 7) / 8 : (lines + 31) / 32)),
+                     dim3(128), 0, c->stream, g, cf(ux, uy, uz), KM, c->lsX, c->lsA));
+    const int yrows = 3 * H * g.nz;
+    const bool fewrows = (yrows + 7) / 8 < c->nsm / 2 && g.ny >= 128;
+    CK(c, launch_pdl(fewrows ? k_ls_sums<1, 32> : k_ls_sums<8, 4>, dim3(fewrows ? yrows : (yrows + 7) / 8),
+                     dim3(LS_STHREADS), 0, c->stream, yrows, g.ny, 1, (long long)g.ny, 1, c->lsA, KM, c->lsY,
+                     c->lsB));
     CK(c, launch_pdl(k_ls_sums<1, 32>, dim3(3 * H * W), dim3(LS_STHREADS), 0, c->stream, 3 * H * W, g.nz, W,
                      (long long)g.nz * W, W, c->lsB, KM, c->lsZ, c->lsG));
     CK(c, launch_pdl(k_ls_modes, dim3(1), dim3(256), 0, c->stream, g, KM, c->lsG, E, er, f, nb));
-    CK(c, launch_pdl(k_ls_correct, dim3((g.ny + LS_CLINES - 1) / LS_CLINES, g.nz), dim3(256), 0,
+    const long cblocks = (long)((g.ny + LS_CLINES - 1) / LS_CLINES) * g.nz;
+    const unsigned xparts = (unsigned)std::max(1L, std::min(g.nx / 64L, 2L * c->nsm / cblocks));
+    CK(c, launch_pdl(k_ls_correct, dim3((g.ny + LS_CLINES - 1) / LS_CLINES, g.nz, xparts), dim3(256), 0,
                            c->stream, g, ff(ux, uy, uz), KM, c->lsG, c->lsX, c->lsY, c->lsZ));
     c->umax_for[0] = c->umax_for[1] = c->umax_for[2] = nullptr;
     return 0;

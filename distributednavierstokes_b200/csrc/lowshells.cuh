@@ -33,8 +33,7 @@ namespace dnsb {
 
 constexpr int LS_KX = 4;             // kx = 0..3
 constexpr int LS_KY = 7;             // ky, kz = -3..3
-constexpr int LS_LINES = 32;         // (y, z) lines per block of the x-sums
-constexpr int LS_XT = 32;            // points per staged tile of a line
+constexpr int LS_TILE = 1024;        // points per component of a block's tile of the x-sums
 constexpr int LS_CLINES = 16;        // lines (one plane) per block of the correction
 
 // the phases e^{+2 pi i r / n} = (cos, sin) for r = 0..n-1 of one direction,
@@ -59,16 +58,26 @@ __device__ __forceinline__ double2 ls_phase_tab(int m, int n, double sign, const
 }
 
 // A[((c * (KM+1) + kx) * nz + (K-1)) * ny + (J-1)] = sum_i u_c(i, J, K) e^{-2 pi i kx i / nx}
+// LINES lines per block, staged LS_TILE / LINES points at a time; a thread sums 32
+// points of a line's tile, the 32 / LINES threads of a line are added at the end.
+// A tile costs about 2 us at few blocks per SM, so few long lines want few tiles
+// each: 32 lines a block, and 8 where those are less than two blocks per SM and a
+// line fills the longer tile (512 x 16 x 16 34.0 -> 9.9 us, 512 x 64 x 64 35.4 ->
+// 18.3, 256 x 32 x 32 18.2 -> 6.1).
+template <int LINES>
 __global__ void __launch_bounds__(128) k_ls_xsums(Geo g, CFields3 u, int KM, const double2 *__restrict__ xph,
                                                   double2 *__restrict__ A, int dep) {
-  constexpr int ROWS = 3 * LS_LINES;
-  __shared__ double tile[ROWS][LS_XT + 1];
-  __shared__ double2 ph[LS_KX][LS_XT];
+  constexpr int ROWS = 3 * LINES, XT = LS_TILE / LINES, SEG = XT / 32;  // SEG warps side by side on a line
+  static_assert(4 % SEG == 0 && ROWS * SEG == 96, "four warps load, 96 threads sum");
+  __shared__ double tile[ROWS][XT + 1];
+  __shared__ double2 ph[LS_KX][XT];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int line0 = blockIdx.x * LS_LINES, nlines = g.ny * g.nz;
+  const int line0 = blockIdx.x * LINES, nlines = g.ny * g.nz;
+  const int l0 = warp / SEG, xs = 32 * (warp % SEG) + lane;    // loads: line l0, l0 + 4 / SEG, .., point xs
+  const int row = tid % ROWS, part = tid / ROWS;               // sums: points 32 part ..
   // the first cell of each staged line
-  __shared__ int first[LS_LINES];
-  if (tid < LS_LINES) {
+  __shared__ int first[LINES];
+  if (tid < LINES) {
     const int line = min(line0 + tid, nlines - 1);
     first[tid] = gidx(g, 1, line % g.ny + 1, line / g.ny + 1);
   }
@@ -77,43 +86,59 @@ __global__ void __launch_bounds__(128) k_ls_xsums(Geo g, CFields3 u, int KM, con
   __syncthreads();
   double a0 = 0.0;
   double2 acc[LS_KX] = {};
-  for (int x0 = 0; x0 < g.nx; x0 += LS_XT) {
-    const int x = x0 + lane;
+  for (int x0 = 0; x0 < g.nx; x0 += XT) {
+    const int x = x0 + xs;
     const bool in = x < g.nx;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const double *f = c == 0 ? u.x : c == 1 ? u.y : u.z;
-      double v[LS_LINES / 4];
+      double v[8];
 #pragma unroll
-      for (int r = 0; r < LS_LINES / 4; r++) v[r] = in ? f[first[warp + 4 * r] + x] : 0.0;
+      for (int r = 0; r < 8; r++) v[r] = in ? f[first[l0 + 4 / SEG * r] + x] : 0.0;
 #pragma unroll
-      for (int r = 0; r < LS_LINES / 4; r++) tile[c * LS_LINES + warp + 4 * r][lane] = v[r];
+      for (int r = 0; r < 8; r++) tile[c * LINES + l0 + 4 / SEG * r][xs] = v[r];
     }
-    if (warp == 0) {
+    if (warp < SEG) {
       const double2 e = in ? xph[x] : make_double2(1.0, 0.0);
       const double2 z1 = make_double2(e.x, -e.y), z2 = cmul(z1, z1);
-      ph[1][lane] = z1;
-      ph[2][lane] = z2;
-      ph[3][lane] = cmul(z2, z1);
+      ph[1][xs] = z1;
+      ph[2][xs] = z2;
+      ph[3][xs] = cmul(z2, z1);
     }
     __syncthreads();
-    if (tid < ROWS) {
+    if (tid < ROWS * SEG) {
+      const double *t = &tile[row][32 * part];
+      const double2(*e)[XT] = reinterpret_cast<const double2(*)[XT]>(&ph[0][32 * part]);
 #pragma unroll 8
-      for (int i = 0; i < LS_XT; i++) {
-        const double v = tile[tid][i];
+      for (int i = 0; i < 32; i++) {
+        const double v = t[i];
         a0 += v;
 #pragma unroll
         for (int kx = 1; kx < LS_KX; kx++) {
-          acc[kx].x = fma(v, ph[kx][i].x, acc[kx].x);
-          acc[kx].y = fma(v, ph[kx][i].y, acc[kx].y);
+          acc[kx].x = fma(v, e[kx][i].x, acc[kx].x);
+          acc[kx].y = fma(v, e[kx][i].y, acc[kx].y);
         }
       }
     }
     __syncthreads();
   }
   acc[0] = make_double2(a0, 0.0);
-  if (tid < ROWS && line0 + tid % LS_LINES < nlines) {
-    const int c = tid / LS_LINES, line = line0 + tid % LS_LINES;
+  if constexpr (SEG > 1) {  // the parts of a line, in order (the tile is free)
+    double2(*sums)[LS_KX][ROWS] = reinterpret_cast<double2(*)[LS_KX][ROWS]>(&ph[0][0]);
+    static_assert(sizeof(double2) * SEG * LS_KX * ROWS <= sizeof ph, "the parts' sums fit the phases");
+    if (part > 0 && part < SEG) {
+#pragma unroll
+      for (int kx = 0; kx < LS_KX; kx++) sums[part][kx][row] = acc[kx];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 1; q < SEG; q++)
+#pragma unroll
+      for (int kx = 0; kx < LS_KX; kx++)
+        if (part == 0) acc[kx] = cadd(acc[kx], sums[q][kx][row]);
+  }
+  if (part == 0 && line0 + row % LINES < nlines) {
+    const int c = row / LINES, line = line0 + row % LINES;
 #pragma unroll
     for (int kx = 0; kx < LS_KX; kx++)
       if (kx <= KM) A[(long long)(c * (KM + 1) + kx) * nlines + line] = acc[kx];
@@ -124,7 +149,9 @@ __global__ void __launch_bounds__(128) k_ls_xsums(Geo g, CFields3 u, int KM, con
 // base(r) = (r / inner) outer + r % inner: the y-sums (rows of A: inner 1)
 // and the z-sums (rows of B, k strided by W: inner W).  Thread (row, output
 // q < W, part of the row): 8 rows in quarters for the many y-rows, one row in
-// 32 parts for the at most 84 z-rows.
+// 32 parts for the at most 84 z-rows and for y-rows of 128 or more points too few
+// to fill half the GPU (clamp of 40 x 250 x 16 46.5 -> 28-34 us, 16 x 512 x 16
+// 44.5 -> 25.4, 64 x 256 x 64 64.8 -> 46.2).
 constexpr int LS_STHREADS = 8 * LS_KY * 4;
 template <int ROWS, int PARTS>
 __global__ void __launch_bounds__(LS_STHREADS)
@@ -209,7 +236,9 @@ __global__ void __launch_bounds__(256) k_ls_modes(Geo g, int KM, double2 *Gm, do
 
 // u_c(i, J, K) += Re sum_{kx, ky, kz} w(kx) G e^{+2 pi i (kx i/nx + ky j/ny + kz k/nz)},
 // then the periodic ghost images of the updated cells.  grid (groups of
-// LS_CLINES rows, nz)
+// LS_CLINES rows, nz, parts of x): few long lines are split along x, 64 points a
+// part at the least, into two blocks per SM (512 x 16 x 16 48.3 -> 9.4 us, 1024 x
+// 16 x 16 94.1 -> 9.9; at 48^3 parts of 24 points were no faster)
 __global__ void __launch_bounds__(256, 4) k_ls_correct(Geo g, Fields3 u, int KM, const double2 *Gm,
                                                     const double2 *__restrict__ xph,
                                                     const double2 *__restrict__ yph,
@@ -240,7 +269,7 @@ __global__ void __launch_bounds__(256, 4) k_ls_correct(Geo g, Fields3 u, int KM,
   }
   __syncthreads();
   double *fc[3] = {u.x, u.y, u.z};
-  for (int i = lane; i < g.nx; i += 32) {
+  for (int i = lane + 32 * blockIdx.z; i < g.nx; i += 32 * gridDim.z) {
     const double2 z1 = xph[i], z2 = cmul(z1, z1), z3 = cmul(z2, z1);
 #pragma unroll
     for (int q = 0; q < LS_CLINES / 8; q++) {

@@ -140,3 +140,39 @@ def test_random_field_and_clamp_bit_reproducible(D):
     f(b, s)
     for c in "xyz":
         assert torch.equal(a[c], b[c])
+
+
+@pytest.mark.parametrize("n", [
+    (512, 16, 16),    # 8 lines a block, every tile of 128 points full
+    (128, 9, 12),     # one tile; a last block of four lines
+    (144, 12, 10),    # a last tile of 16 points: three parts of it without any
+    (1024, 8, 8),
+    (120, 16, 16),    # shorter than that tile: 32 lines a block
+    (256, 96, 96),    # just below two blocks of 32 lines per SM
+    (256, 100, 100),  # just above
+    (40, 250, 16),    # y-sums in 32 parts of 8 (the last of 2)
+    (16, 128, 16),    # ... of 4
+])
+def test_clamp_of_long_boxes_matches_the_transform_path(D, n):
+    """The separable clamp on boxes of few long lines (its sums over lines in parts
+    of a tile, its correction in parts of a line) against shell energies and
+    rescaled shells by 3-D transforms.  Both form the same sums of at most 2.56e6
+    terms in another order, sqrt(eref / E) of them once: 1e-12 of the field."""
+    s = D.setup(n=n, visc=5e-3)
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    u = D.vectorfield(s)
+    for c in "xyz":
+        D.interior(u[c]).copy_(torch.randn((n[2], n[1], n[0]), generator=gen, device="cuda",
+                                           dtype=torch.float64))
+    D.exchange_halo(u, s)
+    ref = D.VectorField({c: u[c].clone() for c in "xyz"})
+    shells = (1, 2, 3)
+    eref = [0.3, 0.2, 0.1]
+    D.shellforcing(u, s, shells=shells, eref=eref)(u, s)
+    E = D.shell_energies(ref, s, shells)
+    for sh, e0, e in zip(shells, eref, E):
+        D.rescale_shell(ref, s, sh, math.sqrt(e0 / e))
+    for c in "xyz":
+        assert float((u[c] - ref[c]).abs().max()) <= 1e-12 * float(ref[c].abs().max()), c
+    assert np.abs(D.shell_energies(u, s, shells) / np.asarray(eref) - 1).max() <= 1e-12
+    s.close()

@@ -369,6 +369,32 @@ def test_momentum_march_planes(oracle_mod, D, cfg, planes, monkeypatch):
         assert rel(N(qd[c]), q[c]) <= 1e-11, c
 
 
+@pytest.mark.parametrize("n,bcy", [((96, 72, 80), "wall"),      # 5 planes a CTA
+                                   ((80, 80, 80), "periodic"),  # 6, the last column of 2
+                                   ((36, 9, 20), "periodic"),   # 1
+                                   ((160, 100, 90), "wall")])   # 8, the last column of 2
+def test_momentum_alone(D, n, bcy, monkeypatch):
+    """momentum! as a call of its own (planes per CTA by its own rule) against the
+    per-cell kernel (DNSB_MOMTILE=0): the same expressions, a multiply and an add
+    contracted or not, 1e-13 of the largest value."""
+    out = []
+    for tile in ("1", "0"):
+        monkeypatch.setenv("DNSB_MOMTILE", tile)
+        s = D.setup(n=n, bc=("periodic", bcy, "periodic"), visc=0.02)
+        gen = torch.Generator(device="cuda").manual_seed(2)
+        u, q = D.vectorfield(s), D.vectorfield(s)
+        for v, amp in ((u, 0.3), (q, 1.0)):
+            for c in "xyz":
+                v[c][s.active(c)] = amp * torch.randn(v[c][s.active(c)].shape, generator=gen, device="cuda",
+                                                      dtype=torch.float64)
+        D.exchange_halo(u, s)
+        D.momentum(q, u, -0.4, 1e-2, s)
+        out.append([D.interior(q[c]).clone() for c in "xyz"])
+        s.close()
+    for a, b in zip(*out):
+        assert float((a - b).abs().max()) <= 1e-13 * float(b.abs().max())
+
+
 @pytest.mark.parametrize("post,pairs", [("1", "0"), ("0", "0"), ("1", "1")])
 @pytest.mark.parametrize("nx", [64, 384])
 def test_rfftx_output_pass_in_registers(oracle_mod, D, nx, post, pairs, monkeypatch):

@@ -317,13 +317,15 @@ __device__ __forceinline__ float2 gelu2(float2 z) {
   const float2 h = mul2(both(0.5f), z);
   return fma2(h, tanh2(u), h);
 }
-// d/dz [0.5 z (1 + t)] = s + s (1 - t) z u'(z) with s = 0.5 (1 + t)
+// d/dz [0.5 z (1 + t)] = s + s (1 - t) z u'(z) with s = 0.5 (1 + t); s (1 - t) z
+// first: it is 0 where t is 1 or -1, and z u' alone passes the largest FP32 value
+// from |z| = 1.5e13 on (0 x infinity)
 __device__ __forceinline__ float2 gelu_grad2(float2 z) {
   const float2 z2 = mul2(z, z);
   const float2 t = tanh2(mul2(z, fma2(both(GELU_C * GELU_A), z2, both(GELU_C))));
-  const float2 zdu = mul2(z, fma2(both(3.f * GELU_C * GELU_A), z2, both(GELU_C)));
+  const float2 du = fma2(both(3.f * GELU_C * GELU_A), z2, both(GELU_C));
   const float2 s = fma2(both(0.5f), t, both(0.5f));
-  return fma2(mul2(s, fma2(both(-1.f), t, both(1.f))), zdu, s);
+  return fma2(mul2(mul2(s, fma2(both(-1.f), t, both(1.f))), z), du, s);
 }
 
 __device__ __forceinline__ uint32_t pack2(float2 v) {

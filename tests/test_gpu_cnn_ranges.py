@@ -81,3 +81,31 @@ def test_sides_from_two_threads(C):  # noqa: F811
     assert not bad, bad
     for cl in cls:
         cl.close()
+
+
+def test_gradients_of_large_preactivations(C):  # noqa: F811
+    """GELU's slope is 1 or 0 far from the origin, up to pre-activations whose
+    square is finite in FP32: the gradients of a network with biases of +-1e15 in
+    its first layer match the oracle's."""
+    closure, O = C
+    batch, crop = 2, 12
+    cl = closure.Closure(batch=batch, crop=crop, seed=3)
+    params = closure.unflatten(cl.get_params())
+    W0, b0 = params[0]
+    params[0] = (W0, np.where(np.arange(b0.size) % 2 == 0, 1e15, -1e15).astype(b0.dtype))
+    cl.set_params(closure.flatten(params))
+    params = closure.unflatten(cl.get_params())
+    P = crop + 8
+    rng = np.random.default_rng(1)
+    x = O.f32(rng.standard_normal((batch, 3, P, P, P)))
+    t = O.f32(rng.standard_normal((batch, 6, crop, crop, crop)))
+    loss, g = cl.batch_grads(torch.from_numpy(x.astype(np.float32)).cuda(),
+                             torch.from_numpy(t.astype(np.float32)).cuda())
+    lref, gref, _ = O.loss_and_grads(params, x, t)
+    assert math.isfinite(loss) and math.isclose(loss, lref, rel_tol=1e-2)
+    gd = closure.unflatten(g)
+    for L in range(4):
+        for k in range(2):
+            assert np.isfinite(gd[L][k]).all(), (L, k)
+            assert l2rel(gd[L][k], gref[L][k]) <= 1e-2, (L, k)
+    cl.close()

@@ -693,14 +693,14 @@ int launch_fftz4(dnsb_ctx *c, bool inv) {
     else LAUNCH(c, DNSB_KIND_FFTZ, CK(c, launch_pdl(k_fftz4<A, B, false>, grid, dim3(F4_THREADS), c->smem_z4, c->stream, g, c->S, c->L4z, c->twz))); \
     return 0;                                                                                      \
   }
-  FFT4_SPLITS(ZF4)
+  FFTZ4_SPLITS(ZF4)
 #undef ZF4
   return fail(c, DNSB_EUNSUP, "no four-step z kernel for %d x %d", c->z1, c->z2);
 }
 
 // shared-memory opt-in of the four-step kernels of one split
 template <int A, int B>
-int allow_fft4(dnsb_ctx *c) {
+int allow_rfftx4(dnsb_ctx *c) {
   int rc;
   constexpr size_t xs = XWarp<A, B>::smem;
   if ((rc = allow_smem(c, k_rfftx4<A, B, RIN_DIVERGENCE>, xs)) ||
@@ -709,18 +709,25 @@ int allow_fft4(dnsb_ctx *c) {
       (rc = allow_smem(c, k_rfftx4<A, B, RIN_PRODUCT>, xs)) ||
       (rc = allow_smem(c, k_irfftx4<A, B, ROUT_INTERIOR>, xs)) ||
       (rc = allow_smem(c, k_irfftx4<A, B, ROUT_IMAGES>, xs)) ||
-      (rc = allow_smem(c, k_irfftx4<A, B, ROUT_REAL>, xs)) ||
-      (rc = allow_smem(c, k_fftz4<A, B, false>, c->smem_z4)) ||
-      (rc = allow_smem(c, k_fftz4<A, B, true>, c->smem_z4)))
+      (rc = allow_smem(c, k_irfftx4<A, B, ROUT_REAL>, xs)))
     return rc;
   return 0;
 }
 
-int allow_fft4_split(dnsb_ctx *c, int a, int b) {
-#define AF4(A, B) \
-  if (a == A && b == B) return allow_fft4<A, B>(c);
-  FFT4_SPLITS(AF4)
-#undef AF4
+// the kernels of the context's compile-time splits
+int allow_fft4(dnsb_ctx *c) {
+  int rc;
+#define AX4(A, B) \
+  if (c->x1 == A && c->x2 == B && (rc = allow_rfftx4<A, B>(c))) return rc;
+  FFT4_SPLITS(AX4)
+#undef AX4
+#define AZ4(A, B)                                                          \
+  if (c->z1 == A && c->z2 == B &&                                          \
+      ((rc = allow_smem(c, k_fftz4<A, B, false>, c->smem_z4)) ||           \
+       (rc = allow_smem(c, k_fftz4<A, B, true>, c->smem_z4))))             \
+    return rc;
+  FFTZ4_SPLITS(AZ4)
+#undef AZ4
   return 0;
 }
 
@@ -758,7 +765,7 @@ int launch_fftz(dnsb_ctx *c, bool inv) {
   // threads all hold a transform; 256^3 53.9 -> 44.0 us, 384 x 256 x 384 128 ->
   // 113); shorter lines are bound by latency and keep the constant indices
   // (64^3: 2.8 us against 3.4)
-  if (c->z1 && !c->use_tma && (g.nz < 128 || !c->az.tier)) return launch_fftz4(c, inv);
+  if (c->z1 && !c->use_tma && g.nz < 128) return launch_fftz4(c, inv);
   if (c->az.tier && !c->use_tma) {
     LAUNCH(c, inv ? DNSB_KIND_IFFTZ : DNSB_KIND_FFTZ,
            CK(c, any_fftz(g, c->az, c->nkx_active ? c->nkx_active : g.nkx, c->Lz_set, inv, c->S, c->twz, c->stream)));
@@ -1211,7 +1218,6 @@ int alloc_shells(dnsb_ctx *c) {
 
 // S = the 3-D transform of the interior of component u
 int spectrum_of(dnsb_ctx *c, const double *u) {
-  const Geo &g = c->g;
   int rc;
   if ((rc = launch_rfftx(c, RIN_FIELD, u, nullptr, nullptr))) return rc;
   if ((rc = launch_fftz(c, false))) return rc;
@@ -1586,9 +1592,7 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
     fail(c, DNSB_ECUDA, "shared-memory opt-in of the transform kernels failed");
     return bail(DNSB_ECUDA);
   }
-  if ((c->x1 && (rc = allow_fft4_split(c, c->x1, c->x2))) ||
-      (c->z1 && (rc = allow_fft4_split(c, c->z1, c->z2))))
-    return bail(rc);
+  if ((rc = allow_fft4(c))) return bail(rc);
   if ((rc = allow_smem(c, k_rfftx<RIN_DIVERGENCE>, c->smem_rx)) ||
       (rc = allow_smem(c, k_rfftx<RIN_REAL>, c->smem_rx)) ||
       (rc = allow_smem(c, k_rfftx<RIN_FIELD>, c->smem_rx)) ||
@@ -2864,7 +2868,6 @@ int sp_to_phys(dnsb_spectral *p, const double2 *uhc, double *v) {
 // the full forward transform of a real n^3 array into S (unnormalised)
 int sp_from_phys(dnsb_spectral *p, const double *r) {
   dnsb_ctx *c = p->c;
-  const Geo &g = c->g;
   SPRC(p, launch_rfftx(c, RIN_REAL, r, nullptr, nullptr));
   SPRC(p, launch_fftz(c, false));
   SPRC(p, launch_yfourier(c, YF_FORWARD));
@@ -2875,7 +2878,6 @@ int sp_from_phys(dnsb_spectral *p, const double *r) {
 // x-transform's loads where the four-step kernel applies
 int sp_from_product(dnsb_spectral *p, const double *va, const double *vb) {
   dnsb_ctx *c = p->c;
-  const Geo &g = c->g;
   if (!c->x1 && !c->ax.tier) {
     k_sp_product<<<RED_BLOCKS, 256, 0, c->stream>>>(sp_n3(p), va, vb, p->r);
     SPKL(p);
@@ -2989,10 +2991,11 @@ int dnsb_spectral_create(int n, int kcut, double l, double visc, int device, voi
   p->s.nc = (long long)(kcut + 1) * p->s.m * p->s.m;
   p->s.kfac = 2 * M_PI / l;
   const size_t n3 = (size_t)n * n * n;
+  const bool truncated = c->ax.tier && c->az.tier && n >= 6;  // on the truncated transforms (SpPlan)
   if ((rc = spalloc(p, &p->v[0], n3)) || (rc = spalloc(p, &p->v[1], n3)) ||
       (rc = spalloc(p, &p->v[2], n3)) || (rc = spalloc(p, &p->r, n3)) ||
       (rc = spalloc(p, &p->ustart, 3 * (size_t)p->s.nc)) ||
-      (rc = spalloc(p, &p->du, 3 * (size_t)p->s.nc)) ||
+      (!truncated && (rc = spalloc(p, &p->du, 3 * (size_t)p->s.nc))) ||
       (rc = spalloc(p, &p->partial, (size_t)RED_BLOCKS + 1)) || (rc = spalloc(p, &p->umax, 2)) ||
       (rc = spalloc(p, &p->shellbuf, 3 * (size_t)(p->nshell = (int)std::floor(std::sqrt(3.0) * kcut) + 1))) ||
       (rc = spalloc(p, &p->shellpart, (size_t)RED_BLOCKS * SP_SHELLS))) {
@@ -3003,7 +3006,7 @@ int dnsb_spectral_create(int n, int kcut, double l, double visc, int device, voi
   // The truncated transforms' six buffers of (kcut + 1) n^2 values are the
   // context's spectrum and the fields that the solver does not use otherwise
   // (n^3 real values hold them from n = 6 on: (n/3 + 1) n^2 complex).
-  if (c->ax.tier && c->az.tier && n >= 6) {
+  if (truncated) {
     SpPlan &a = p->any;
     a.s = SpCube{n, kcut, 2 * kcut + 1, p->s.nc, p->s.kfac};
     a.x = c->ax;

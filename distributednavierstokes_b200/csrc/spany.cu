@@ -57,7 +57,7 @@ cudaError_t sp_any_allow(int device, const SpPlan &p) {
     if (e == cudaSuccess) e = raise_smem(device, k_sp_xinv4<A, B_>, XWarp<A, B_>::smem);           \
     if (e == cudaSuccess) e = raise_smem(device, k_sp_xprod4<A, B_>, sp_xprod4_smem<A, B_>());     \
   }
-  FFT4_SPLITS(ALLOW4)
+  SP4_SPLITS(ALLOW4)
 #undef ALLOW4
   by_tier(p.x.tier, [&](auto t) {
     constexpr int T = decltype(t)::value;
@@ -93,7 +93,7 @@ cudaError_t sp_any_phys(const SpPlan &p, const double2 *uh, double *const v[3], 
     return launch_pdl(k_sp_xinv4<A, B_>, grid, dim3(128), XWarp<A, B_>::smem, st, s, B,            \
                       SpFields{{v[0], v[1], v[2]}}, p.twM, p.twN);                                 \
   }
-  FFT4_SPLITS(XINV4)
+  SP4_SPLITS(XINV4)
 #undef XINV4
   return by_tier(p.x.tier, [&](auto t) {
     constexpr int T = decltype(t)::value;
@@ -121,7 +121,7 @@ cudaError_t sp_any_products(const SpPlan &p, double *const v[3], unsigned long l
     e = launch_pdl(k_sp_xprod4<A, B_>, grid, dim3(128), sp_xprod4_smem<A, B_>(), st, s,            \
                    SpFields{{v[0], v[1], v[2]}}, F, vmax, p.twM, p.twN);                           \
   }
-  FFT4_SPLITS(XPROD4)
+  SP4_SPLITS(XPROD4)
 #undef XPROD4
   if (!by_warps) e = by_tier(p.x.tier, [&](auto t) {
     constexpr int T = decltype(t)::value;

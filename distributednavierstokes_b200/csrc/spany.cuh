@@ -194,7 +194,10 @@ __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
   }
 }
 
-// The same by warps, for the splits with a compile-time kernel (xwarp.cuh).
+// The same by warps, for the sides with a compile-time split of n/2 (xwarp.cuh);
+// n = 512 and 768 have no run-time split along y and z, so that neither takes these
+// transforms.
+#define SP4_SPLITS(X) X(16, 12) X(16, 8) X(8, 12) X(8, 8) X(8, 6) X(8, 4)
 template <int N1, int N2>
 __global__ void __launch_bounds__(128, (XWarp<N1, N2>::BLOCKS))
     k_sp_xinv4(SpCube s, SpBufs B, SpFields out, const double2 *__restrict__ twM,

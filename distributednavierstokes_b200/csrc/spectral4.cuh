@@ -14,6 +14,10 @@ namespace dnsb {
 
 constexpr int F4_THREADS = 256;
 
+// the splits of nz that k_fftz4 is compiled for: those below 128 (from there on the
+// run-time split is the faster, launch_fftz)
+#define FFTZ4_SPLITS(X) X(8, 12) X(8, 8) X(8, 6) X(8, 4)
+
 // Complex FFT along z of L contiguous lines of S (n = N1*N2 = nz); INV
 // scales by 1/nz.  Shared memory: transpose buffer + n twiddles.
 template <int N1, int N2, bool INV>

@@ -186,7 +186,7 @@ __device__ __forceinline__ void xw_ordered(double2 *buf, const double2 *tw, int 
   __syncwarp();
 }
 
-// the splits with a compile-time kernel (nx/2 = N1 N2)
+// the splits of nx/2 = N1 N2 with a compile-time x-kernel
 #define FFT4_SPLITS(X) X(16, 24) X(16, 16) X(16, 12) X(16, 8) X(8, 12) X(8, 8) X(8, 6) X(8, 4)
 
 }  // namespace dnsb

@@ -91,3 +91,18 @@ def test_a_choice_of_another_build_is_timed_again(monkeypatch, tmp_path):
         json.dump(data, f)
     autotune.tune_sizes([32], cache=cache, device="cpu")
     assert calls == [32, 32, 32]
+def test_the_z_field_is_the_one_that_the_kernel_reads():
+    import os
+    import re
+
+    csrc = os.path.join(os.path.dirname(autotune.__file__), "csrc")
+    with open(os.path.join(csrc, "spectral4.cuh")) as f:
+        splits = re.search(r"#define FFTZ4_SPLITS\(X\) (.*)", f.read()).group(1)
+    assert sorted(int(a) * int(b) for a, b in re.findall(r"X\((\d+), (\d+)\)", splits)) == \
+        sorted(autotune.Z4_SIDES)
+    for n in (32, 48, 64, 96):
+        assert "lines_z4" in autotune.candidates(n) and "lines_z" not in autotune.candidates(n)
+    for n in (40, 108, 128, 256):
+        assert "lines_z" in autotune.candidates(n) and "lines_z4" not in autotune.candidates(n)
+
+

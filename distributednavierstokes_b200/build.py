@@ -25,9 +25,9 @@ HEADERS = {
     "dnsb.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "spectral.cuh", "spectral4.cuh", "stencil.cuh",
                 "tma.cuh", "ysolve.cuh", "gradmom.cuh", "zyz.cuh", "spsolver.cuh", "lowshells.cuh",
                 "cnn_host.h", "fftany.h", "launch.h", "pdl.cuh", "spany.h", "xwarp.cuh"],
-    "fftany.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "fftany.cuh", "fftany.h", "launch.h", "pdl.cuh"],
+    "fftany.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "fftany.cuh", "fftany.h", "launch.h", "pdl.cuh", "tiers.h"],
     "spany.cu": ["common.cuh", "fft.cuh", "fft4.cuh", "fftany.cuh", "fftany.h", "launch.h", "pdl.cuh",
-                 "spany.cuh", "spany.h", "xwarp.cuh"],
+                 "spany.cuh", "spany.h", "tiers.h", "xwarp.cuh"],
     "cnn.cu": ["cnn.cuh", "cnn_host.h", "launch.h", "pdl.cuh"],
 }
 

@@ -5,34 +5,18 @@
 
 #include "fftany.cuh"
 #include "launch.h"
+#include "tiers.h"
 
 namespace dnsb {
 namespace {
-
-constexpr size_t kSmemPerBlock = 110 * 1024;  // two blocks per SM at the least
-
-template <int T>
-using tier_c = std::integral_constant<int, T>;
-
-// f(integral_constant<tier>)
-template <class F>
-cudaError_t by_tier(int tier, F f) {
-  switch (tier) {
-    case 10: return f(tier_c<10>());
-    case 16: return f(tier_c<16>());
-    case 25: return f(tier_c<25>());
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-int threads_for(int items) { return std::min(FA_THREADS, std::max(32, (items + 31) / 32 * 32)); }
 
 // Lines per block: enough for FA_THREADS register transforms, fewer where
 // the grid would leave SMs without a block (small boxes: latency, not
 // throughput, is what their transforms cost), and within shared memory.
 int lines_for(const AnySplit &sp, int asked, long long lines, int least, size_t bytes_per_line, size_t fixed) {
   int L = asked > 0 ? asked : std::max(least, FA_THREADS / std::max(sp.n1, sp.n2));
-  while (asked <= 0 && L > least && (lines + L - 1) / L < 2 * 148 && L / 2 * std::max(sp.n1, sp.n2) >= 64)
+  const long long few = 2LL * sm_count();
+  while (asked <= 0 && L > least && (lines + L - 1) / L < few && L / 2 * std::max(sp.n1, sp.n2) >= 64)
     L = std::max(least, L / 2);
   while (L > 1 && fixed + L * bytes_per_line > kSmemPerBlock) L--;
   return L;

@@ -51,6 +51,22 @@ cudaError_t launch_as(bool dependent, void (*kernel)(P...), dim3 grid, dim3 bloc
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// SMs of the current device (148 where it cannot be told)
+inline int sm_count() {
+  static std::mutex mu;
+  static std::map<int, int> known;
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    return 148;
+  }
+  return known[dev] = n;
+}
+
 // Resident blocks of a kernel on the whole device (cached per device, kernel
 // and launch shape).
 inline long resident_blocks(const void *kernel, int threads, size_t smem) {
@@ -61,13 +77,12 @@ inline long resident_blocks(const void *kernel, int threads, size_t smem) {
   std::lock_guard<std::mutex> lock(mu);
   auto it = known.find({dev, kernel, threads, smem});
   if (it != known.end()) return it->second;
-  int per = 0, nsm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess ||
-      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+  int per = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 0;  // not known: an ordinary launch
   }
-  return known[{dev, kernel, threads, smem}] = (long)per * nsm;
+  return known[{dev, kernel, threads, smem}] = (long)per * sm_count();
 }
 
 // Launch of a kernel whose last argument says whether it is a programmatic

@@ -5,26 +5,10 @@
 
 #include "launch.h"
 #include "spany.cuh"
+#include "tiers.h"
 
 namespace dnsb {
 namespace {
-
-constexpr size_t kSmemPerBlock = 110 * 1024;
-
-template <int T>
-using tier_c = std::integral_constant<int, T>;
-
-template <class F>
-cudaError_t by_tier(int tier, F f) {
-  switch (tier) {
-    case 10: return f(tier_c<10>());
-    case 16: return f(tier_c<16>());
-    case 25: return f(tier_c<25>());
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-int threads_for(int items) { return std::min(FA_THREADS, std::max(32, (items + 31) / 32 * 32)); }
 
 // lines per block: FA_THREADS register transforms, within shared memory, at
 // most `most`

@@ -124,6 +124,8 @@ struct Partials {
 // Work is numbered over quads of the partials' columns (dy, co), rows (dx, ci)
 // fastest, so that a thread reads 16 bytes of each split and a warp 512; 8 threads share a quad's splits (each
 // adds every 8th, the sums are added in order), seven loads in flight at once.
+// An ordinary launch, as k_tail, k_crops and k_batch_in behind it are, and without a
+// trigger: k_conv loads the weights ahead of its wait (test_dependent_launches.py).
 // One launch at the step's end: as four reductions between the backward kernels
 // (5.2 us each, ordinary launches that kept the next convolution from starting
 // early) and an Adam launch (5.9 us, two double pow per thread) they were 27 us
@@ -312,7 +314,7 @@ __global__ void k_batch_in(const float *x, const float *t, int B, int crop, int 
 __global__ void k_infer_in(const double *v, const double *ux, const double *uy, const double *uz,
                            int n, int P, const float *in_scale, uint4 *x0, int dep) {
   dnsb::pdl_wait(dep);
-  dnsb::pdl_trigger(dep);  // past the wait: the convolution reads the weights before its own
+  dnsb::pdl_trigger(dep);  // past the wait, as the convolution reads the weights ahead of its own
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
   if (x >= P) return;
   const long i = ((long)z * P + y) * P + x;

@@ -486,7 +486,8 @@ __global__ void __launch_bounds__(CONV_THREADS, 1)
   // The weights, by the lane that set the barriers.  They are written by an
   // ordinary launch (k_update), and the kernel that follows it in the chain is
   // an ordinary launch too or lets its dependents start only past its own wait
-  // (k_infer_in), so this kernel starts with them complete and visible
+  // (k_infer_in), so this kernel starts with them complete and visible.  Every
+  // kernel between them is held to that by tests/test_dependent_launches.py
   if (threadIdx.x == 0) {
     mb_expect(wbar, a.w_bytes);
     bulk_load(wsm, a.wpack, a.w_bytes, wbar);

@@ -108,3 +108,25 @@ def test_shared_memory_limits_are_only_raised():
     for f in sorted(os.listdir(CSRC)):
         if f.endswith((".cu", ".cuh", ".h")) and f != "launch.h":
             assert "cudaFuncAttributeMaxDynamicSharedMemorySize" not in source(f), f
+
+
+def test_weights_ahead_of_the_wait():
+    """k_conv copies its weights before it waits.  They are complete then as long as
+    what runs between k_update, which writes them, and a convolution are ordinary
+    launches without a trigger, or let their dependents start past their own wait."""
+    host, device = source("cnn.cu"), source("cnn.cuh")
+    bodies = {name: body for text in (host, device) for name, _, body in kernels(text)}
+    conv = bodies["k_conv"]
+    assert conv.index("bulk_load(wsm, a.wpack") < conv.index("griddepcontrol.wait")
+    # nothing else that another kernel writes is touched before it
+    ahead = conv[:conv.index("griddepcontrol.wait")]
+    assert not re.search(r"a\.(bias|zin|target|out|zout|infer_out|oscale|loss_part)\b|tma4\(", ahead)
+    ordinary = {"k_update", "k_tail", "k_crops", "k_batch_in"}
+    for name in ordinary:
+        assert re.search(rf"\b{name}<<<", host), name
+        assert not re.search(rf"launch_(as|pdl)\([^;]*\b{name}\b", host), name
+        assert "pdl_trigger(" not in bodies[name] and "launch_dependents" not in bodies[name], name
+    body = bodies["k_infer_in"]
+    assert body.index("pdl_wait(") < body.index("pdl_trigger(")
+    # every kernel of the closure is one of these
+    assert set(bodies) == ordinary | {"k_infer_in", "k_conv", "k_wgrad"}

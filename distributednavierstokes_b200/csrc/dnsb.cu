@@ -166,6 +166,7 @@ struct dnsb_ctx {
   int zyz_mode = 1;                    // 1: k_zyz (32-row chunks), 2: k_zyz2 (16-row chunks)
   int nkx_active = 0;                  // z-FFTs on kx < nkx_active only (0: all; spectral solver)
   int x1 = 0, x2 = 0, z1 = 0, z2 = 0;  // compile-time four-step splits of nx/2 and nz (0: none)
+  int xwarp = -1;  // x-transforms by warps: 0 never, 1 always, -1 by their rule (by_warps)
   AnySplit ax, ay_, az;  // run-time splits of nx/2, ny and nz (tier 0: none, the Stockham kernels)
   int Lx_set = 0, Lz_set = 0, Ly_set = 0;  // lines per block asked for (0: the launch rules)
   int L4z = 8;                         // lines per CTA of the z-FFT
@@ -734,8 +735,10 @@ int allow_fft4(dnsb_ctx *c) {
 // The x-transforms of one warp per 32 / max(N1, N2) lines where they give two
 // blocks per SM; fewer lines are bound by latency, and the kernels that spread
 // them over more threads are the faster (64^3 step 108 against 115 us).
+// DNSB_XWARP takes either everywhere.
 bool by_warps(const dnsb_ctx *c) {
   if (!c->x1 || !c->ax.tier) return c->x1 != 0;
+  if (c->xwarp >= 0) return c->xwarp != 0;
   const int lines = 4 * (32 / std::max(c->x1, c->x2));
   return (long)c->g.ny * ((c->g.nz + lines - 1) / lines) >= 2L * c->nsm;
 }
@@ -1553,6 +1556,7 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
   // periodic y the run-time splits
   if (envint("DNSB_FFT4", 1) != 0) {
     int a = 0, b = 0;
+    c->xwarp = envint("DNSB_XWARP", -1);
     c->ax = any_split(M);
     c->az = any_split(nz);
     if (!g.wall) c->ay_ = any_split(ny);

@@ -395,17 +395,14 @@ def test_momentum_alone(D, n, bcy, monkeypatch):
         assert float((a - b).abs().max()) <= 1e-13 * float(b.abs().max())
 
 
-@pytest.mark.parametrize("post,pairs", [("1", "0"), ("0", "0"), ("1", "1")])
+@pytest.mark.parametrize("warps", ["1", "0"])
 @pytest.mark.parametrize("nx", [64, 384])
-def test_rfftx_output_pass_in_registers(oracle_mod, D, nx, post, pairs, monkeypatch):
-    """The divergence x-FFT with its output pass in registers (the default)
-    and with the separate shared-memory pass (DNSB_RXPOST=0), and the
-    inverse x-FFT with its pair pre-processing inside the first FFT pass
-    (DNSB_IXPAIRS=1), at the splits 8 x 4 and 16 x 12; nz = 12 leaves a
-    short last group of lines: Poisson solve, projection and one step agree
-    with the oracle."""
-    monkeypatch.setenv("DNSB_RXPOST", post)
-    monkeypatch.setenv("DNSB_IXPAIRS", pairs)
+def test_x_transforms_by_warps(oracle_mod, D, nx, warps, monkeypatch):
+    """The real x-transforms by warps (DNSB_XWARP=1; a box of this size takes the
+    run-time-split kernels by the rule, and with 0), at the splits 8 x 4 and 16 x
+    12; nz = 12 leaves a short last group of lines: Poisson solve, projection and
+    one step agree with the oracle."""
+    monkeypatch.setenv("DNSB_XWARP", warps)
     kw = dict(n=(nx, 8, 12), lims=((0, 4 * math.pi), (-1, 1), (0, 4 * math.pi / 3)),
               bc=("periodic", "wall", "periodic"), stretch=R.tanhstretch(1.5),
               visc=1 / 395, bodyforce=(1.0, 0.0, 0.0), ydiffusion="implicit")

@@ -47,3 +47,10 @@ def test_matches_general_path(n, kcut, monkeypatch):
         assert err <= 1e-13, (name, err)
     for x, y in zip(va, vb):
         assert abs(x - y) <= 1e-13 * y
+
+
+@pytest.mark.parametrize("n,kcut", [(192, None), (256, None), (256, 80), (384, 40)])
+def test_matches_general_path_at_production_sizes(n, kcut, monkeypatch):
+    """The x-kernels by warps at the splits 16 x 8 and 16 x 12 (and 8 x 12)."""
+    test_matches_general_path(n, kcut, monkeypatch)
+    torch.cuda.empty_cache()

@@ -50,7 +50,9 @@ class Bar:
         return ok
 
 
-def simulate(ntiles, Do, z0, sub, nslot, seed, groups=4, nacc=4):
+def simulate(ntiles, Do, z0, sub, nslot, seed, groups=4, nacc=4, before=0, after=0):
+    """`before` / `after`: sub-tiles of the first / last tile that belong to the CTAs
+    before and after this one (the ranges are cut at sub-tiles)."""
     rnd = random.Random(seed)
     tiles = []
     for t in range(z0, z0 + ntiles):
@@ -62,7 +64,11 @@ def simulate(ntiles, Do, z0, sub, nslot, seed, groups=4, nacc=4):
     tempty = [Bar(4) for _ in range(nacc)]
     slot_plane = [None] * nslot
     mmas, commits, landing = [], [], []
-    nsubs = ntiles * sub
+    count = [sub] * ntiles
+    count[0] -= before
+    count[-1] -= after
+    assert min(count) > 0
+    nsubs = sum(count)
 
     def producer():
         g = sl = ph = 0
@@ -84,7 +90,7 @@ def simulate(ntiles, Do, z0, sub, nslot, seed, groups=4, nacc=4):
         sz, pg = [0, 0, 0], [0, 0, 0]
         i = 0
         last_a = last_i = -1
-        for fresh, last in tiles:
+        for (fresh, last), n in zip(tiles, count):
             for _ in (range(3) if fresh else range(1)):
                 while not full[gs].test(gph, gid // nslot):
                     yield
@@ -93,7 +99,7 @@ def simulate(ntiles, Do, z0, sub, nslot, seed, groups=4, nacc=4):
                 gs += 1
                 if gs == nslot:
                     gs, gph = 0, gph ^ 1
-            for sb in range(sub):
+            for sb in range(n):
                 ii = i + sb
                 if ii % 2 != r:
                     continue
@@ -110,7 +116,7 @@ def simulate(ntiles, Do, z0, sub, nslot, seed, groups=4, nacc=4):
             if last:
                 commits.append((r, len(mmas), empty[sz[1]]))
                 commits.append((r, len(mmas), empty[sz[2]]))
-            i += sub
+            i += n
             yield
         if last_a >= 0:
             while not tfull[last_a].test((last_i // nacc) & 1, last_i // nacc):
@@ -165,6 +171,28 @@ def test_conv_protocol(sub, nslot):
     for ntiles, Do, z0 in ((10, 5, 0), (7, 9, 2), (4, 1, 0), (8, 6, 3), (1, 4, 2)):
         for seed in range(6):
             simulate(ntiles, Do, z0, sub, nslot, seed)
+
+
+@pytest.mark.parametrize("sub", [2, 3, 4])
+@pytest.mark.parametrize("nslot", [4, 6, 7])
+def test_ranges_cut_inside_tiles(sub, nslot):
+    for ntiles, Do, z0 in ((10, 5, 0), (7, 9, 2), (4, 1, 0), (2, 6, 5)):
+        for before in range(sub):
+            for seed in range(3):
+                simulate(ntiles, Do, z0, sub, nslot, seed, before=before, after=(before + seed) % sub)
+
+
+def test_the_counts_are_the_kernel_s():
+    import os
+    import re
+
+    with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                           "distributednavierstokes_b200", "csrc", "cnn.cuh")) as f:
+        src = f.read()
+    kernel = src[src.index("k_conv(const __grid_constant__"):src.index("k_wgrad(const __grid_constant__")]
+    assert "constexpr int CONV_GROUPS = 4;" in src and "constexpr int NACC = 4;" in kernel
+    init = dict(re.findall(r"mb_init\(&(\w+)\[i\], (\d+)\)", kernel))
+    assert init == {"full": "1", "empty": "2", "tfull": "1", "tempty": "4"}
 
 
 def test_fewer_groups_than_accumulators_alias():

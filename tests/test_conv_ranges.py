@@ -1,32 +1,59 @@
-"""The sub-tile ranges of the closure convolution (SubWalk in
-distributednavierstokes_b200/csrc/cnn.cuh), mirrored on the host: the CTAs'
+"""The sub-tile ranges of the closure convolution: SubWalk as it stands in
+distributednavierstokes_b200/csrc/cnn.cuh, compiled for the host.  The CTAs'
 ranges cover every (sample, plane, sub-tile) once, differ by at most one
 sub-tile, and say truthfully where a tile's planes have to be loaded (`fresh`)
 and where they are used for the last time (`last`).
 """
+import os
+import re
+import shutil
+import subprocess
+
 import pytest
 
+SOURCE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                      "distributednavierstokes_b200", "csrc", "cnn.cuh")
+PROGRAM = """
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+using std::min;
+#define __device__
+#define __forceinline__ inline
+struct ConvArgs { int Do, spp, sub, tpp; };
+%s
+int main(int, char **v) {
+  ConvArgs a;
+  a.Do = atoi(v[1]);
+  a.spp = atoi(v[2]);
+  a.sub = atoi(v[3]);
+  a.tpp = (a.spp + a.sub - 1) / a.sub;
+  SubWalk w;
+  w.start(a, atoi(v[4]), atoi(v[5]));
+  while (w.tile(a)) printf("%%d %%d %%d %%d %%d %%d %%d\\n", w.b, w.j, w.z, w.lo, w.hi, w.fresh, w.last);
+}
+"""
 
-def walk(B, Do, spp, sub, s0, s1):
-    tpp = -(-spp // sub)
-    b, r = divmod(s0, spp * Do)
-    j, r = divmod(r, sub * Do)
-    n = min(sub, spp - j * sub)
-    z, lo = divmod(r, n)
-    z, left, first = z - 1, s1 - s0, True
-    while left > 0:
-        z += 1
-        if z == Do:
-            z, j = 0, j + 1
-            if j == tpp:
-                j, b = 0, b + 1
-            n = min(sub, spp - j * sub)
-        if not first:
-            lo = 0
-        hi = min(n, lo + left)
-        left -= hi - lo
-        yield b, j, z, lo, hi, first or z == 0, left == 0 or z == Do - 1
-        first = False
+
+@pytest.fixture(scope="module")
+def walk(tmp_path_factory):
+    cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else shutil.which("g++")
+    if not cxx:
+        pytest.skip("no host compiler")
+    with open(SOURCE) as f:
+        struct = re.search(r"^struct SubWalk \{.*?^\};", f.read(), re.S | re.M).group(0)
+    d = tmp_path_factory.mktemp("subwalk")
+    (d / "w.cpp").write_text(PROGRAM % struct)
+    subprocess.run([cxx, "-std=c++17", "-o", str(d / "w"), str(d / "w.cpp")], check=True)
+
+    def run(Do, spp, sub, s0, s1):
+        out = subprocess.run([str(d / "w")] + [str(v) for v in (Do, spp, sub, s0, s1)], check=True,
+                             capture_output=True, text=True).stdout
+        for line in out.splitlines():
+            b, j, z, lo, hi, fresh, last = (int(v) for v in line.split())
+            yield b, j, z, lo, hi, bool(fresh), bool(last)
+
+    return run
 
 
 @pytest.mark.parametrize("B,Do,spp,sub,grid", [
@@ -37,7 +64,7 @@ def walk(B, Do, spp, sub, s0, s1):
     (1, 3, 1, 4, 3),
     (3, 1, 5, 2, 7),       # one plane: every tile loads afresh
 ])
-def test_ranges(B, Do, spp, sub, grid):
+def test_ranges(walk, B, Do, spp, sub, grid):
     nsub = B * Do * spp
     grid = min(grid, nsub)
     seen = []
@@ -46,7 +73,7 @@ def test_ranges(B, Do, spp, sub, grid):
         assert s1 - s0 in (nsub // grid, nsub // grid + 1)
         ring = []                      # planes loaded, in order
         held = 0
-        for b, j, z, lo, hi, fresh, last in walk(B, Do, spp, sub, s0, s1):
+        for b, j, z, lo, hi, fresh, last in walk(Do, spp, sub, s0, s1):
             assert lo < hi
             ring = ([(b, j, z), (b, j, z + 1)] if fresh else ring) + [(b, j, z + 2)]
             held += 3 if fresh else 1

@@ -1,14 +1,42 @@
 """Barrier protocol of the weight-gradient kernel (cnn.cuh, k_wgrad), simulated
-on the CPU: the copying lane, the three MMA-issuing warps (one per dz), two of the
-warps that sum g, copies that land late and in any order, MMAs that finish late (each warp's in order, with
+on the CPU: the copying lane, the MMA-issuing warps (one per dz), the warps that sum
+g, copies that land late and in any order, MMAs that finish late (each warp's in order, with
 their commits), run in random interleavings.  No run may deadlock, overwrite a slot that an
-unfinished MMA reads, or let an MMA read a plane other than its own.
+unfinished MMA reads, or let an MMA read a plane other than its own.  The slots and the
+arrivals that a phase takes are read from the kernel's source.
 """
+import os
 import random
+import re
 
 import pytest
 
-PLANES, GRADS = 4, 3
+with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                       "distributednavierstokes_b200", "csrc", "cnn.cuh")) as f:
+    SOURCE = f.read()
+KERNEL = SOURCE[SOURCE.index("k_wgrad(const __grid_constant__"):]
+
+
+def constant(name):
+    return int(re.search(rf"constexpr int {name} = (\d+);", SOURCE).group(1))
+
+
+def arrivals(bar):
+    """The arrivals that complete a phase of a barrier: mb_init(&bar[i], a [+ b])."""
+    return [int(v) for v in re.search(rf"mb_init\(&{bar}\[i\], (\d+(?: \+ \d+)?)\)", KERNEL).group(1).split(" + ")]
+
+
+PLANES, GRADS = constant("WG_PLANES"), constant("WG_GRADS")
+ISSUERS, SUMMERS = arrivals("gempty")
+WARPS = constant("NTHREADS") // 32
+
+
+def test_the_counts_are_those_of_the_roles():
+    """One copying warp, ISSUERS issuing and SUMMERS summing; every issuing warp
+    releases a plane of h, every one of both kinds a plane of g."""
+    assert WARPS == 1 + ISSUERS + SUMMERS and ISSUERS == 3
+    assert arrivals("hempty") == [ISSUERS] and arrivals("hfull") == arrivals("gfull") == [1]
+    assert f"warp <= {ISSUERS})" in KERNEL       # the issuing warps; those above sum
 
 
 class Bar:
@@ -30,8 +58,8 @@ class Bar:
 def simulate(B, kpp, Do, nsplit, split, rng):
     n = B * kpp * Do
     s0, s1 = n * split // nsplit, n * (split + 1) // nsplit
-    hfull, hempty = [Bar(1) for _ in range(PLANES)], [Bar(3) for _ in range(PLANES)]
-    gfull, gempty = [Bar(1) for _ in range(GRADS)], [Bar(3 + 2) for _ in range(GRADS)]
+    hfull, hempty = [Bar(1) for _ in range(PLANES)], [Bar(ISSUERS) for _ in range(PLANES)]
+    gfull, gempty = [Bar(1) for _ in range(GRADS)], [Bar(ISSUERS + SUMMERS) for _ in range(GRADS)]
     hslot, gslot = [None] * PLANES, [None] * GRADS
     copies = []                                  # in flight
     mmas = [[], [], []]                          # per lane: (slots read, barriers to arrive on)
@@ -103,8 +131,9 @@ def simulate(B, kpp, Do, nsplit, split, rng):
             gempty[st].complete()
             yield "go"
 
-    summed = [], []
-    agents = {"p": producer(), 0: issuer(0), 1: issuer(1), 2: issuer(2), "s": summer(summed[0]), "t": summer(summed[1])}
+    summed = [[] for _ in range(SUMMERS)]
+    agents = {"p": producer(), **{dz: issuer(dz) for dz in range(ISSUERS)},
+              **{f"s{i}": summer(out) for i, out in enumerate(summed)}}
     idle = 0
     while agents or copies or any(mmas):
         acts = list(agents) + (["copy"] if copies else []) + [("mma", d) for d in range(3) if mmas[d]]
@@ -122,7 +151,7 @@ def simulate(B, kpp, Do, nsplit, split, rng):
             except StopIteration:
                 del agents[a]
         assert idle < 2000, "deadlock"
-    assert read == [list(range(s0, s1))] * 3 and summed == (list(range(s0, s1)),) * 2
+    assert read == [list(range(s0, s1))] * ISSUERS and summed == [list(range(s0, s1))] * SUMMERS
 
 
 @pytest.mark.parametrize("B,kpp,Do,nsplit", [(1, 1, 1, 1), (1, 2, 1, 1), (2, 3, 2, 1), (2, 2, 5, 3),

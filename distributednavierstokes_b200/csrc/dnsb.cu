@@ -132,11 +132,14 @@ struct dnsb_ctx {
   // the two-barrier k_gradmom_march at 384x256x384
   int gm_pipe = 1;
   dim3 gmgrid;
-  // least cells for the fused kernel in explicit steps: it saves two field
-  // passes of six (256^3 step 2.77 -> 2.70 ms, 192 x 128 x 192 0.847 ->
-  // 0.838), but a stage of fields that stay in L2 is faster as two kernels
-  // with more blocks (128^3 0.441 against 0.450, 64^3 0.116 against 0.121)
-  long long efuse_cells = 4000000;
+  // Least cells for the fused kernel in explicit steps.  It saves two field passes
+  // of six, but a stage of fields that partly stay in L2 is faster as two kernels
+  // with more blocks.  Fused over separate, step time, on 31 boxes: 0.97-0.99 from
+  // 16 million cells on (256^3 2.699 against 2.733 ms, 384 x 256 x 384 5.63 and
+  // 5.72), 0.99-1.00 at 13-16 (240^3 2.492 and 2.496), 1.00-1.01 at 8-13, 1.00-1.05
+  // at 4-8 (162 x 162 x 180 1.114 and 1.058; 192^3 and 192 x 128 x 192 0.99), 1.02-
+  // 1.08 below (128^3 0.452 and 0.443)
+  long long efuse_cells = 13000000;
 
   dim3 cgrid, cblock;  // launch shape of the per-cell step kernels
   // scratch
@@ -1541,7 +1544,7 @@ int dnsb_create_tuned(const dnsb_grid *gr, const dnsb_tuning *tun, int device, v
     c->cgrid = dim3((nx + bx - 1) / bx, (ny + by - 1) / by, nz);
     c->mom_tile = envint("DNSB_MOMTILE", 1) != 0;
     c->fuse = envint("DNSB_FUSE", 1) != 0;
-    c->efuse_cells = envint("DNSB_EFUSE", 4000000);
+    c->efuse_cells = envint("DNSB_EFUSE", (int)c->efuse_cells);
     c->tblock = dim3(MC_X, MC_Y, 1);
     c->tgrid = dim3((nx + MC_X - 1) / MC_X, (ny + MC_Y - 1) / MC_Y, nz);
     c->gm_pipe = std::max(0, std::min(3, envint("DNSB_GMPIPE", c->gm_pipe)));

@@ -533,7 +533,10 @@ int setup_conv_attr(dnsb_cnn *c, size_t smem) {
 // Weight gradient: shared memory of K-blocks of R rows, and the rows with the
 // least estimated time: a plane's Do + 2 rows in ceil((Do + 2) / R) blocks of
 // R P positions padded to 16, about 48 positions' worth of waits per block, and
-// 15 % where the padding needs a copy per chunk (crop 32: 4 rows of 40).
+// 15 % where the padding needs a copy per chunk.  Against every number of rows that
+// fits (1 to 16; crops of 12 to 80, odd ones among them, 1 to 8 of them) the choice
+// is within 0.5 % of the best step, 2.4 % at crop 12; with one row a step takes 1.4
+// to 3.5 times as long.
 size_t wgrad_smem(int P, int R, int ci, int co) {
   const size_t chunk = (size_t)((R * P + 15) / 16 * 16) * 16;
   return WG_PLANES * 3 * ci * chunk + WG_GRADS * 3 * co * chunk + 256 + 1024;
@@ -573,9 +576,11 @@ int alloc_volume(dnsb_cnn *c, Volume &V, int side, int B, bool training) {
   // up to four 126-output sub-tiles per plane load (fewer copies per
   // output): the most whose wider patch fits the plane and a ring of
   // RING_GOOD planes, else of at least RING_MIN.  Three planes are in use; with
-  // one ahead (3 sub-tiles, 4 slots at side 64) the next plane's copy is not
-  // done in time: 85.7 us an inference of 64^3, 81.6 with 6 slots and 1 or 2
-  // sub-tiles (training on 8 crops of 32^3 about the same, 358 and 360 us)
+  // one or two ahead the next plane's copy is not done in time: an inference of
+  // 64^3 takes 85.6 us with 3 sub-tiles and 4 slots, 84.8 with 2 and 5, 81.7 with 1
+  // and 7 (training on 8 crops of 32^3 about the same, 358 and 360 us).  Where no
+  // choice reaches RING_GOOD, one sub-tile has 5 slots and is no faster than two
+  // with 4 (side 80 144.2 against 138.5 us, 84 162.6 and 159.2, 88 178.3 and 177.3).
   {
     auto most = [&](int s, int e) {
       for (int want : {RING_GOOD, RING_MIN})

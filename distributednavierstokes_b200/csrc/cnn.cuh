@@ -427,10 +427,11 @@ struct SubWalk {
 // (32 -> 32 channels, per sub-tile: 18 MMAs of about 50 cycles; 16 epilogue warps,
 // 2.3k cycles of arithmetic and stores and 1.1k of tensor-memory reads and
 // shuffles each, every fourth sub-tile).  64^3 inference, four layers, before ->
-// now 90.3 -> 81.6 us: ranges cut at sub-tiles and six ring slots (86.2 -> 81.6),
+// now 90.3 -> 81.6 us: ranges cut at sub-tiles and a ring of seven slots (86.2 -> 81.6),
 // MMAs issued by a whole warp's uniform loop (88.5 -> 86.2), packed FP32 pairs, two
 // shuffles per output instead of three and the weights ahead of the wait
 // (90.2 -> 88.5).  Training on 8 crops of 32^3: with these 428 -> 360 us a step.
+// The tensor pipe is active 31 % of a 32 -> 32 layer at 64^3 (29 us on its own).
 template <int CI, int CO, int MODE>
 __global__ void __launch_bounds__(CONV_THREADS, 1)
     k_conv(const __grid_constant__ CUtensorMap tin, const ConvArgs a) {
@@ -835,15 +836,16 @@ struct WgradArgs {
 };
 
 // h: CI chunks (A operand, shifted in x), g: CO chunks (B operand, shifted in
-// y).  Bound by the MMAs (about 50 cycles each) and the set-up and stores around them
-// (a third plane of g in flight: 34.1 -> 33.1 us): per step (one
-// plane of one row block) six boxes of 64-byte positions and 3 KBp / 16 MMAs of
-// N = 96 (56 cycles each) for 27 taps.  With the taps stacked four at a time
-// on the rows (N = 32) every position was copied 34 times and took 7 MMAs of 52
-// cycles per 16 positions: 85.6 us for a 32 x 32-channel layer of 8 crops of
-// 32^3 (959 MB of copies, 11.7 TB/s); now 53.4 us with one issuing lane for the
-// three dz, 33.1 us with an issuing warp each and 29.3 us with the partial sums
-// stored 512 contiguous bytes a warp instead of 16 a lane at a stride of 384.
+// y): per step (one plane of one row block) six boxes of 64-byte positions and
+// 3 KBp / 16 MMAs of N = 96 (48 cycles each) for 27 taps.
+// Of a 32 x 32-channel layer of 8 crops of 32^3 (56k cycles, 29-32 us) the tensor
+// pipe takes 24k (43 %; 51 % of the first layer), set-up and the partial sums' stores
+// about 5k each; the rest is spent waiting for planes.  With the taps stacked four
+// at a time on the rows (N = 32) every position was copied 34 times and took 7 MMAs
+// of 52 cycles per 16 positions: 85.6 us (959 MB of copies, 11.7 TB/s); 53.4 us
+// with one issuing lane for the three dz, 34.1 with an issuing warp each, 33.1 with
+// a third plane of g in flight and 29.3 with the partial sums stored 512 contiguous
+// bytes a warp instead of 16 a lane at a stride of 384.
 template <int CI, int CO>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_wgrad(const __grid_constant__ CUtensorMap th, const __grid_constant__ CUtensorMap tg,

@@ -120,7 +120,8 @@ __device__ __forceinline__ void fa_step2(int N1, int N2, int P, int LS, int L, c
   });
 }
 
-// Complex FFT along z of L contiguous lines of S, in place (k_fftz).
+// Complex FFT along z of L contiguous lines of S, in place (k_fftz).  256^3: 46 us,
+// DRAM at 0.69 of the copy rate, the shared-memory pipe 70 % busy.
 template <int TIER, bool INV>
 __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
     k_fftz_any(int n, int N1, int N2, int L, long long nlines, double2 *S,
@@ -147,9 +148,10 @@ __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
 // rows.  Lines lie across threads (l fastest): L = 8 values of 16 bytes are
 // one 128-byte segment, in memory and as one conflict-free shared-memory
 // wavefront, so the buffer needs no padding.
-// Bound: HBM (two passes of the half spectrum) beside 86 FP64 operations per
-// value.  256^3 (16 x 16, L = 8): 170.6 us with the Stockham k_yfourier, 106
-// here (two passes at the copy rate: 41 us); 32^3: 6.8 -> 5.8 us.
+// Bound by the latency of its loads at 16 warps per SM (128 registers): DRAM at 0.33
+// of the copy rate, the FP64 pipe 31 % busy.  256^3 (16 x 16, L = 8): 170.6 us with
+// the Stockham k_yfourier, 98 here (two passes at the copy rate: 41 us); 32^3: 6.8
+// -> 5.8 us.
 template <int TIER, int YMODE>
 __global__ void __launch_bounds__(FA_THREADS, fa_blocks(TIER))
     k_y_any(Geo g, int N1, int N2, int L, double2 *S, const double2 *__restrict__ twy,

@@ -235,6 +235,9 @@ constexpr size_t GRADMOM_SMEM = sizeof(double) * (2 * 3 + 3 + 4 + 3 * 3) * GP_N;
 // u_z east and north) are the ones this thread read as plane K's centre in
 // the previous iteration and stay in registers.  Ring slots: u* 2, p 3,
 // delta 5, projected u 3 (x 3 components).
+// Bound by issue: 630 to 660 instructions per cell, 2.4 to 2.5 a cycle of 4, at three
+// blocks per SM (registers and shared memory both); DRAM at 0.55 of the copy rate
+// (384 x 128 x 256 semi-implicit 415 us, 256^3 explicit 488), FP64 pipe 30 %.
 // MOM_EXPLICIT: the same fusion for explicit stages (u = W - grad psi with
 // psi = delta, next W' = u + B q with ghost images into `out`, which must not
 // alias us): no pressure is staged or written.

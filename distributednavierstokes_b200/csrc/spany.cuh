@@ -16,10 +16,17 @@
 //   stage: one kernel reads the six spectra and the state and writes the
 //     projected state and the next start.
 // 4 + 3 launches per stage instead of 42; passes (n^3 values of 8 bytes, kcut
-// = n/3) 15 + 17 + 6 instead of about 90.  256^3 step 6.84 -> 4.02 ms (the six
-// products 407 us at 2.3 TB/s, bound by the FP64 work of six half-length
-// transforms per line; inverse x 219, z 184 + 175, y 93 + 152, stage 102 us),
-// 128^3 1.49 -> 0.57 ms, 32^3 0.71 -> 0.12 ms.
+// = n/3) 15 + 17 + 6 instead of about 90.  256^3 step 6.84 -> 4.03 ms, 128^3 1.49
+// -> 0.57 ms, 32^3 0.71 -> 0.12 ms.
+// Per launch at 256^3 (counters: DRAM bytes over time, share of the shared-memory
+// and L1 pipe, of the FP64 pipe):
+//   six products 417 us, 2.2 TB/s, 83 %, 35 %: the shared-memory pipe (each product
+//     reads two velocities and crosses the buffer twice; 3 blocks of 72 KB, 12
+//     warps per SM)
+//   inverse x 219 us, 2.8 TB/s, 83 %, 30 %: the same pipe
+//   inverse z 188 us, 2.1 TB/s, 32 %, 12 %: latency of the loads from the compact
+//     lines (m values of 16 bytes, every other one off its 32-byte sector)
+//   forward z 178 us, 4.8 TB/s; forward y 151, 3.8; inverse y 93, 2.8; stage 107, 5.3
 // The kernels are those of fftany.cuh with other load and store maps.
 #pragma once
 #include "fftany.cuh"

@@ -12,7 +12,10 @@
 // its rate forward, 40 % inverse).  Here LW = 32 / max(N1, N2) lines fill the
 // lanes of both steps, warps drift apart so that one's loads run under
 // another's arithmetic, and the buffer of a step is reused by the next (every
-// lane reads its inputs before any writes).  The spectrum is touched LW lines
+// lane reads its inputs before any writes).  At 256^3 the divergence and forward
+// transform then take 129 us (4.0 TB/s of DRAM, 0.61 of the copy rate), the inverse
+// 97 (its spectrum partly in L2); the shared-memory pipe is 66 % busy in both (74 %
+// at M = 192), with 16 warps per SM held by the registers.  The spectrum is touched LW lines
 // of 16 bytes at a time (32 or 64 bytes: whole sectors); the CTA's four warps
 // take adjacent lines.
 #pragma once

@@ -721,6 +721,9 @@ int allow_rfftx4(dnsb_ctx *c) {
 // the kernels of the context's compile-time splits
 int allow_fft4(dnsb_ctx *c) {
   int rc;
+  // (lines_z4 is held to what fits also where no kernel takes it)
+  if (c->z1 && c->smem_z4 > 227 * 1024)
+    return fail(c, DNSB_ECUDA, "%d lines of the z-transform need %zu bytes of shared memory", c->L4z, c->smem_z4);
 #define AX4(A, B) \
   if (c->x1 == A && c->x2 == B && (rc = allow_rfftx4<A, B>(c))) return rc;
   FFT4_SPLITS(AX4)

@@ -158,6 +158,9 @@ def test_launch_shapes_do_not_change_results(D):
         assert torch.equal(u0[c], u1[c]), c
     with pytest.raises(Exception):
         D.setup(**kw, tuning=dict(cell_bx=48, cell_by=2))   # not a multiple of 32
+    for nz in (96, 256):                                    # beyond shared memory, read (96) or not (256)
+        with pytest.raises(Exception):
+            D.setup(n=(24, 16, nz), tuning=dict(lines_z4=200))
     s0.close()
     s1.close()
 
